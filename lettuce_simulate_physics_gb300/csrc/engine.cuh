@@ -25,16 +25,28 @@ struct TreeState;     // tree.cu
 struct AdjointState;  // adjoint.cu
 struct LetStore;      // let.cu
 
+// Nodes in the reference's order, as their readers take them: what the opening test needs in one
+// 32-byte sector (the children of a node are contiguous, so a team of eight lanes reads two whole
+// lines), and what a cell's evaluation needs in one 64-byte record.
+struct alignas(32) NodeTest {
+    float4 com;   // (cx, cy, cz, rcrit2)
+    uint4 range;  // (lo, hi, first, nchild)
+};
+struct alignas(64) NodeCell {
+    float4 com;  // (cx, cy, cz, m)
+    float4 lo;   // low parts of the FP64 centre of mass
+    float4 q0;   // (qxx, qxy, qxz, qyy)
+    float4 q1;   // (qyz, qzz, rcrit2, 0)
+};
+
 // Read-only view of the built tree for the walk.
 struct TreeView {
-    const uint4* nd_range;    // (lo, hi, first, nchild), reference node order
-    const float4* nd_com;     // (cx, cy, cz, m)
-    const float4* nd_comlo;   // low parts of the FP64 centre of mass
-    const float4* nd_q0;      // (qxx, qxy, qxz, qyy)
-    const float4* nd_q1;      // (qyz, qzz, rcrit2, 0)
+    const NodeTest* nd_test;
+    const NodeCell* nd_cell;
     const uint2* grp_range;   // walk groups (lo, hi), reference order
     const float4* grp_box;    // 2 per group: (bx, by, bz, 0), (hx, hy, hz, 0)
     const unsigned* ngroups;  // device-side group count
+    const uint32_t* grp_order;  // the order the walks take the groups in (nullptr: as numbered)
     size_t T;
     // For the walk's vector-Jacobian product: parent of every node (root: 0xffffffff), leaf of
     // every body, node of every leaf.
@@ -138,7 +150,7 @@ struct Engine {
     DevBuf partial;      // split-j partial sums (scratch)
     DevBuf diag_partial; // per-block FP64 partials
     DevBuf flush_buf;
-    DevBuf walk_stack;   // per-warp traversal stacks of the tree walk
+    DevBuf walk_stack;   // overflow of the walks' shared traversal stacks
     DevBuf vjp_scratch;  // per-node adjoints of the tree walk's vector-Jacobian product
     DevBuf small;        // error word, tickets, counters, FP64 results
     unsigned* pinned_small = nullptr;

@@ -1,5 +1,5 @@
 // Locally-essential trees (LETs): the reference's multi-rank support (src/backend.hpp:50-86).
-//  - let_upload: remote trees to the device for the walk (walk_common.cuh traverse_let), indices
+//  - let_upload: remote trees to the device for the walk (walk.cu), indices
 //    made global over the concatenated trees, every link checked on the host first.
 //  - let_body_blocks: blocks of 128 consecutive bodies with their FP32 bounding boxes, the direct
 //    method's receiver groups (src/cpu_backend.cpp:695-728).
@@ -73,9 +73,9 @@ __global__ void k_let_decide(TreeView tv, const uint32_t* __restrict__ front, in
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nf) return;
     const uint32_t nd = front[k];
-    const uint4 r = tv.nd_range[nd];
-    const float4 com = tv.nd_com[nd];
-    const float rc2 = tv.nd_q1[nd].z;
+    const uint4 r = tv.nd_test[nd].range;
+    const float4 com = tv.nd_test[nd].com;
+    const float rc2 = com.w;
     const float dx = fmaxf(__fsub_rn(fabsf(__fsub_rn(com.x, bc.x)), bh.x), 0.f);
     const float dy = fmaxf(__fsub_rn(fabsf(__fsub_rn(com.y, bc.y)), bh.y), 0.f);
     const float dz = fmaxf(__fsub_rn(fabsf(__fsub_rn(com.z, bc.z)), bh.z), 0.f);
@@ -87,7 +87,7 @@ __global__ void k_let_decide(TreeView tv, const uint32_t* __restrict__ front, in
             b = r.y - r.x;
         } else {
             kd = 2;
-            for (uint32_t ch = r.z; ch < r.z + r.w; ++ch) c += tv.nd_com[ch].w > 0.f ? 1u : 0u;
+            for (uint32_t ch = r.z; ch < r.z + r.w; ++ch) c += tv.nd_cell[ch].com.w > 0.f ? 1u : 0u;
         }
     }
     kind[k] = kd;
@@ -138,8 +138,8 @@ __global__ void k_let_emit(TreeView tv, const float4* __restrict__ hm, const uin
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nf) return;
     const uint32_t nd = front[k];
-    const uint4 r = tv.nd_range[nd];
-    const float4 com = tv.nd_com[nd], q0 = tv.nd_q0[nd], q1 = tv.nd_q1[nd];
+    const uint4 r = tv.nd_test[nd].range;
+    const float4 com = tv.nd_cell[nd].com, q0 = tv.nd_cell[nd].q0, q1 = tv.nd_cell[nd].q1;
     lg_let_node o;
     o.cx = com.x; o.cy = com.y; o.cz = com.z; o.mass = com.w;
     o.qxx = q0.x; o.qxy = q0.y; o.qxz = q0.z; o.qyy = q0.w; o.qyz = q1.x; o.qzz = q1.y;
@@ -157,7 +157,7 @@ __global__ void k_let_emit(TreeView tv, const float4* __restrict__ hm, const uin
         o.child_count = static_cast<int32_t>(ccount[k]);
         uint32_t j = cs[k];
         for (uint32_t ch = r.z; ch < r.z + r.w; ++ch)
-            if (tv.nd_com[ch].w > 0.f) next[j++] = ch;
+            if (tv.nd_cell[ch].com.w > 0.f) next[j++] = ch;
     }
     out[base + k] = o;
 }
@@ -246,6 +246,7 @@ TreeView let_body_blocks(Engine& e, int block) {
     TreeView v{};
     v.grp_range = s.blk_range.as<uint2>();
     v.grp_box = s.blk_box.as<float4>();
+    v.grp_order = nullptr;
     v.ngroups = s.blk_count.as<unsigned>();
     v.T = 0;
     return v;
@@ -292,7 +293,7 @@ void let_export(Engine& e, const float lo[3], const float hi[3], const lg_force_
     const TreeView tv = tree_view(e);
     // Root of zero mass (or no bodies): empty LET.
     float4 root{};
-    LG_CK(cudaMemcpyAsync(&root, tv.nd_com, 16, cudaMemcpyDeviceToHost, st));
+    LG_CK(cudaMemcpyAsync(&root, &tv.nd_cell->com, 16, cudaMemcpyDeviceToHost, st));
     LG_CK(cudaStreamSynchronize(st));
     if (!(root.w > 0.f)) {
         *nnodes = *nbodies = 0;

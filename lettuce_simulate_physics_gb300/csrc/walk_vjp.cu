@@ -188,7 +188,8 @@ __device__ void vjp_flush(const VjpArgs& a, VjpSmem& s, int lane, int np, uint32
         const int cc = min(VCCH, nc - c0);
         for (int k = lane; k < cc; k += 32) {
             const uint32_t nd = s.clist[c0 + k];
-            const float4 com = a.tv.nd_com[nd], cl = a.tv.nd_comlo[nd], q0 = a.tv.nd_q0[nd], q1 = a.tv.nd_q1[nd];
+            const NodeCell& rec = a.tv.nd_cell[nd];
+            const float4 com = rec.com, cl = rec.lo, q0 = rec.q0, q1 = rec.q1;
             const float X = (com.x - ox) + cl.x, Y = (com.y - oy) + cl.y, Z = (com.z - oz) + cl.z;
             s.cx[k] = X; s.cy[k] = Y; s.cz[k] = Z;
             s.cm[k] = com.w;
@@ -357,6 +358,7 @@ __global__ void __launch_bounds__(VWBS) k_walk_vjp(VjpArgs a) {
         if (lane == 0) g = atomicAdd(a.group_ctr, 1u);
         g = __shfl_sync(0xffffffffu, g, 0);
         if (g >= ngroups) break;
+        if (a.tv.grp_order) g = a.tv.grp_order[g];
         const uint2 gr = a.tv.grp_range[g];
         const float4 bc = a.tv.grp_box[2 * g], bh = a.tv.grp_box[2 * g + 1];
         for (uint32_t plo = gr.x; plo < gr.y; plo += VPASS) {
@@ -419,7 +421,7 @@ __global__ void k_moment_chain(TreeView tv, const BodyArrays b, int n, const dou
         const double dM = nadj[node], dcx = nadj[T + node], dcy = nadj[2 * T + node], dcz = nadj[3 * T + node];
         const double qxx = nadj[4 * T + node], qxy = nadj[5 * T + node], qxz = nadj[6 * T + node];
         const double qyy = nadj[7 * T + node], qyz = nadj[8 * T + node], qzz = nadj[9 * T + node];
-        const float4 c = tv.nd_com[node], cl = tv.nd_comlo[node];
+        const float4 c = tv.nd_cell[node].com, cl = tv.nd_cell[node].lo;
         const double M = c.w;
         const double ex = xb - (static_cast<double>(c.x) + cl.x);
         const double ey = yb - (static_cast<double>(c.y) + cl.y);
