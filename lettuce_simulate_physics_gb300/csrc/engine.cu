@@ -142,7 +142,7 @@ void Engine::upload(size_t count, const float* x, const float* y, const float* z
     kick_rec = drift_rec = false;
     block_ready = false;
     times = lg_phase_times{};
-    tree_reset_guess(*this);
+    tree_reset(*this);
     if (n == 0) return;
     const size_t fb = count * 4;
     BodyArrays b = bodies(0);

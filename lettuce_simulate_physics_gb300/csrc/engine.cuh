@@ -174,7 +174,8 @@ size_t tree_held_bytes(const Engine& e);
 TreeView tree_view(Engine& e);
 bool tree_verify(Engine& e, const unsigned* counts_host);
 const unsigned* tree_counts_device(Engine& e);
-void tree_reset_guess(Engine& e);
+void tree_reset_guess(Engine& e);  // the next build reads its sizes
+void tree_reset(Engine& e);        // new bodies: nothing known of their tree
 double tree_theta(const Engine& e);
 // Forest mode (ensembles): the tree covers bodies [0, n_tree) of nsys systems; sys (per body),
 // sys_off (nsys + 1 body offsets) and inv_theta_sys (per system) are device arrays the caller

@@ -12,9 +12,10 @@
 //
 // Construction (no level-by-level loop, no recursion):
 //  1. bbox and key frame (FP64), keys (src/cpu_backend.cpp:418-428 formula), identity values.
-//  2. Onesweep radix sort (Adinets & Merrill 2022): one histogram pass for all eight 8-bit digits,
-//     then one kernel per digit with decoupled look-back across tiles; digits that are constant
-//     over all keys are skipped on the device. Stable, so the permutation equals the reference's.
+//  2. Onesweep radix sort (Adinets & Merrill 2022) by the leading key digits the tree's depth needs:
+//     histograms of all 8-bit digits with the keys, then one kernel per digit with decoupled
+//     look-back across tiles; ties ordered by the whole keys in the gather. Stable, so the
+//     permutation equals the reference's.
 //  3. Key restarts: runs of > 16 identical keys are re-keyed in their own bounding cube (the
 //     reference's rekey, src/cpu_backend.cpp:503-530) and sorted by the new keys inside each run;
 //     runs whose composite keys still tie are re-keyed again, up to FRAMES frames (depth 126).
@@ -84,18 +85,22 @@ constexpr unsigned FLAG_AGG = 1u << 30, FLAG_INC = 2u << 30, VAL_MASK = (1u << 3
 #endif
 constexpr int LB_BATCH = LG_LB_BATCH;  // predecessors read per look-back round trip
 
-struct SortCtl {
-    unsigned sel;
-    unsigned skip[PASSES];
-    unsigned tile_ctr[PASSES];
-    unsigned done_ctr[PASSES];
+// Device memory that one kernel zeroes for those after it (16-byte words).
+struct ZeroSpan {
+    uint4* p;
+    size_t words;
+};
+constexpr int ZSPANS = 3;
+struct ZeroList {
+    ZeroSpan span[ZSPANS];
 };
 
 }  // namespace
 
 struct TreeState {
     // sort
-    DevBuf keysA, keysB, valsA, valsB, hist, lookback, ctl;
+    DevBuf keysA, keysB, valsA, valsB, hist, lookback;
+    bool sort_full = false;  // a partial sort met a run too long to order locally: all key bits from now on
     // sorted frame-0 keys, per-body tree data
     DevBuf skey, bdepth, flag, leafid;
     // frame, key-restart runs and frames (index 0 of the per-frame buffers unused)
@@ -132,7 +137,7 @@ struct TreeState {
     const uint32_t* sys_off = nullptr;
     const float* inv_theta_sys = nullptr;
     uint64_t generation = 0;  // bumped by every build that may grow (reallocate) tree buffers
-    DevBuf mkeys;   // forest: Morton keys before the (system, key) sort
+    DevBuf mkeys;   // Morton keys in the bodies' order before the sort
     // merged walk groups
     bool merged = false;
     DevBuf mcount, moff, mrange, mbox;
@@ -272,7 +277,16 @@ __device__ __forceinline__ void write_frame(const long long (&v)[6], double* f) 
     f[4] = __ddiv_rn(static_cast<double>(1u << MAX_LEVEL), side);
 }
 
-__global__ void k_frame(const BodyArrays b, int n, long long* partial, unsigned* ticket, double* frame) {
+__device__ __forceinline__ void zero_spans(const ZeroList& z) {
+#pragma unroll
+    for (int q = 0; q < ZSPANS; ++q)
+        for (size_t k = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; k < z.span[q].words;
+             k += static_cast<size_t>(gridDim.x) * blockDim.x)
+            z.span[q].p[k] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+__global__ void k_frame(const BodyArrays b, int n, long long* partial, unsigned* ticket, double* frame, ZeroList z) {
+    zero_spans(z);
     __shared__ long long sh[6][BS / 32];
     __shared__ bool last;
     long long v[6];
@@ -302,17 +316,34 @@ __global__ void k_frame(const BodyArrays b, int n, long long* partial, unsigned*
     }
 }
 
+// Morton keys, the keys the sort works on (their values, the positions, are left to the first pass),
+// and the digit histograms of the sort's passes. The sort key is the leading `levels` octal digits
+// of the Morton key, under the system's index with sys_key. One histogram per block in shared
+// memory, blocks few enough that adding them up stays cheap.
 __global__ void k_keys(const uint32_t* __restrict__ sys, const BodyArrays b, int n, const double* __restrict__ frame,
-                       uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double* f = frame + 5 * sys_of(sys, i);
-    keys[i] = morton(b.x[i], b.y[i], b.z[i], f[0], f[1], f[2], f[4]);
-    vals[i] = static_cast<uint32_t>(i);
+                       uint64_t* __restrict__ mkeys, uint64_t* __restrict__ keys, int levels, int passes, int sys_key,
+                       unsigned* __restrict__ hist) {
+    __shared__ unsigned h[PASSES * RADIX];
+    for (int k = threadIdx.x; k < passes * RADIX; k += blockDim.x) h[k] = 0;
+    __syncthreads();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t s = sys_of(sys, i);
+        const double* f = frame + 5 * s;
+        const uint64_t m = morton(b.x[i], b.y[i], b.z[i], f[0], f[1], f[2], f[4]);
+        uint64_t k = m >> (3 * (MAX_LEVEL - levels));
+        if (sys_key) k |= static_cast<uint64_t>(s) << (3 * levels);
+        mkeys[i] = m;
+        keys[i] = k;
+        for (int p = 0; p < passes; ++p) atomicAdd(&h[p * RADIX + static_cast<int>((k >> (8 * p)) & 255)], 1u);
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < passes * RADIX; k += blockDim.x)
+        if (h[k]) atomicAdd(&hist[k], h[k]);
 }
 
 // Forest: one block per system computes its key frame over its body range [off[s], off[s + 1]).
-__global__ void k_frame_sys(const BodyArrays b, const uint32_t* __restrict__ off, double* frame) {
+__global__ void k_frame_sys(const BodyArrays b, const uint32_t* __restrict__ off, double* frame, ZeroList z) {
+    zero_spans(z);
     __shared__ long long sh[6][BS / 32];
     const uint32_t lo = off[blockIdx.x], hi = off[blockIdx.x + 1];
     long long v[6];
@@ -330,75 +361,60 @@ __global__ void k_sys_keys(const uint32_t* __restrict__ sys, const uint32_t* __r
 }
 
 // ---- onesweep radix sort ---------------------------------------------------------------------
-__global__ void k_sort_hist(const uint64_t* __restrict__ keys, int n, unsigned* __restrict__ hist) {
-    __shared__ unsigned h[PASSES][RADIX];
-    for (int k = threadIdx.x; k < PASSES * RADIX; k += blockDim.x) (&h[0][0])[k] = 0;
+// Digit histograms of keys already in memory (the key restarts' sorts).
+__global__ void k_sort_hist(const uint64_t* __restrict__ keys, int n, int passes, unsigned* __restrict__ hist) {
+    __shared__ unsigned h[PASSES * RADIX];
+    for (int k = threadIdx.x; k < passes * RADIX; k += blockDim.x) h[k] = 0;
     __syncthreads();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint64_t k = keys[i];
-#pragma unroll
-        for (int p = 0; p < PASSES; ++p) atomicAdd(&h[p][(k >> (8 * p)) & 255], 1u);
+        for (int p = 0; p < passes; ++p) atomicAdd(&h[p * RADIX + static_cast<int>((k >> (8 * p)) & 255)], 1u);
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < PASSES * RADIX; k += blockDim.x) {
-        const unsigned v = (&h[0][0])[k];
-        if (v) atomicAdd(&hist[k], v);
-    }
+    for (int k = threadIdx.x; k < passes * RADIX; k += blockDim.x)
+        if (h[k]) atomicAdd(&hist[k], h[k]);
 }
 
-// Exclusive digit offsets per pass; a pass whose digit is constant over all keys is skipped.
-__global__ void k_sort_offsets(unsigned* __restrict__ hist, int n, SortCtl* ctl) {
-    __shared__ unsigned s[RADIX];
-    const int d = threadIdx.x;
-    for (int p = 0; p < PASSES; ++p) {
-        const unsigned c = hist[p * RADIX + d];
-        s[d] = c;
-        __syncthreads();
-        // Hillis-Steele inclusive scan over 256 entries.
-        for (int o = 1; o < RADIX; o <<= 1) {
-            unsigned t = d >= o ? s[d - o] : 0;
-            __syncthreads();
-            s[d] += t;
-            __syncthreads();
-        }
-        hist[p * RADIX + d] = s[d] - c;
-        const int full = __syncthreads_or(c == static_cast<unsigned>(n));
-        if (d == 0) {
-            ctl->skip[p] = full ? 1u : 0u;
-            ctl->tile_ctr[p] = 0;
-            ctl->done_ctr[p] = 0;
-        }
-        __syncthreads();
+// Exclusive sum over the block's 256 threads (sh: one word per warp); begins with a barrier.
+__device__ __forceinline__ unsigned block_excl_sum(unsigned v, unsigned* sh) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
     }
-    if (d == 0) ctl->sel = 0;
+    __syncthreads();
+    if (lane == 31) sh[w] = incl;
+    __syncthreads();
+    unsigned before = 0;
+#pragma unroll
+    for (int u = 0; u < SORT_BS / 32; ++u)
+        if (u < w) before += sh[u];
+    return before + incl - v;
 }
 
-__global__ void __launch_bounds__(SORT_BS) k_sort_pass(uint64_t* __restrict__ kA, uint32_t* __restrict__ vA,
-                                                       uint64_t* __restrict__ kB, uint32_t* __restrict__ vB, int n,
-                                                       int pass, const unsigned* __restrict__ offsets,
-                                                       unsigned* __restrict__ lookback, SortCtl* ctl,
+// One pass: (src_k, src_v) to (dst_k, dst_v) by the digit at `shift`; src_v null: values are the
+// positions. hist: the digit's counts over all keys; tile_ctr and lookback start at zero.
+__global__ void __launch_bounds__(SORT_BS) k_sort_pass(const uint64_t* __restrict__ src_k,
+                                                       const uint32_t* __restrict__ src_v,
+                                                       uint64_t* __restrict__ dst_k, uint32_t* __restrict__ dst_v, int n,
+                                                       int shift, const unsigned* __restrict__ hist,
+                                                       unsigned* __restrict__ lookback, unsigned* tile_ctr,
                                                        unsigned* err) {
     __shared__ unsigned warp_hist[SORT_BS / 32][RADIX];
     __shared__ unsigned gbase[RADIX];       // global start of each digit for this tile
-    __shared__ unsigned tstart[RADIX];      // inclusive scan of the tile's digit counts
+    __shared__ unsigned tstart[RADIX];      // start of each digit in the staged tile
     __shared__ uint64_t stage_k[SORT_TILE]; // the tile in digit order
     __shared__ uint32_t stage_v[SORT_TILE];
-    __shared__ unsigned tile_s, sel_s;
-    if (ctl->skip[pass]) return;
+    __shared__ unsigned tile_s, scan_s[SORT_BS / 32];
+    static_assert(SORT_BS == RADIX, "one thread per digit");
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    if (tid == 0) {
-        tile_s = atomicAdd(&ctl->tile_ctr[pass], 1u);
-        sel_s = *reinterpret_cast<volatile unsigned*>(&ctl->sel);
-    }
+    if (tid == 0) tile_s = atomicAdd(tile_ctr, 1u);
     for (int k = tid; k < (SORT_BS / 32) * RADIX; k += SORT_BS) (&warp_hist[0][0])[k] = 0;
-    __syncthreads();
+    // The digit's start among all keys; the barriers also publish tile_s and the cleared counts.
+    const unsigned digit_start = block_excl_sum(hist[tid], scan_s);
     const unsigned tile = tile_s;
-    const unsigned ntiles = (n + SORT_TILE - 1) / SORT_TILE;
-    const uint64_t* src_k = sel_s ? kB : kA;
-    const uint32_t* src_v = sel_s ? vB : vA;
-    uint64_t* dst_k = sel_s ? kA : kB;
-    uint32_t* dst_v = sel_s ? vA : vB;
-    const int shift = 8 * pass;
     const int tile0 = tile * SORT_TILE;
     const int wbase = tile0 + w * (32 * SORT_IPT);
     const int tile_n = min(SORT_TILE, n - tile0);
@@ -406,17 +422,18 @@ __global__ void __launch_bounds__(SORT_BS) k_sort_pass(uint64_t* __restrict__ kA
     uint64_t key[SORT_IPT];
     uint32_t val[SORT_IPT];
     unsigned rank[SORT_IPT];
-    int dig[SORT_IPT];
     const unsigned lt = (1u << lane) - 1u;
-    // Stable rank inside the tile: keys in index order (warp, round, lane).
 #pragma unroll
     for (int r = 0; r < SORT_IPT; ++r) {
         const int i = wbase + r * 32 + lane;
-        const bool valid = i < n;
-        key[r] = valid ? src_k[i] : 0;
-        val[r] = valid ? src_v[i] : 0;
+        key[r] = i < n ? src_k[i] : 0;
+        val[r] = i < n ? (src_v ? src_v[i] : static_cast<uint32_t>(i)) : 0;
+    }
+    // Stable rank inside the tile: keys in index order (warp, round, lane).
+#pragma unroll
+    for (int r = 0; r < SORT_IPT; ++r) {
+        const bool valid = wbase + r * 32 + lane < n;
         const int d = valid ? static_cast<int>((key[r] >> shift) & 255) : -1 - lane;
-        dig[r] = d;
         const unsigned peers = __match_any_sync(0xffffffffu, d);
         const unsigned before = __popc(peers & lt);
         unsigned basev = 0;
@@ -477,26 +494,16 @@ __global__ void __launch_bounds__(SORT_BS) k_sort_pass(uint64_t* __restrict__ kA
             }
             lb[d] = FLAG_INC | ((prefix + tile_count) & VAL_MASK);
         }
-        gbase[d] = offsets[pass * RADIX + d] + prefix;
-        // Exclusive scan of the tile's digit counts (Hillis-Steele over 256 threads).
-        tstart[d] = tile_count;
+        gbase[d] = digit_start + prefix;
+        tstart[d] = block_excl_sum(tile_count, scan_s);
     }
     __syncthreads();
-    for (int o = 1; o < RADIX; o <<= 1) {
-        const unsigned t = tid >= o ? tstart[tid - o] : 0u;
-        __syncthreads();
-        tstart[tid] += t;
-        __syncthreads();
-    }
-    // tstart now holds the inclusive scan: digit d starts at tstart[d - 1] (0 for d = 0).
     // Stage the tile in digit order (tile-local position = digit start + rank within the digit).
 #pragma unroll
     for (int r = 0; r < SORT_IPT; ++r) {
-        const int i = wbase + r * 32 + lane;
-        if (i < n) {
-            const int d = dig[r];
-            const unsigned excl = (d > 0 ? tstart[d - 1] : 0u);
-            const unsigned pos = excl + warp_hist[w][d] + rank[r];
+        if (wbase + r * 32 + lane < n) {
+            const int d = static_cast<int>((key[r] >> shift) & 255);
+            const unsigned pos = tstart[d] + warp_hist[w][d] + rank[r];
             stage_k[pos] = key[r];
             stage_v[pos] = val[r];
         }
@@ -506,62 +513,65 @@ __global__ void __launch_bounds__(SORT_BS) k_sort_pass(uint64_t* __restrict__ kA
     for (int p = tid; p < tile_n; p += SORT_BS) {
         const uint64_t k = stage_k[p];
         const int d = static_cast<int>((k >> shift) & 255);
-        const unsigned excl = (d > 0 ? tstart[d - 1] : 0u);
-        const unsigned gpos = gbase[d] + (p - excl);
-        dst_k[gpos] = k;
-        dst_v[gpos] = stage_v[p];
-    }
-    // The last tile to finish flips the buffer selector (every tile has read it by then).
-    __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        if (atomicAdd(&ctl->done_ctr[pass], 1u) == ntiles - 1) ctl->sel ^= 1u;
+        const unsigned gpos = gbase[d] + (p - tstart[d]);
+        if (gpos < static_cast<unsigned>(n)) {  // false only after a wait that timed out
+            dst_k[gpos] = k;
+            dst_v[gpos] = stage_v[p];
+        }
     }
 }
 
-// Gathers every body array into the other body set in the order of the permutation in vals;
-// copies the sorted keys; optionally carries a second key array through the permutation.
+// Gathers every body array into the other body set in the sorted order, and the Morton keys with
+// them (mkeys: by body before the sort). A sort by the leading digits only (partial) leaves runs of
+// bodies with equal sort keys in their former order; each body of such a run finds its place by
+// counting the run's bodies with a smaller Morton key (or an equal one, before it), so the order is
+// that of a stable sort by the whole keys. A run of more than LEAF_MAX is left as it is and
+// flagged: the tree is then deeper than the sorted digits, and the sort is redone with all of them.
+// key1_in (optional): a second key carried through the permutation (no partial runs then).
 __global__ void k_permute(const BodyArrays src, BodyArrays dst, const uint64_t* __restrict__ keys,
-                          const uint32_t* __restrict__ vals, uint64_t* __restrict__ skey,
-                          const uint64_t* __restrict__ key1_in, uint64_t* __restrict__ key1_out, int n,
-                          const uint64_t* __restrict__ key_src, int n_total) {
+                          const uint32_t* __restrict__ vals, const uint64_t* __restrict__ mkeys,
+                          uint64_t* __restrict__ skey, const uint64_t* __restrict__ key1_in,
+                          uint64_t* __restrict__ key1_out, int n, int n_total, int partial, unsigned* long_run) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_total) return;
-    // Bodies past the tree's range (the forest's direct systems) keep their place.
-    const uint32_t j = i < n ? vals[i] : static_cast<uint32_t>(i);
-    if (i < n && skey) skey[i] = key_src ? key_src[j] : keys[i];
-    if (i >= n) {
-        dst.x[i] = src.x[i]; dst.y[i] = src.y[i]; dst.z[i] = src.z[i];
-        dst.hm[i] = src.hm[i]; dst.lo[i] = src.lo[i];
-        dst.vx[i] = src.vx[i]; dst.vy[i] = src.vy[i]; dst.vz[i] = src.vz[i];
-        dst.m[i] = src.m[i]; dst.id[i] = src.id[i]; dst.cost[i] = src.cost[i];
-        dst.level[i] = src.level[i];
-        return;
+    int to = i;
+    uint32_t j = static_cast<uint32_t>(i);  // bodies past the tree's range (the forest's direct systems) stay
+    if (i < n) {
+        j = vals[i];
+        if (j >= static_cast<uint32_t>(n)) return;  // only after a wait that timed out
+        if (skey) {
+            const uint64_t m = mkeys[j];
+            if (partial) {
+                const uint64_t k = keys[i];
+                int a = i, e = i + 1;
+                while (a > 0 && i - a <= LEAF_MAX && keys[a - 1] == k) --a;
+                while (e < n && e - i <= LEAF_MAX && keys[e] == k) ++e;
+                if (e - a > LEAF_MAX) {
+                    *long_run = 1u;
+                } else if (e - a > 1) {
+                    to = a;
+                    for (int q = a; q < e; ++q) {
+                        const uint64_t mq = mkeys[vals[q]];
+                        to += mq < m || (mq == m && q < i) ? 1 : 0;
+                    }
+                }
+            }
+            skey[to] = m;
+        }
+        if (key1_in) key1_out[to] = key1_in[j];
     }
-    if (key1_in) key1_out[i] = key1_in[j];
-    dst.x[i] = src.x[j];
-    dst.y[i] = src.y[j];
-    dst.z[i] = src.z[j];
-    dst.hm[i] = src.hm[j];
-    dst.lo[i] = src.lo[j];
-    dst.vx[i] = src.vx[j];
-    dst.vy[i] = src.vy[j];
-    dst.vz[i] = src.vz[j];
-    dst.m[i] = src.m[j];
-    dst.id[i] = src.id[j];
-    dst.cost[i] = src.cost[j];
-    dst.level[i] = src.level[j];
-}
-
-// After the passes: if the sorted pairs ended in buffer B, copy them to A (so every sort returns
-// its result in A), and reset the selector.
-__global__ void k_sort_finish(uint64_t* __restrict__ kA, uint32_t* __restrict__ vA, const uint64_t* __restrict__ kB,
-                              const uint32_t* __restrict__ vB, const SortCtl* ctl, int n) {
-    if (ctl->sel == 0) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        kA[i] = kB[i];
-        vA[i] = vB[i];
-    }
+    dst.x[to] = src.x[j];
+    dst.y[to] = src.y[j];
+    dst.z[to] = src.z[j];
+    dst.hm[to] = src.hm[j];
+    dst.lo[to] = src.lo[j];
+    dst.vx[to] = src.vx[j];
+    dst.vy[to] = src.vy[j];
+    dst.vz[to] = src.vz[j];
+    dst.m[to] = src.m[j];
+    dst.id[to] = src.id[j];
+    dst.cost[to] = src.cost[j];
+    dst.level[to] = src.level[j];
 }
 
 // ---- exclusive scan (decoupled look-back) ----------------------------------------------------
@@ -753,10 +763,6 @@ __global__ void k_fill_u64(uint64_t* a, uint64_t v, int n) {
 __global__ void k_fill_i32(int* a, int v, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) a[i] = v;
-}
-__global__ void k_iota(uint32_t* a, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = static_cast<uint32_t>(i);
 }
 
 // ---- leaves ----------------------------------------------------------------------------------
@@ -1433,32 +1439,40 @@ void scan_u32(Engine& e, TreeState& t, const uint32_t* in, uint32_t* out, int n,
     ++e.launches;
 }
 
-// Sorts (keys, vals) held in (keysA, valsA); result in the buffer ctl->sel selects.
-void sort_pairs(Engine& e, TreeState& t, int n) {
-    cudaStream_t s = e.stream;
-    const int tiles = (n + SORT_TILE - 1) / SORT_TILE;
-    t.hist.reserve(PASSES * RADIX * 4);
-    t.lookback.reserve(static_cast<size_t>(PASSES) * tiles * RADIX * 4);
-    t.ctl.reserve(sizeof(SortCtl));
-    LG_CK(cudaMemsetAsync(t.hist.as<char>(), 0, PASSES * RADIX * 4, s));
-    LG_CK(cudaMemsetAsync(t.lookback.as<char>(), 0, static_cast<size_t>(PASSES) * tiles * RADIX * 4, s));
-    const int hb = std::min(e.sms * 4, std::max(1, grid_for(n, 1024)));
-    k_sort_hist<<<hb, 256, 0, s>>>(t.keysA.as<uint64_t>(), n, t.hist.as<unsigned>());
-    LG_LAUNCHED();
-    k_sort_offsets<<<1, RADIX, 0, s>>>(t.hist.as<unsigned>(), n, t.ctl.as<SortCtl>());
-    LG_LAUNCHED();
-    for (int p = 0; p < PASSES; ++p) {
-        k_sort_pass<<<tiles, SORT_BS, 0, s>>>(t.keysA.as<uint64_t>(), t.valsA.as<uint32_t>(), t.keysB.as<uint64_t>(),
-                                              t.valsB.as<uint32_t>(), n, p, t.hist.as<unsigned>(),
-                                              t.lookback.as<unsigned>() + static_cast<size_t>(p) * tiles * RADIX,
-                                              t.ctl.as<SortCtl>(), e.err_word());
+int sort_tiles(int n) { return (n + SORT_TILE - 1) / SORT_TILE; }
+
+// Histograms and pass counters, then the passes' look-back words: zero before a sort begins.
+size_t hist_words(void) { return (PASSES * RADIX + 16) * 4 / 16; }
+size_t lookback_words(int n, int passes) { return static_cast<size_t>(passes) * sort_tiles(n) * RADIX * 4 / 16; }
+
+// Sorts the n keys in keysA by their low 8 * passes bits, values starting as the positions (or as
+// valsA); histograms already in t.hist. Returns which buffers hold the result (0: A, 1: B).
+int sort_passes(Engine& e, TreeState& t, int n, int passes, bool iota, int pass0 = 0, int from = 0) {
+    uint64_t* k[2] = {t.keysA.as<uint64_t>(), t.keysB.as<uint64_t>()};
+    uint32_t* v[2] = {t.valsA.as<uint32_t>(), t.valsB.as<uint32_t>()};
+    const int tiles = sort_tiles(n);
+    unsigned* hist = t.hist.as<unsigned>();
+    for (int p = pass0; p < passes; ++p, from ^= 1) {
+        k_sort_pass<<<tiles, SORT_BS, 0, e.stream>>>(k[from], iota && p == 0 ? nullptr : v[from], k[from ^ 1], v[from ^ 1], n,
+                                                     8 * p, hist + p * RADIX,
+                                                     t.lookback.as<unsigned>() + static_cast<size_t>(p) * tiles * RADIX,
+                                                     hist + PASSES * RADIX + p, e.err_word());
         LG_LAUNCHED();
+        ++e.launches;
     }
-    k_sort_finish<<<std::max(1, std::min(4 * e.sms, grid_for(n, BS))), BS, 0, s>>>(
-        t.keysA.as<uint64_t>(), t.valsA.as<uint32_t>(), t.keysB.as<uint64_t>(), t.valsB.as<uint32_t>(),
-        t.ctl.as<SortCtl>(), n);
+    return from;
+}
+
+// The same with the histograms formed and everything zeroed here; result in A (passes is even).
+void sort_pairs(Engine& e, TreeState& t, int n, bool iota) {
+    cudaStream_t s = e.stream;
+    LG_CK(cudaMemsetAsync(t.hist.as<char>(), 0, hist_words() * 16, s));
+    LG_CK(cudaMemsetAsync(t.lookback.as<char>(), 0, lookback_words(n, PASSES) * 16, s));
+    const int hb = std::min(e.sms * 4, std::max(1, grid_for(n, 1024)));
+    k_sort_hist<<<hb, 256, 0, s>>>(t.keysA.as<uint64_t>(), n, PASSES, t.hist.as<unsigned>());
     LG_LAUNCHED();
-    e.launches += 3 + PASSES;
+    ++e.launches;
+    sort_passes(e, t, n, PASSES, iota);
 }
 
 void reserve_sort(TreeState& t, int n) {
@@ -1466,6 +1480,25 @@ void reserve_sort(TreeState& t, int n) {
     t.keysA.reserve(cnt * 8); t.keysB.reserve(cnt * 8);
     t.valsA.reserve(cnt * 4); t.valsB.reserve(cnt * 4);
     t.skey.reserve(cnt * 8);
+    t.mkeys.reserve(cnt * 8);
+    t.hist.reserve(hist_words() * 16);
+    t.lookback.reserve(lookback_words(n, PASSES) * 16);
+    t.counts.reserve(64);
+}
+
+// Octal digits to sort by when no earlier build says how deep the tree is: one and a half times
+// log8 n and two more (cells of that depth hold a few bodies at most in the scenarios' density
+// ranges: the trees of 8e3, 1e5, 1e6 and 1.6e7 bodies are 7, 9, 11 and 13 deep).
+int default_levels(int n) {
+    int l = 0;
+    while ((1ll << (3 * l)) < n) ++l;
+    return std::min(MAX_LEVEL, l + (l + 1) / 2 + 2);
+}
+
+int bits_for(int count) {
+    int b = 0;
+    while ((1 << b) < count) ++b;
+    return b;
 }
 
 }  // namespace
@@ -1485,57 +1518,88 @@ void tree_sort(Engine& e) {
     if (n >= (1 << 30)) fail(kRuntime, "cuda tree: n >= 2^30 exceeds the sort's look-back counters");
     reserve_sort(t, n);
     t.frame.reserve(static_cast<size_t>(std::max(t.nsys, 1)) * 5 * 8 + 64);
-    t.counts.reserve(64);
     t.restarted = false;
     t.nframes = 1;
-    if (sys) {
-        k_frame_sys<<<t.nsys, BS, 0, s>>>(e.bodies(e.cur), t.sys_off, t.frame.as<double>());
-    } else {
-        const int fb = std::min(2 * e.sms, grid_for(n, BS));
-        e.diag_partial.reserve(static_cast<size_t>(fb) * 12 * 8);
-        k_frame<<<fb, BS, 0, s>>>(e.bodies(e.cur), n, e.diag_partial.as<long long>(), e.ticket(), t.frame.as<double>());
-    }
-    LG_LAUNCHED();
-    if (sys) t.mkeys.reserve(static_cast<size_t>(n) * 8 + 8);
-    k_keys<<<grid_for(n, BS), BS, 0, s>>>(sys, e.bodies(e.cur), n, t.frame.as<double>(),
-                                          sys ? t.mkeys.as<uint64_t>() : t.keysA.as<uint64_t>(), t.valsA.as<uint32_t>());
-    LG_LAUNCHED();
-    e.launches += 2;
-    if (sys) LG_CK(cudaMemcpyAsync(t.keysA.as<uint64_t>(), t.mkeys.as<uint64_t>(), static_cast<size_t>(n) * 8,
-                                   cudaMemcpyDeviceToDevice, s));
-    sort_pairs(e, t, n);
-    if (sys) {
-        // Forest: stable sort by system on top of the key order -> (system, key) order.
-        k_sys_keys<<<grid_for(n, BS), BS, 0, s>>>(sys, t.valsA.as<uint32_t>(), t.keysA.as<uint64_t>(), n);
+    unsigned* counts = t.counts.as<unsigned>();
+    const int sysbits = sys ? bits_for(t.nsys) : 0;
+    const int run_cap = std::max(1, n / (LEAF_MAX + 1) + 1);  // runs hold more than LEAF_MAX bodies each
+    unsigned R = 0;
+    // The leading digits decide the order of all bodies but those of one cell that deep: as many
+    // digits are sorted as the tree was deep last time (with its headroom), in whole 8-bit passes
+    // (8e3 bodies: 4 passes, 1e5: 5, 1e6: 5, 1.6e7: 6, of 8 for all 63 bits), and bodies that tie
+    // are ordered where they are gathered (k_permute). A tree that turns out deeper is found there,
+    // and the sort redone with every digit; so it is from then on. With the clearing, the
+    // histograms and the digits' scans folded into the kernels around the passes: sort phase 142 ->
+    // 54 us (8191 bodies), 160 -> 75 (1e5), 302 -> 184 (1e6 disk), 2.76 -> 2.12 ms (1.6e7); below
+    // 1e6 it is the latency of 7 or 8 dependent launches, above, the passes' traffic.
+    for (bool full = t.sort_full || t.restart_mode;; full = true) {
+        int levels = MAX_LEVEL, passes = PASSES;
+        if (!full) {
+            const int want = t.have_guess ? std::min(t.max_depth, MAX_LEVEL) : default_levels(n);
+            passes = std::max(1, (3 * want + sysbits + 7) / 8);
+            levels = std::min(MAX_LEVEL, (8 * passes - sysbits) / 3);
+            full = passes >= PASSES;
+        }
+        if (full) {
+            levels = MAX_LEVEL;
+            passes = PASSES;
+        }
+        ZeroList z{};
+        z.span[0] = {t.counts.as<uint4>(), 4};
+        z.span[1] = {t.hist.as<uint4>(), hist_words()};
+        z.span[2] = {t.lookback.as<uint4>(), lookback_words(n, passes)};
+        if (sys) {
+            k_frame_sys<<<t.nsys, BS, 0, s>>>(e.bodies(e.cur), t.sys_off, t.frame.as<double>(), z);
+        } else {
+            const int fb = std::min(2 * e.sms, grid_for(n, BS));
+            e.diag_partial.reserve(static_cast<size_t>(fb) * 12 * 8);
+            k_frame<<<fb, BS, 0, s>>>(e.bodies(e.cur), n, e.diag_partial.as<long long>(), e.ticket(),
+                                      t.frame.as<double>(), z);
+        }
+        LG_LAUNCHED();
+        // With every digit sorted the system index does not fit beside them: it is sorted on its own.
+        k_keys<<<std::min(2 * e.sms, grid_for(n, 512)), 512, 0, s>>>(
+            sys, e.bodies(e.cur), n, t.frame.as<double>(), t.mkeys.as<uint64_t>(), t.keysA.as<uint64_t>(), levels, passes,
+            sys && !full ? 1 : 0, t.hist.as<unsigned>());
+        LG_LAUNCHED();
+        e.launches += 2;
+        int at = sort_passes(e, t, n, passes, true);
+        if (full && sys) {
+            k_sys_keys<<<grid_for(n, BS), BS, 0, s>>>(sys, t.valsA.as<uint32_t>(), t.keysA.as<uint64_t>(), n);
+            LG_LAUNCHED();
+            ++e.launches;
+            sort_pairs(e, t, n, false);
+            at = 0;
+        }
+        const int other = e.cur ^ 1;
+        k_permute<<<grid_for(n_total, BS), BS, 0, s>>>(
+            e.bodies(e.cur), e.bodies(other), at ? t.keysB.as<uint64_t>() : t.keysA.as<uint64_t>(),
+            at ? t.valsB.as<uint32_t>() : t.valsA.as<uint32_t>(), t.mkeys.as<uint64_t>(), t.skey.as<uint64_t>(), nullptr,
+            nullptr, n, n_total, full ? 0 : 1, counts + 7);
         LG_LAUNCHED();
         ++e.launches;
-        sort_pairs(e, t, n);
+        e.cur = other;
+        if (full) {
+            // Key restarts (src/cpu_backend.cpp:536-544): runs of identical keys longer than a leaf.
+            // (A partial sort flags any run that long.)
+            t.runs.reserve(static_cast<size_t>(run_cap) * 8);
+            k_find_runs<<<grid_for(n, BS), BS, 0, s>>>(sys, t.skey.as<uint64_t>(), nullptr, nullptr, 1, n,
+                                                       t.runs.as<uint2>(), counts, run_cap);
+            LG_LAUNCHED();
+            ++e.launches;
+        }
+        // Key restarts are rare: unless the last build needed them, assume none and let the check
+        // after the walk (tree_verify) catch a miss; otherwise read the counts now.
+        t.speculative = t.have_guess && !t.restart_mode;
+        if (t.speculative) return;
+        LG_CK(cudaMemcpyAsync(e.pinned_small, counts, 32, cudaMemcpyDeviceToHost, s));
+        LG_CK(cudaStreamSynchronize(s));
+        R = e.pinned_small[0];
+        if (full || !e.pinned_small[7]) break;
+        t.sort_full = true;
     }
-    int other = e.cur ^ 1;
-    k_permute<<<grid_for(n_total, BS), BS, 0, s>>>(e.bodies(e.cur), e.bodies(other), t.keysA.as<uint64_t>(),
-                                                   t.valsA.as<uint32_t>(), t.skey.as<uint64_t>(), nullptr, nullptr, n,
-                                                   sys ? t.mkeys.as<uint64_t>() : nullptr, n_total);
-    LG_LAUNCHED();
-    ++e.launches;
-    e.cur = other;
-
-    // Key restarts (src/cpu_backend.cpp:536-544): runs of identical keys longer than a leaf.
-    unsigned* counts = t.counts.as<unsigned>();
-    LG_CK(cudaMemsetAsync(counts, 0, 64, s));
-    const int run_cap = std::max(1, n / (LEAF_MAX + 1) + 1);  // runs hold more than LEAF_MAX bodies each
-    t.runs.reserve(static_cast<size_t>(run_cap) * 8);
-    k_find_runs<<<grid_for(n, BS), BS, 0, s>>>(sys, t.skey.as<uint64_t>(), nullptr, nullptr, 1, n, t.runs.as<uint2>(),
-                                               counts, run_cap);
-    LG_LAUNCHED();
-    ++e.launches;
-    // Key restarts are rare: unless the last build needed them, assume none and let the check after
-    // the walk (tree_verify) catch a miss; otherwise read the run count now.
-    t.speculative = t.have_guess && !t.restart_mode;
-    if (t.speculative) return;
-    LG_CK(cudaMemcpyAsync(e.pinned_small, counts, 4, cudaMemcpyDeviceToHost, s));
-    LG_CK(cudaStreamSynchronize(s));
     // Runs are disjoint and longer than LEAF_MAX, so there are fewer than run_cap.
-    unsigned R = std::min(e.pinned_small[0], static_cast<unsigned>(run_cap));
+    R = std::min(R, static_cast<unsigned>(run_cap));
     t.restart_mode = R > 0;
     if (R == 0) return;
     t.restarted = true;
@@ -1567,17 +1631,15 @@ void tree_sort(Engine& e) {
         k_run_keys<<<R, BS, 0, s>>>(b, t.runs.as<uint2>(), t.fcube[f].as<double>(), key1, runid, nfr, f);
         LG_LAUNCHED();
         LG_CK(cudaMemcpyAsync(t.keysA.as<uint64_t>(), key1, static_cast<size_t>(n) * 8, cudaMemcpyDeviceToDevice, s));
-        k_iota<<<grid_for(n, BS), BS, 0, s>>>(t.valsA.as<uint32_t>(), n);
-        LG_LAUNCHED();
-        sort_pairs(e, t, n);
+        sort_pairs(e, t, n, true);
         k_seg_keys<<<grid_for(n, BS), BS, 0, s>>>(t.valsA.as<uint32_t>(), runid, t.runs.as<uint2>(),
                                                   t.keysA.as<uint64_t>(), n);
         LG_LAUNCHED();
-        sort_pairs(e, t, n);
+        sort_pairs(e, t, n, false);
         const int other = e.cur ^ 1;
         k_permute<<<grid_for(n_total, BS), BS, 0, s>>>(e.bodies(e.cur), e.bodies(other), t.keysA.as<uint64_t>(),
-                                                       t.valsA.as<uint32_t>(), nullptr, key1, t.fkey[f].as<uint64_t>(), n,
-                                                       nullptr, n_total);
+                                                       t.valsA.as<uint32_t>(), nullptr, nullptr, key1,
+                                                       t.fkey[f].as<uint64_t>(), n, n_total, 0, nullptr);
         LG_LAUNCHED();
         e.cur = other;
         ft.key[f] = t.fkey[f].as<uint64_t>();
@@ -1587,7 +1649,7 @@ void tree_sort(Engine& e) {
         t.nframes = f + 1;
         k_put_table<<<1, 1, 0, s>>>(ft, t.ftab.as<FrameTable>());
         LG_LAUNCHED();
-        e.launches += 8;
+        e.launches += 7;
         if (f + 1 == FRAMES) break;  // runs left now stay leaves at depth MAX_DEPTH
         // The next frame's runs: bodies re-keyed in this frame whose composite keys still tie.
         LG_CK(cudaMemsetAsync(counts + 6, 0, 4, s));
@@ -1803,9 +1865,11 @@ bool tree_verify(Engine& e, const unsigned* counts_host) {
     if (!t.speculative) return true;
     const unsigned R = counts_host[0], K = counts_host[1], T = counts_host[2];
     const int depth = static_cast<int>(counts_host[4]);
-    const bool ok = (t.restarted || R == 0) && K <= t.K && T <= t.T && depth <= t.max_depth;
+    const bool long_run = counts_host[7] != 0;  // the tree is deeper than the digits sorted
+    const bool ok = (t.restarted || R == 0) && K <= t.K && T <= t.T && depth <= t.max_depth && !long_run;
     if (!ok) {
         if (!t.restarted && R > 0) t.restart_mode = true;
+        if (long_run) t.sort_full = true;
         t.have_guess = false;  // next build reads exact sizes
     }
     return ok;
@@ -1819,7 +1883,7 @@ namespace {
 __global__ void k_tree_check(const unsigned* __restrict__ counts, unsigned K, unsigned T, int depth, int restarted,
                              unsigned* sticky) {
     const bool ok = (restarted || counts[0] == 0) && counts[1] <= K && counts[2] <= T &&
-                    static_cast<int>(counts[4]) <= depth;
+                    static_cast<int>(counts[4]) <= depth && counts[7] == 0;
     if (!ok) atomicOr(sticky, 1u);
 }
 }  // namespace
@@ -1834,6 +1898,7 @@ void tree_set_forest(Engine& e, int n_tree, int nsys, const uint32_t* sys, const
     t.inv_theta_sys = inv_theta_sys;
     t.have_guess = false;
     t.restart_mode = false;
+    t.sort_full = false;
 }
 
 bool tree_sync_free_ready(const Engine& e) { return e.tree->have_guess && !e.tree->restart_mode; }
@@ -1850,6 +1915,10 @@ void tree_check_async(Engine& e, unsigned* sticky) {
 void tree_reset_guess(Engine& e) {
     e.tree->have_guess = false;
     e.tree->restart_mode = false;
+}
+void tree_reset(Engine& e) {
+    tree_reset_guess(e);
+    e.tree->sort_full = false;
 }
 double tree_theta(const Engine& e) { return e.tree->theta; }
 
@@ -1966,7 +2035,7 @@ lg_memory_estimate memory_need(uint64_t n, int method) {
 size_t tree_held_bytes(const Engine& e) {
     const TreeState& t = *e.tree;
     size_t h = 0;
-    for (const DevBuf* d : {&t.keysA, &t.keysB, &t.valsA, &t.valsB, &t.hist, &t.lookback, &t.ctl, &t.skey, &t.key1tmp,
+    for (const DevBuf* d : {&t.keysA, &t.keysB, &t.valsA, &t.valsB, &t.hist, &t.lookback, &t.mkeys, &t.skey, &t.key1tmp,
                             &t.nfr, &t.ftab, &t.bdepth, &t.flag, &t.leafid, &t.frame, &t.runs, &t.counts,
                             &t.leaf_first, &t.leaf_depth, &t.leaf_c, &t.leaf_pre, &t.leaf_node, &t.pn_lohi,
                             &t.pn_meta, &t.pn_nchild, &t.pn_cb, &t.pn_cpu, &t.nd_test, &t.nd_cell, &t.nd_geo, &t.nd_parent, &t.gflag, &t.gidx, &t.grp_node, &t.leaf_cnt, &t.ups, &t.dep_nodes, &t.leaf_order,
