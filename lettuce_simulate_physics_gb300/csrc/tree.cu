@@ -21,21 +21,26 @@
 //     runs whose composite keys still tie are re-keyed again, up to FRAMES frames (depth 126).
 //     Composite keys (frame 0, then the restart frames) order the bodies as the reference's nested
 //     rekeys do, and a common-prefix length over them drives steps 4-6.
-//  4. Leaves from key windows: body i's leaf depth is 1 + the deepest common octal prefix of any
-//     window of LEAF_MAX+1 consecutive sorted keys that contains i (the first depth at which its
-//     cell holds <= LEAF_MAX bodies); group depth likewise with windows of group_max+1.
-//  5. Octree nodes in pre-order, enumerated per leaf: leaf l owns the ancestors at depths
-//     c+1 .. depth-1, c = common prefix with the previous leaf (Karras 2012's adjacent-key rule in
-//     octree form). A scan gives every node's pre-order index; body ranges, parents and children
-//     follow from binary searches over the sorted keys.
-//  6. Node indices of the reference (children contiguous, child blocks in parent pre-order):
-//     first child of v = 1 + exclusive scan of nchild over pre-order.
+//  4. Leaves from key windows (k_leaves): body i's leaf depth is 1 + the deepest common octal prefix of
+//     any window of LEAF_MAX+1 consecutive sorted keys that contains i (the first depth at which its
+//     cell holds <= LEAF_MAX bodies); group depth likewise with windows of group_max+1. The same
+//     launch numbers the leaves and their nodes by one decoupled look-back.
+//  5. Octree nodes in pre-order (k_nodes): leaf l owns the ancestors at depths c+1 .. depth-1, c =
+//     common prefix with the previous leaf (Karras 2012's adjacent-key rule in octree form); body
+//     ranges and parents follow from searches over the sorted keys, and every node sets its octant's
+//     bit in its parent's child mask.
+//  6. Node indices of the reference (children contiguous, child blocks in parent pre-order): first
+//     child of v = 1 + exclusive scan of the masks' bit counts over pre-order (k_node_scan), a child's
+//     place under its parent the bits below its own (k_nodes_out).
 //  7. Upsweep in FP64, children always combined in index order: one launch for the leaves (one
-//     thread per leaf, leaves bucketed by body count), then one launch per depth from the deepest
-//     (four lanes per node, each sequential sum folded by one lane). The group boxes are computed
-//     on a side stream meanwhile. (A single-launch form in which the last-arriving child of each
-//     node combines it was measured slower: its combines run one node per thread in sparse warps,
-//     and an FP64 warp instruction costs the same however few lanes are active.)
+//     thread per leaf, leaves bucketed by body count), then the depths from the deepest (four lanes
+//     per node, each sequential sum folded by one lane), the narrow depths at the top together in
+//     one launch. The group boxes are computed on a side stream meanwhile. (A single-launch form in
+//     which the last-arriving child of each node combines it was measured slower: its combines run
+//     one node per thread in sparse warps, and an FP64 warp instruction costs the same however few
+//     lanes are active.)
+// Steps 4 to 6 are four launches (they were 22 with their scans, and 13 clears; build phase 238 ->
+// 146 us at 8191 bodies, 289 -> 200 at 1e5, 514 -> 385 on the 1e6 disk, 4.16 -> 3.26 ms at 1.6e7).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -90,7 +95,7 @@ struct ZeroSpan {
     uint4* p;
     size_t words;
 };
-constexpr int ZSPANS = 3;
+constexpr int ZSPANS = 4;
 struct ZeroList {
     ZeroSpan span[ZSPANS];
 };
@@ -102,22 +107,22 @@ struct TreeState {
     DevBuf keysA, keysB, valsA, valsB, hist, lookback;
     bool sort_full = false;  // a partial sort met a run too long to order locally: all key bits from now on
     // sorted frame-0 keys, per-body tree data
-    DevBuf skey, bdepth, flag, leafid;
+    DevBuf skey, leafid;
     // frame, key-restart runs and frames (index 0 of the per-frame buffers unused)
     DevBuf frame, runs, counts, key1tmp, nfr, ftab;
     DevBuf fkey[FRAMES], frunid[FRAMES], fcube[FRAMES];
     int nframes = 1;  // key frames of the last restarted build
     // leaves
-    DevBuf leaf_first, leaf_depth, leaf_c, leaf_pre, leaf_node;
+    DevBuf leaf_first, leaf_depth, leaf_gdepth, leaf_c, leaf_pre, leaf_node, leaf_state;
     // pre-order nodes
-    DevBuf pn_lohi, pn_meta, pn_nchild, pn_cb, pn_cpu;
+    DevBuf pn_lohi, pn_meta, pn_parent, pn_first, node_zero;
     // reference-order nodes
     DevBuf nd_test, nd_cell, nd_geo, nd_parent;
     // groups
-    DevBuf gflag, gidx, grp_node, grp_range, grp_box, grp_order, grp_class, leaf_cnt;
+    DevBuf grp_node, grp_range, grp_box, grp_order;
     // upsweep order
-    DevBuf ups, dep_nodes, leaf_order;
-    // scan state
+    DevBuf dep_nodes, leaf_order;
+    // scan state (merged walk groups)
     DevBuf scan_state, scan_ctr;
     size_t K = 0, T = 0, ngroups = 0;  // sizes the last build was launched with
     int max_depth = 0;
@@ -766,70 +771,202 @@ __global__ void k_fill_i32(int* a, int v, int n) {
 }
 
 // ---- leaves ----------------------------------------------------------------------------------
-// Per body: leaf depth and group depth from window common prefixes, capped at 21 times the frames
-// the body has keys in. bdepth packs (leaf depth, group depth) as bytes.
-// Each block handles DEPTH_BS bodies: it first forms, in shared memory, the common prefixes
-// c_w(j) = cpl(key j, key j+w) of every window start its bodies need (w = 16 and w = group_max),
-// then every thread takes the maxima over its windows from shared memory.
-constexpr int DEPTH_BS = 256;
-constexpr int GMAX_LIMIT = 1024;
+// One decoupled look-back over the sorted bodies gives the leaves and their nodes: leaf depths, leaf
+// starts, every leaf's index, range and first pre-order node, in one launch. (As depth, flag, scan,
+// information, index and second-scan launches with their clears it was 13 operations.) Latency
+// bound below 1e5 bodies; at 1e6 it reads the keys once and writes 4 bytes a body and 14 a leaf.
+//
+// Exclusive prefix of the tile from its predecessors' published sums (one warp, 32 predecessors a
+// round trip): state words carry a flag (SFLAG_AGG: the tile's own sum, SFLAG_INC: the sum up to and
+// including it) over two 31-bit sums.
+constexpr unsigned long long TWO31 = (1ull << 31) - 1;
+__device__ unsigned long long look_back(volatile unsigned long long* state, int tile, int lane, unsigned* err) {
+    unsigned long long prefix = 0;
+    unsigned spins = 0;
+    for (int j = tile - 1; j >= 0; j -= 32) {
+        unsigned long long v;
+        unsigned inc, need;
+        for (;;) {
+            v = j - lane >= 0 ? state[j - lane] : static_cast<unsigned long long>(SFLAG_INC);
+            inc = __ballot_sync(0xffffffffu, (v & SFLAG_INC) != 0);
+            // The predecessors needed: up to the nearest inclusive one, or all 32.
+            need = inc ? (inc & (0u - inc)) * 2u - 1u : 0xffffffffu;
+            if (!(~__ballot_sync(0xffffffffu, (v & (SFLAG_INC | SFLAG_AGG)) != 0) & need)) break;
+            if (++spins > kSpinCap) {
+                if (lane == 0) atomicOr(err, kErrWaitTimeout);
+                break;
+            }
+        }
+        unsigned long long add = (need >> lane) & 1u ? v & SVAL : 0ull;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+        prefix += add;
+        if (inc) break;
+    }
+    return prefix;
+}
 
-__global__ void __launch_bounds__(DEPTH_BS) k_body_depth(const uint32_t* __restrict__ sys, const uint64_t* __restrict__ k0,
-                                                         const FrameTable* ft, int n, int gmax,
-                                                         uint16_t* __restrict__ bdepth) {
-    __shared__ int8_t c16[DEPTH_BS + LEAF_MAX];
-    __shared__ int8_t cg[DEPTH_BS + GMAX_LIMIT];
-    const int i0 = blockIdx.x * DEPTH_BS;
-    // Window starts j in [i0 - w, i0 + DEPTH_BS): slot j - (i0 - w).
-    for (int t = threadIdx.x; t < DEPTH_BS + LEAF_MAX; t += DEPTH_BS) {
+// Block-wide exclusive prefix of v (two 31-bit sums), the tiles before it included; *total: the sum
+// up to and including the tile. warp_sum, tile_prefix: shared scratch. All threads of the block.
+template <int THREADS>
+__device__ __forceinline__ unsigned long long tile_scan(unsigned long long v, int tile, volatile unsigned long long* state,
+                                                        unsigned long long* warp_sum, unsigned long long* tile_prefix,
+                                                        unsigned long long* total, unsigned* err) {
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    unsigned long long incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) warp_sum[w] = incl;
+    __syncthreads();
+    if (w == 0) {
+        unsigned long long sum = 0;
+#pragma unroll
+        for (int u = 0; u < THREADS / 32; ++u) sum += warp_sum[u];
+        if (lane == 0) state[tile] = (tile == 0 ? SFLAG_INC : SFLAG_AGG) | sum;
+        const unsigned long long prefix = look_back(state, tile, lane, err);
+        if (lane == 0) {
+            if (tile) state[tile] = SFLAG_INC | ((prefix + sum) & SVAL);
+            *tile_prefix = prefix;
+        }
+    }
+    __syncthreads();
+    unsigned long long before = *tile_prefix, sum = 0;
+#pragma unroll
+    for (int u = 0; u < THREADS / 32; ++u) {
+        if (u < w) before += warp_sum[u];
+        sum += warp_sum[u];
+    }
+    *total = *tile_prefix + sum;
+    return before + incl - v;
+}
+
+constexpr int GMAX_LIMIT = 1024;
+constexpr int LEAF_BS = 256, LEAF_IPT = 4, LEAF_TILE = LEAF_BS * LEAF_IPT;
+inline int leaf_tiles(int n) { return grid_for(n, LEAF_TILE); }
+
+// counts[1], counts[2]: leaves, nodes; counts[4]: deepest leaf; counts[8]: 1 if they fit Kcap and Tcap
+// and the bodies are sorted (no long run flagged): what follows runs only then.
+struct LeafOut {
+    uint32_t* lid;         // per body: its leaf
+    uint32_t* first;       // per leaf: first body (one past the last leaf: n)
+    uint32_t* pre;         // per leaf: pre-order index of the first node it owns (one past: node count)
+    uint8_t *depth, *gdepth;  // per leaf: its depth, the depth of its walk group
+    int8_t* c;             // per leaf: common octal prefix with the body before it (-1: none)
+};
+
+// Maximum of `count` consecutive values from every place, by doubling: on return v[t] holds the
+// maximum of v[t .. t + 2^p), 2^p the largest power of two up to count.
+__device__ __forceinline__ int window_max(int8_t* v, int size, int count) {
+    int p = 1;
+    for (; 2 * p <= count; p *= 2) {
+        constexpr int PER = (LEAF_TILE + 1 + GMAX_LIMIT + LEAF_BS - 1) / LEAF_BS;
+        int8_t r[PER];
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int t = threadIdx.x + q * LEAF_BS;
+            if (t < size) r[q] = t + p < size ? max(v[t], v[t + p]) : v[t];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int t = threadIdx.x + q * LEAF_BS;
+            if (t < size) v[t] = r[q];
+        }
+        __syncthreads();
+    }
+    return p;
+}
+
+__global__ void __launch_bounds__(LEAF_BS) k_leaves(const uint32_t* __restrict__ sys, const uint64_t* __restrict__ k0,
+                                                    const FrameTable* ft, int n, int gmax, LeafOut out,
+                                                    unsigned long long* state, unsigned* tile_ctr, unsigned* counts,
+                                                    unsigned Kcap, unsigned Tcap, ZeroList z, unsigned* err) {
+    // Common prefixes of every window of LEAF_MAX + 1 and of gmax + 1 sorted keys that holds one of
+    // the tile's bodies or the one before them; then their maxima over a body's windows.
+    __shared__ int8_t c16[LEAF_TILE + 1 + LEAF_MAX];
+    __shared__ int8_t cg[LEAF_TILE + 1 + GMAX_LIMIT];
+    __shared__ unsigned long long warp_sum[LEAF_BS / 32], prefix_s;
+    __shared__ unsigned tile_s;
+    zero_spans(z);
+    const int tid = threadIdx.x;
+    if (tid == 0) tile_s = atomicAdd(tile_ctr, 1u);
+    __syncthreads();
+    const int tile = static_cast<int>(tile_s), i0 = tile * LEAF_TILE - 1;  // slot q stands for body i0 + q
+    for (int t = tid; t < LEAF_TILE + 1 + LEAF_MAX; t += LEAF_BS) {
         const int j = i0 - LEAF_MAX + t;
         c16[t] = static_cast<int8_t>((j >= 0 && j + LEAF_MAX < n) ? cpl_key(sys, k0, ft, j, j + LEAF_MAX) : -1);
     }
-    for (int t = threadIdx.x; t < DEPTH_BS + gmax; t += DEPTH_BS) {
+    for (int t = tid; t < LEAF_TILE + 1 + gmax; t += LEAF_BS) {
         const int j = i0 - gmax + t;
         cg[t] = static_cast<int8_t>((j >= 0 && j + gmax < n) ? cpl_key(sys, k0, ft, j, j + gmax) : -1);
     }
     __syncthreads();
-    const int i = i0 + threadIdx.x;
-    if (i >= n) return;
-    // Windows containing i start at j in [i - w, i], i.e. slots [threadIdx.x, threadIdx.x + w].
-    int best = -1;
-    for (int t = threadIdx.x; t <= threadIdx.x + LEAF_MAX; ++t) best = max(best, static_cast<int>(c16[t]));
+    const int p16 = window_max(c16, LEAF_TILE + 1 + LEAF_MAX, LEAF_MAX + 1);
+    const int pg = window_max(cg, LEAF_TILE + 1 + gmax, gmax + 1);
+    // The windows that hold slot q's body start in slots q .. q + w (w the window's length less one).
     // A body's keys end with the last frame it was re-keyed in: coincident bodies, and bodies of a
     // run past the last frame, stay one leaf there.
-    const int cap = ft ? MAX_LEVEL * ft->nfr[i] : MAX_LEVEL;
-    const int ld = min(best + 1, cap);
-    int gbest = -1;
-    for (int t = threadIdx.x; t <= threadIdx.x + gmax; ++t) gbest = max(gbest, static_cast<int>(cg[t]));
-    const int gd = min(ld, gbest + 1);
-    bdepth[i] = static_cast<uint16_t>(ld | (gd << 8));
-}
-
-__global__ void k_leaf_flags(const uint32_t* __restrict__ sys, const uint64_t* __restrict__ k0, const FrameTable* ft,
-                             const uint16_t* __restrict__ bdepth, int n, uint32_t* __restrict__ flag) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int d = bdepth[i] & 255;
-    uint32_t f = 1;
-    if (i > 0 && (bdepth[i - 1] & 255) == d && cpl_key(sys, k0, ft, i - 1, i) >= d) f = 0;
-    flag[i] = f;
-}
-
-// leaf_first, leaf_depth, leaf_c, and the node count of each leaf (its owned ancestors + itself).
-__global__ void k_leaf_info(const uint32_t* __restrict__ sys, const uint64_t* __restrict__ k0, const FrameTable* ft,
-                            const uint16_t* __restrict__ bdepth, const uint32_t* __restrict__ flag,
-                            const uint32_t* __restrict__ lid, int n, uint32_t* leaf_first, uint8_t* leaf_depth,
-                            int8_t* leaf_c, uint32_t* leaf_nodes, int* max_depth) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !flag[i]) return;
-    const uint32_t l = lid[i];
-    const int d = bdepth[i] & 255;
-    atomicMax(max_depth, d);
-    const int c = i == 0 ? -1 : cpl_key(sys, k0, ft, i - 1, i);
-    leaf_first[l] = static_cast<uint32_t>(i);
-    leaf_depth[l] = static_cast<uint8_t>(d);
-    leaf_c[l] = static_cast<int8_t>(c);
-    leaf_nodes[l] = static_cast<uint32_t>(d - 1 - c + 1);
+    auto leaf_depth = [&](int q, int i) {
+        const int best = max(c16[q], c16[q + LEAF_MAX + 1 - p16]);
+        return min(best + 1, ft ? MAX_LEVEL * ft->nfr[i] : MAX_LEVEL);
+    };
+    int depth[LEAF_IPT], c[LEAF_IPT];
+    bool flag[LEAF_IPT];
+    unsigned long long mine = 0;
+    int deepest = 0;
+    const int q0 = 1 + tid * LEAF_IPT;
+    int before = i0 + q0 > 0 && i0 + q0 <= n ? leaf_depth(q0 - 1, i0 + q0 - 1) : -1;
+#pragma unroll
+    for (int u = 0; u < LEAF_IPT; ++u) {
+        const int q = q0 + u, i = i0 + q;
+        flag[u] = false;
+        depth[u] = c[u] = -1;
+        if (i < n) {
+            depth[u] = leaf_depth(q, i);
+            c[u] = i > 0 ? cpl_key(sys, k0, ft, i - 1, i) : -1;
+            flag[u] = i == 0 || before != depth[u] || c[u] < depth[u];
+            before = depth[u];
+            if (flag[u]) {
+                // The leaf owns its ancestors at depths c + 1 .. depth - 1, and itself.
+                mine += 1ull + (static_cast<unsigned long long>(depth[u] - c[u]) << 31);
+                deepest = max(deepest, depth[u]);
+            }
+        }
+    }
+    deepest = __reduce_max_sync(0xffffffffu, deepest);
+    if ((tid & 31) == 0) atomicMax(reinterpret_cast<int*>(counts + 4), deepest);
+    unsigned long long total;
+    const unsigned long long at = tile_scan<LEAF_BS>(mine, tile, state, warp_sum, &prefix_s, &total, err);
+    uint32_t l = static_cast<uint32_t>(at & TWO31), pre = static_cast<uint32_t>(at >> 31);
+#pragma unroll
+    for (int u = 0; u < LEAF_IPT; ++u) {
+        const int q = q0 + u, i = i0 + q;
+        if (i >= n) break;
+        if (flag[u]) {
+            const int gbest = max(cg[q], cg[q + gmax + 1 - pg]);
+            out.first[l] = static_cast<uint32_t>(i);
+            out.pre[l] = pre;
+            out.depth[l] = static_cast<uint8_t>(depth[u]);
+            out.gdepth[l] = static_cast<uint8_t>(min(depth[u], gbest + 1));
+            out.c[l] = static_cast<int8_t>(c[u]);
+            ++l;
+            pre += static_cast<uint32_t>(depth[u] - c[u]);
+        }
+        out.lid[i] = l - 1;
+    }
+    if (tile == (n + LEAF_TILE - 1) / LEAF_TILE - 1 && tid == 0) {
+        const unsigned K = static_cast<unsigned>(total & TWO31), T = static_cast<unsigned>(total >> 31);
+        if (K <= static_cast<unsigned>(n)) {
+            out.first[K] = static_cast<uint32_t>(n);
+            out.pre[K] = T;
+        }
+        counts[1] = K;
+        counts[2] = T;
+        counts[8] = K <= Kcap && T <= Tcap && counts[7] == 0 ? 1u : 0u;
+    }
 }
 
 // ---- nodes -----------------------------------------------------------------------------------
@@ -837,100 +974,195 @@ struct NodeCtx {
     const uint32_t* sys;  // per-body system (forest) or null
     const uint64_t* k0;          // sorted frame-0 keys
     const FrameTable* ft;        // key restart frames, or null
-    const uint32_t* leaf_first;  // K+1
-    const uint8_t* leaf_depth;
-    const int8_t* leaf_c;
-    const uint32_t* leaf_pre;    // K+1
-    const uint32_t* lid;         // per body
-    const uint16_t* bdepth;
+    LeafOut leaf;
     int n;
-    const unsigned* Kdev;  // leaf count (device)
-    unsigned Kcap;         // capacity the leaf arrays were sized for
+    const unsigned* counts;
     unsigned nroots;       // systems in the forest (1 for one system); roots take node indices 0..nroots-1
 };
 
-__device__ __forceinline__ int leaf_count(const NodeCtx& c) { return static_cast<int>(min(*c.Kdev, c.Kcap)); }
-__device__ __forceinline__ uint32_t eff(const unsigned* dev, uint32_t cap) { return min(*dev, cap); }
+// Whether the leaves are there and fit what the build was launched for, and their number and the nodes'.
+__device__ __forceinline__ bool build_ok(const unsigned* counts) { return counts[8] != 0; }
 
-// Pre-order index of the node at depth d whose first body is b (b must start that node).
-__device__ __forceinline__ uint32_t node_at(const NodeCtx& c, uint32_t b, int d) {
-    const uint32_t l = c.lid[b];
-    return c.leaf_pre[l] + static_cast<uint32_t>(d - c.leaf_c[l] - 1);
-}
+// Pre-order nodes as k_nodes leaves them. meta: depth | leaf << 8 | group << 9 | octal digit under
+// the parent << 10; mask (zero before): which of a node's eight octants have a child; first: its
+// first child in the reference's numbering (k_node_scan).
+struct PreNodes {
+    uint2* lohi;
+    uint16_t* meta;
+    uint32_t* parent;  // pre-order index, 0xffffffff for a root
+    uint32_t* mask;
+    uint32_t* first;
+};
 
-// End of the body range sharing `d` octal digits with body lo.
-__device__ __forceinline__ uint32_t range_end(const NodeCtx& c, uint32_t lo, int d) {
-    uint32_t a = lo + 1, b = static_cast<uint32_t>(c.n);
-    while (a < b) {
-        uint32_t mid = (a + b) >> 1;
-        if (cpl_key(c.sys, c.k0, c.ft, lo, mid) >= d) a = mid + 1;
-        else b = mid;
+// The last index in [a, end) for which share(index) holds, known to hold at a and to hold on a
+// leading part of the range: probes at growing powers of eight, then seven probes a round, all
+// loads of a round in flight together. A search costs two or three rounds for a small node and
+// about fourteen for the root of 1e6 bodies (forty dependent loads by bisection).
+template <class F>
+__device__ __forceinline__ int last_sharing(int a, int end, F&& share) {
+    long long step = 1;
+    int hi = end;  // first index known not to share (or the end)
+    for (;; step *= 8) {
+        const long long probe = a + step;
+        if (probe >= end) break;
+        if (!share(static_cast<int>(probe))) {
+            hi = static_cast<int>(probe);
+            break;
+        }
+        a = static_cast<int>(probe);
+    }
+    while (hi - a > 1) {
+        const int gap = max(1, (hi - a + 7) / 8);
+        int na = a, nhi = hi;
+        bool ok[7];
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+            const int m = a + (q + 1) * gap;
+            ok[q] = m < hi && share(m);
+        }
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+            const int m = a + (q + 1) * gap;
+            if (m < hi) {
+                if (ok[q]) na = m;
+                else nhi = min(nhi, m);
+            }
+        }
+        a = na;
+        hi = nhi;
     }
     return a;
 }
 
-// Per pre-order node: (lo, hi) and meta = depth | leaf << 8 | group << 9.
-__global__ void k_nodes_pre(NodeCtx c, uint32_t Tcap, const unsigned* Tdev, uint2* pn_lohi, uint16_t* pn_meta) {
-    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= eff(Tdev, Tcap)) return;
-    // Leaf owning v: last l with leaf_pre[l] <= v.
-    int a = 0, b = leaf_count(c);
+// Ranges, flags and parents of the pre-order nodes (one thread per node), and the parents' child
+// masks. Leaf l owns nodes pre[l] .. pre[l + 1) - 1, at depths c[l] + 1 .. depth[l]; the parent of a
+// node that is not its leaf's first is the node before it, that of a first node the node at depth
+// c[l] that also holds the body before the leaf.
+constexpr int NODE_BS = 256;
+__global__ void __launch_bounds__(NODE_BS) k_nodes(NodeCtx x, PreNodes pn) {
+    __shared__ int l_first;
+    if (!build_ok(x.counts)) return;
+    const uint32_t T = x.counts[2];
+    const int K = static_cast<int>(x.counts[1]);
+    const uint32_t v0 = blockIdx.x * NODE_BS;
+    if (v0 >= T) return;
+    if (threadIdx.x < 32) {  // the leaf that owns the block's first node: 32 probes a round
+        int a = 0, b = K;    // pre[a] <= v0 < pre[b]
+        while (b - a > 1) {
+            const int gap = max(1, (b - a + 32) / 33);
+            const int m = a + (static_cast<int>(threadIdx.x) + 1) * gap;
+            const unsigned le = __ballot_sync(0xffffffffu, m < b && x.leaf.pre[m] <= v0);
+            const int k = __popc(le);  // the probes that hold are the first ones
+            b = min(b, a + (k + 1) * gap);
+            a += k * gap;
+        }
+        if (threadIdx.x == 0) l_first = a;
+    }
+    __syncthreads();
+    const uint32_t v = v0 + threadIdx.x;
+    if (v >= T) return;
+    // A block's nodes belong to at most NODE_BS leaves from the first.
+    int a = l_first, b = min(K, l_first + NODE_BS);
     while (b - a > 1) {
-        int mid = (a + b) >> 1;
-        if (c.leaf_pre[mid] <= v) a = mid;
-        else b = mid;
+        const int m = (a + b) >> 1;
+        if (x.leaf.pre[m] <= v) a = m;
+        else b = m;
     }
-    const int l = a;
-    const int d = c.leaf_c[l] + 1 + static_cast<int>(v - c.leaf_pre[l]);
-    const bool leaf = d == c.leaf_depth[l];
-    const uint32_t lo = c.leaf_first[l];
-    const uint32_t hi = leaf ? c.leaf_first[l + 1] : range_end(c, lo, d);
-    const bool group = d == (c.bdepth[lo] >> 8);
-    pn_lohi[v] = make_uint2(lo, hi);
-    pn_meta[v] = static_cast<uint16_t>(d | (leaf ? 256 : 0) | (group ? 512 : 0));
+    const int l = a, c = x.leaf.c[l], d = c + 1 + static_cast<int>(v - x.leaf.pre[l]);
+    const bool leaf = d == x.leaf.depth[l];
+    const int lo = static_cast<int>(x.leaf.first[l]), lend = static_cast<int>(x.leaf.first[l + 1]);
+    int hi = lend;
+    if (!leaf) hi = 1 + last_sharing(lend - 1, x.n, [&](int j) { return cpl_key(x.sys, x.k0, x.ft, lo, j) >= d; });
+    uint32_t parent = 0xffffffffu;
+    int digit = 0;
+    if (d > 0) {
+        digit = digit_at(x.k0, x.ft, lo, d);
+        if (d > c + 1) {
+            parent = v - 1;
+        } else {
+            // Mirrored: the place lo - 1 - j shares c digits with lo for j from 0 to the answer.
+            const int back = last_sharing(0, lo, [&](int j) { return cpl_key(x.sys, x.k0, x.ft, lo - 1 - j, lo) >= c; });
+            const uint32_t pl = x.leaf.lid[lo - 1 - back];
+            parent = x.leaf.pre[pl] + static_cast<uint32_t>(c - x.leaf.c[pl] - 1);
+        }
+        if (parent < T) atomicOr(&pn.mask[parent], 1u << digit);
+    }
+    pn.lohi[v] = make_uint2(static_cast<uint32_t>(lo), static_cast<uint32_t>(hi));
+    pn.meta[v] = static_cast<uint16_t>(d | (leaf ? 256 : 0) | (d == x.leaf.gdepth[l] ? 512 : 0) | digit << 10);
+    pn.parent[v] = parent;
 }
 
-// Children of internal pre-order node v, in order; returns the count.
-template <class F>
-__device__ __forceinline__ int for_children(const NodeCtx& c, const uint2* pn_lohi, uint32_t v, int d, F&& f) {
-    const uint2 r = pn_lohi[v];
-    uint32_t b = r.x;
-    int k = 0;
-    // An octree node has at most 8 children; the cap keeps a malformed range from looping.
-    while (b < r.y && k < 8) {
-        const uint32_t ch = node_at(c, b, d + 1);
-        f(k, ch);
-        const uint32_t nb = pn_lohi[ch].y;
-        if (nb <= b) break;
-        b = nb;
-        ++k;
-    }
-    return k;
+// Upsweep bookkeeping: internal nodes bucketed by depth, leaves bucketed by body count.
+constexpr int NDEP = MAX_DEPTH + 2;  // depth buckets (depth <= MAX_DEPTH + 1 with headroom)
+constexpr int NLSZ = 18;   // leaf-size buckets: 1..16, then larger
+constexpr int NBUCKET = NDEP + NLSZ;
+struct UpsweepIndex {
+    unsigned count[NBUCKET];  // depths, then leaf sizes
+    unsigned cur[NBUCKET];
+    unsigned off[NBUCKET + 1];  // where a bucket starts in its list (written by k_nodes_out)
+};
+
+__device__ __forceinline__ int bucket_of(uint16_t meta, uint2 r) {
+    return meta & 256 ? NDEP + static_cast<int>(min(r.y - r.x, 17u)) : meta & 255;
 }
 
-__global__ void k_nchild(NodeCtx c, uint32_t Tcap, const unsigned* Tdev, const uint2* pn_lohi, const uint16_t* pn_meta,
-                         uint32_t* pn_nchild) {
-    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= Tcap) return;
-    if (v >= eff(Tdev, Tcap)) {
-        pn_nchild[v] = 0;  // scanned over the capacity
-        return;
+// One scan over the pre-order nodes: the first child of every node in the reference's numbering (child
+// blocks in parent pre-order, after the roots), the walk groups' nodes in order (counts[3] their
+// number), and the bucket counts of the upsweep.
+constexpr int NSCAN_BS = 256, NSCAN_IPT = 4, NSCAN_TILE = NSCAN_BS * NSCAN_IPT;
+__global__ void __launch_bounds__(NSCAN_BS) k_node_scan(NodeCtx x, PreNodes pn, unsigned long long* state,
+                                                        unsigned* tile_ctr, unsigned* counts, UpsweepIndex* ix,
+                                                        uint32_t* grp_node, unsigned* err) {
+    __shared__ unsigned long long warp_sum[NSCAN_BS / 32], prefix_s;
+    __shared__ unsigned tile_s, bucket[NBUCKET];
+    if (!build_ok(x.counts)) return;
+    const uint32_t T = x.counts[2];
+    const int tid = threadIdx.x;
+    if (tid == 0) tile_s = atomicAdd(tile_ctr, 1u);
+    if (tid < NBUCKET) bucket[tid] = 0;
+    __syncthreads();
+    const int tile = static_cast<int>(tile_s);
+    const uint32_t v0 = static_cast<uint32_t>(tile) * NSCAN_TILE + tid * NSCAN_IPT;
+    if (static_cast<uint32_t>(tile) * NSCAN_TILE >= T) return;  // past the last tile: nobody waits for it
+    unsigned long long mine = 0;
+    unsigned nch[NSCAN_IPT];
+    bool group[NSCAN_IPT];
+#pragma unroll
+    for (int u = 0; u < NSCAN_IPT; ++u) {
+        const uint32_t v = v0 + u;
+        nch[u] = 0;
+        group[u] = false;
+        if (v < T) {
+            const uint16_t meta = pn.meta[v];
+            nch[u] = __popc(pn.mask[v]);
+            group[u] = (meta & 512) != 0;
+            atomicAdd(&bucket[bucket_of(meta, pn.lohi[v])], 1u);
+            mine += nch[u] + (group[u] ? 1ull << 31 : 0ull);
+        }
     }
-    const uint16_t meta = pn_meta[v];
-    int k = 0;
-    if (!(meta & 256)) k = for_children(c, pn_lohi, v, meta & 255, [](int, uint32_t) {});
-    pn_nchild[v] = static_cast<uint32_t>(k);
+    unsigned long long total;
+    const unsigned long long at = tile_scan<NSCAN_BS>(mine, tile, state, warp_sum, &prefix_s, &total, err);
+    uint32_t first = x.nroots + static_cast<uint32_t>(at & TWO31), g = static_cast<uint32_t>(at >> 31);
+#pragma unroll
+    for (int u = 0; u < NSCAN_IPT; ++u) {
+        const uint32_t v = v0 + u;
+        if (v >= T) break;
+        pn.first[v] = first;
+        first += nch[u];
+        if (group[u]) {
+            if (g < T) grp_node[g] = v;
+            ++g;
+        }
+    }
+    if (tid < NBUCKET && bucket[tid]) atomicAdd(&ix->count[tid], bucket[tid]);
+    if (v0 < T && T <= v0 + NSCAN_IPT) counts[3] = min(static_cast<uint32_t>(total >> 31), T);
 }
 
-__global__ void k_cpu_index(NodeCtx c, uint32_t Tcap, const unsigned* Tdev, const uint2* pn_lohi,
-                            const uint16_t* pn_meta, const uint32_t* pn_cb, uint32_t* pn_cpu) {
-    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= eff(Tdev, Tcap)) return;
-    const uint16_t meta = pn_meta[v];
-    if ((meta & 255) == 0) pn_cpu[v] = sys_of(c.sys, static_cast<int>(pn_lohi[v].x));  // a system's root
-    if (meta & 256) return;
-    const uint32_t first = c.nroots + pn_cb[v];
-    for_children(c, pn_lohi, v, meta & 255, [&](int k, uint32_t ch) { pn_cpu[ch] = first + k; });
+// A pre-order node's index in the reference's numbering.
+__device__ __forceinline__ uint32_t ref_index(const NodeCtx& x, const PreNodes& pn, uint32_t v, uint16_t meta, uint32_t lo,
+                                              uint32_t parent) {
+    if ((meta & 255) == 0) return sys_of(x.sys, static_cast<int>(lo));  // a system's root
+    return pn.first[parent] + __popc(pn.mask[parent] & ((1u << (meta >> 10)) - 1u));
 }
 
 // Geometric centre (FP64, the reference's iterative halving, src/cpu_backend.cpp:575-582 and
@@ -961,44 +1193,82 @@ __device__ void node_geo(const NodeCtx& c, const double* frame, uint32_t b, int 
     }
 }
 
-__global__ void k_nodes_out(NodeCtx c, uint32_t Tcap, const unsigned* Tdev, const uint2* pn_lohi, const uint16_t* pn_meta,
-                            const uint32_t* pn_nchild, const uint32_t* pn_cb, const uint32_t* pn_cpu,
-                            const double* frame, NodeTest* nd_test,
-                            float4* nd_geo, uint32_t* nd_parent, uint32_t* leaf_node, const uint32_t* gidx,
-                            uint32_t* grp_node, int* max_depth, unsigned* err) {
-    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t T = eff(Tdev, Tcap);
-    if (v >= T) return;
-    const uint16_t meta = pn_meta[v];
-    const int d = meta & 255;
-    const bool leaf = meta & 256;
-    const uint2 r = pn_lohi[v];
-    const uint32_t me = pn_cpu[v];
-    const uint32_t nch = pn_nchild[v];
-    const uint32_t first = leaf ? r.x : c.nroots + pn_cb[v];
-    if (me >= T || (!leaf && first + nch > T) || r.x >= r.y || r.y > static_cast<uint32_t>(c.n)) {
-        atomicOr(err, kErrNodeOverflow);
-        return;
+// The nodes in the reference's order, and the buckets of the upsweep filled.
+__global__ void __launch_bounds__(NODE_BS) k_nodes_out(NodeCtx x, PreNodes pn, const double* frame, NodeTest* nd_test,
+                                                       float4* nd_geo, uint32_t* nd_parent, uint32_t* leaf_node,
+                                                       UpsweepIndex* ix, uint32_t* dep_nodes, uint32_t* leaf_order,
+                                                       unsigned* err) {
+    __shared__ unsigned start[NBUCKET], count[NBUCKET];
+    if (!build_ok(x.counts)) return;
+    const uint32_t T = x.counts[2], K = x.counts[1];
+    const int tid = threadIdx.x;
+    if (blockIdx.x * NODE_BS >= T) return;
+    // Where the buckets start: exclusive sums of the counts, depths and leaf sizes apart.
+    if (tid < NBUCKET) {
+        start[tid] = ix->count[tid];
+        count[tid] = 0;
     }
-    nd_test[me].range = make_uint4(r.x, r.y, first, leaf ? 0u : nch);
-    double gx, gy, gz, half;
-    node_geo(c, frame, r.x, d, gx, gy, gz, half);
-    nd_geo[me] = make_float4(static_cast<float>(gx), static_cast<float>(gy), static_cast<float>(gz),
-                             static_cast<float>(half));
-    if (v == 0) nd_parent[0] = 0xffffffffu;
-    if (!leaf)
-        for (uint32_t k = 0; k < nch; ++k) nd_parent[first + k] = me;
-    if (leaf) {
-        const uint32_t l = c.lid[r.x];
-        if (l < static_cast<uint32_t>(leaf_count(c))) leaf_node[l] = me;
-        else atomicOr(err, kErrNodeOverflow);
+    __syncthreads();
+    unsigned before = 0;
+    if (tid < NBUCKET)
+        for (int k = tid < NDEP ? 0 : NDEP; k < tid; ++k) before += start[k];
+    const unsigned own = tid < NBUCKET ? start[tid] : 0u;
+    __syncthreads();
+    if (tid < NBUCKET) {
+        start[tid] = before;
+        if (blockIdx.x == 0) {
+            ix->off[tid] = before;
+            if (tid == NBUCKET - 1) ix->off[NBUCKET] = before + own;
+        }
     }
-    if (meta & 512) {
-        const uint32_t gi = gidx[v];
-        if (gi < T) grp_node[gi] = v;
-        else atomicOr(err, kErrNodeOverflow);
+    __syncthreads();
+    const uint32_t v = blockIdx.x * NODE_BS + tid;
+    uint32_t me = 0xffffffffu;
+    int bucket = -1;
+    unsigned rank = 0;
+    if (v < T) {
+        const uint16_t meta = pn.meta[v];
+        const int d = meta & 255;
+        const bool leaf = meta & 256;
+        const uint2 r = pn.lohi[v];
+        const uint32_t parent = pn.parent[v];
+        const uint32_t nch = __popc(pn.mask[v]);
+        const uint32_t first = leaf ? r.x : pn.first[v];
+        if (d == 0 || parent < T) me = ref_index(x, pn, v, meta, r.x, parent);
+        if (me >= T || (!leaf && (nch == 0 || first + nch > T)) || r.x >= r.y || r.y > static_cast<uint32_t>(x.n)) {
+            atomicOr(err, kErrNodeOverflow);
+        } else {
+            nd_test[me].range = make_uint4(r.x, r.y, first, leaf ? 0u : nch);
+            double gx, gy, gz, half;
+            node_geo(x, frame, r.x, d, gx, gy, gz, half);
+            nd_geo[me] = make_float4(static_cast<float>(gx), static_cast<float>(gy), static_cast<float>(gz),
+                                     static_cast<float>(half));
+            uint32_t up = 0xffffffffu;
+            if (d > 0) {
+                const uint32_t pp = pn.parent[parent];
+                const uint16_t pmeta = pn.meta[parent];
+                if ((pmeta & 255) == 0 || pp < T) up = ref_index(x, pn, parent, pmeta, pn.lohi[parent].x, pp);
+            }
+            nd_parent[me] = up;
+            if (leaf) {
+                const uint32_t l = x.leaf.lid[r.x];
+                if (l < K) leaf_node[l] = me;
+                else atomicOr(err, kErrNodeOverflow);
+            }
+            bucket = bucket_of(meta, r);
+            rank = atomicAdd(&count[bucket], 1u);
+        }
     }
-    atomicMax(max_depth, d);
+    __syncthreads();
+    if (tid < NBUCKET && count[tid]) start[tid] += atomicAdd(&ix->cur[tid], count[tid]);
+    __syncthreads();
+    if (bucket < 0) return;
+    const unsigned pos = start[bucket] + rank;
+    if (bucket < NDEP) {
+        if (pos < T) dep_nodes[pos] = me;
+    } else if (pos < K) {
+        leaf_order[pos] = me;
+    }
 }
 
 // Walk order of the groups: classes of body count, largest first. A group's walk costs about its
@@ -1019,20 +1289,19 @@ __device__ __forceinline__ int group_class(uint32_t count, uint32_t ngroups) {
 
 // Group boxes from the bodies' float positions (src/cpu_backend.cpp:604-616); cls[c] counts the
 // groups of class c.
-__global__ void k_groups(const uint32_t* grp_node, const uint2* pn_lohi, uint32_t Tcap, const unsigned* Tdev,
-                         const BodyArrays b, const unsigned* ngroups, uint2* grp_range, float4* grp_box, unsigned* cls) {
+__global__ void k_groups(const uint32_t* grp_node, const uint2* pn_lohi, uint32_t Tcap, const unsigned* counts,
+                         const BodyArrays b, uint2* grp_range, float4* grp_box, unsigned* cls) {
     __shared__ unsigned count[GCLASS];
     if (threadIdx.x < GCLASS) count[threadIdx.x] = 0;
     __syncthreads();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t T = eff(Tdev, Tcap);
-    if (g < *ngroups && g < Tcap) {
-        // A slot that a missed size guess left unfilled is an empty group.
+    const uint32_t G = min(counts[3], Tcap);  // zero when the build did not run
+    if (g < G) {
         const uint32_t v = grp_node[g];
-        uint2 r = v < T ? pn_lohi[v] : make_uint2(0u, 0u);
+        uint2 r = v < counts[2] ? pn_lohi[v] : make_uint2(0u, 0u);
         if (r.x >= r.y) r = make_uint2(0u, 0u);
         grp_range[g] = r;
-        atomicAdd(&count[group_class(r.y - r.x, *ngroups)], 1u);
+        atomicAdd(&count[group_class(r.y - r.x, G)], 1u);
         if (r.x < r.y) {
             float4 p = b.hm[r.x];
             float mnx = p.x, mny = p.y, mnz = p.z, mxx = mnx, mxy = mny, mxz = mnz;
@@ -1068,7 +1337,7 @@ __global__ void k_group_order(const uint2* grp_range, uint32_t Tcap, const unsig
     unsigned rank = 0;
     if (g < G) {
         const uint2 r = grp_range[g];
-        c = group_class(r.y - r.x, *ngroups);
+        c = group_class(r.y - r.x, G);
         rank = atomicAdd(&count[c], 1u);
     }
     __syncthreads();
@@ -1084,27 +1353,24 @@ __global__ void k_group_order(const uint2* grp_range, uint32_t Tcap, const unsig
 // parent, contiguous bodies) are packed greedily, in order, into groups of <= group_max bodies:
 // fewer, fuller walk groups. Every packed group is still contained in its parent, whose walk
 // rule opens it, so the lists stay exact-rule lists for the larger box.
-__device__ __forceinline__ uint32_t group_parent(const uint32_t* grp_node, const uint32_t* pn_cpu,
-                                                 const uint32_t* nd_parent, uint32_t T, uint32_t g) {
+__device__ __forceinline__ uint32_t group_parent(const uint32_t* grp_node, const uint32_t* pn_parent, uint32_t T, uint32_t g) {
     const uint32_t v = grp_node[g];
-    if (v >= T) return 0xffffffffu;
-    const uint32_t c = pn_cpu[v];
-    return c < T ? nd_parent[c] : 0xffffffffu;
+    return v < T ? pn_parent[v] : 0xffffffffu;
 }
 
 template <bool WRITE>
-__global__ void k_merge_groups(const uint32_t* grp_node, const uint32_t* pn_cpu, const uint32_t* nd_parent,
+__global__ void k_merge_groups(const uint32_t* grp_node, const uint32_t* pn_parent,
                                const uint2* grp_range, const unsigned* ngroups, uint32_t Tcap, const unsigned* Tdev,
                                int gmax, uint32_t* mcount, const uint32_t* moff, uint2* mrange) {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= Tcap) return;
-    const uint32_t T = eff(Tdev, Tcap), G = min(*ngroups, Tcap);
+    const uint32_t T = min(*Tdev, Tcap), G = min(*ngroups, Tcap);
     if (g >= G) {
         if (!WRITE) mcount[g] = 0;
         return;
     }
-    const uint32_t P = group_parent(grp_node, pn_cpu, nd_parent, T, g);
-    const bool start = g == 0 || group_parent(grp_node, pn_cpu, nd_parent, T, g - 1) != P ||
+    const uint32_t P = group_parent(grp_node, pn_parent, T, g);
+    const bool start = g == 0 || group_parent(grp_node, pn_parent, T, g - 1) != P ||
                        grp_range[g - 1].y != grp_range[g].x;
     if (!start) {
         if (!WRITE) mcount[g] = 0;
@@ -1113,7 +1379,7 @@ __global__ void k_merge_groups(const uint32_t* grp_node, const uint32_t* pn_cpu,
     uint32_t bins = 0, cur = 0, lo = grp_range[g].x, hi = lo;
     for (uint32_t h = g; h < G; ++h) {
         const uint2 r = grp_range[h];
-        if (h > g && (group_parent(grp_node, pn_cpu, nd_parent, T, h) != P || r.x != hi)) break;
+        if (h > g && (group_parent(grp_node, pn_parent, T, h) != P || r.x != hi)) break;
         const uint32_t sz = r.y - r.x;
         if (cur > 0 && cur + sz > static_cast<uint32_t>(gmax)) {
             if (WRITE) mrange[moff[g] + bins] = make_uint2(lo, hi);
@@ -1184,76 +1450,15 @@ __device__ void store_moments(Moments mo, uint32_t node, double M, double cx, do
 #define DSUB __dsub_rn
 #define DFMA __fma_rn
 
-// Upsweep bookkeeping: internal nodes bucketed by depth, leaves bucketed by body count.
-constexpr int NDEP = MAX_DEPTH + 2;  // depth buckets (depth <= MAX_DEPTH + 1 with headroom)
-constexpr int NLSZ = 18;   // leaf-size buckets: 1..16, then larger
-struct UpsweepIndex {
-    unsigned dep_count[NDEP], dep_off[NDEP + 1], dep_cur[NDEP];
-    unsigned lsz_count[NLSZ], lsz_off[NLSZ + 1], lsz_cur[NLSZ];
-};
-
-__device__ __forceinline__ int lsz_bucket(uint32_t cnt) { return cnt > 16 ? 17 : static_cast<int>(cnt); }
-
-// Pass 1: bucket counts (block-aggregated). Pass 2 (phase 1): scatter into bucket order.
-__global__ void k_upsweep_bucket(const uint2* pn_lohi, const uint16_t* pn_meta, const uint32_t* pn_cpu, uint32_t Tcap,
-                                 const unsigned* Tdev, UpsweepIndex* ix, int phase, uint32_t* dep_nodes,
-                                 uint32_t* leaf_order) {
-    const uint32_t T = eff(Tdev, Tcap);
-    __shared__ unsigned sc[NDEP + NLSZ], sbase[NDEP + NLSZ];
-    for (int k = threadIdx.x; k < NDEP + NLSZ; k += blockDim.x) sc[k] = 0;
-    __syncthreads();
-    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    int bucket = -1;
-    unsigned rank = 0;
-    uint32_t me = 0;
-    if (v < T) {
-        const uint16_t meta = pn_meta[v];
-        me = pn_cpu[v];
-        if (meta & 256) {
-            const uint2 r = pn_lohi[v];
-            bucket = NDEP + lsz_bucket(r.y - r.x);
-        } else {
-            bucket = meta & 255;
-        }
-        rank = atomicAdd(&sc[bucket], 1u);
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < NDEP + NLSZ; k += blockDim.x) {
-        if (!sc[k]) continue;
-        if (phase == 0) {
-            atomicAdd(k < NDEP ? &ix->dep_count[k] : &ix->lsz_count[k - NDEP], sc[k]);
-        } else {
-            sbase[k] = k < NDEP ? ix->dep_off[k] + atomicAdd(&ix->dep_cur[k], sc[k])
-                                : ix->lsz_off[k - NDEP] + atomicAdd(&ix->lsz_cur[k - NDEP], sc[k]);
-        }
-    }
-    if (phase == 0) return;
-    __syncthreads();
-    if (bucket < 0) return;
-    const unsigned pos = sbase[bucket] + rank;
-    if (bucket < NDEP) dep_nodes[pos] = me;
-    else leaf_order[pos] = me;
-}
-
-__global__ void k_upsweep_offsets(UpsweepIndex* ix) {
-    if (threadIdx.x != 0) return;
-    unsigned run = 0;
-    for (int k = 0; k < NDEP; ++k) { ix->dep_off[k] = run; run += ix->dep_count[k]; }
-    ix->dep_off[NDEP] = run;
-    run = 0;
-    for (int k = 0; k < NLSZ; ++k) { ix->lsz_off[k] = run; run += ix->lsz_count[k]; }
-    ix->lsz_off[NLSZ] = run;
-}
-
 // Leaf moments about each leaf's centre of mass in FP64 (src/cpu_backend.cpp:619-640), one
 // thread per leaf, leaves taken in body-count order so a warp's loops have equal trip counts.
-__global__ void k_leaf_moments(const uint32_t* __restrict__ leaf_order, uint32_t Kcap, const unsigned* Kdev,
-                               uint32_t Tcap, const unsigned* Tdev,
+__global__ void k_leaf_moments(const uint32_t* __restrict__ leaf_order, const unsigned* counts,
                                const float4* __restrict__ nd_geo, const BodyArrays b, Moments mo, float inv_theta,
                                const float* __restrict__ inv_theta_sys, const uint32_t* __restrict__ sys, unsigned* err) {
     const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t T = eff(Tdev, Tcap);
-    if (l >= eff(Kdev, Kcap)) return;
+    if (!build_ok(counts)) return;
+    const uint32_t T = counts[2];
+    if (l >= counts[1]) return;
     const uint32_t node = leaf_order[l];
     if (node >= T) {
         atomicOr(err, kErrNodeOverflow);
@@ -1303,17 +1508,15 @@ __device__ __forceinline__ double shfl_d(double v, int src_lane) { return __shfl
 constexpr int COMBINE_BS = 128;
 constexpr int COMBINE_NODES = COMBINE_BS / 4;  // nodes per block and round
 
-__global__ void __launch_bounds__(COMBINE_BS) k_combine_level(const uint32_t* __restrict__ dep_nodes,
-                                                              const UpsweepIndex* ix, int depth, uint32_t Tcap,
-                                                              const unsigned* Tdev,
-                                                              const float4* __restrict__ nd_geo, Moments mo,
-                                                              float inv_theta, const float* __restrict__ inv_theta_sys,
-                                                              const uint32_t* __restrict__ sys, unsigned* err) {
-    const uint32_t T = eff(Tdev, Tcap);
-    const unsigned lo = ix->dep_off[depth], hi = ix->dep_off[depth + 1];
+// The nodes of one depth, taken by `warps` warps of which this is number wid. FAR: the children were
+// written by other SMs in the same launch and are read past the L1 cache.
+template <bool FAR>
+__device__ __forceinline__ void combine_depth(const uint32_t* __restrict__ dep_nodes, const UpsweepIndex* ix, int depth,
+                                              uint32_t T, const float4* __restrict__ nd_geo, const Moments& mo,
+                                              float inv_theta, const float* __restrict__ inv_theta_sys,
+                                              const uint32_t* __restrict__ sys, unsigned wid, unsigned warps, unsigned* err) {
+    const unsigned lo = ix->off[depth], hi = depth + 1 < NDEP ? ix->off[depth + 1] : lo;
     const int lane = threadIdx.x & 31, j = lane & 3, base = lane & ~3;
-    const unsigned warps = (gridDim.x * blockDim.x) >> 5;
-    const unsigned wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     for (unsigned k0 = lo + 8 * wid; k0 < hi; k0 += 8 * warps) {  // warp-uniform
         const unsigned k = k0 + static_cast<unsigned>(lane >> 2);
         bool valid = k < hi;
@@ -1342,9 +1545,10 @@ __global__ void __launch_bounds__(COMBINE_BS) k_combine_level(const uint32_t* __
             qa[sl] = cm;
             qb[sl] = cm;
             if (c < nch) {
-                cm = mo.cell[r.z + c].com;
-                qa[sl] = mo.cell[r.z + c].q0;
-                qb[sl] = mo.cell[r.z + c].q1;
+                const NodeCell* ch = mo.cell + r.z + c;
+                cm = FAR ? __ldcg(&ch->com) : ch->com;
+                qa[sl] = FAR ? __ldcg(&ch->q0) : ch->q0;
+                qb[sl] = FAR ? __ldcg(&ch->q1) : ch->q1;
             }
             m[sl] = cm.w;
             ccx[sl] = cm.x;
@@ -1406,22 +1610,40 @@ __global__ void __launch_bounds__(COMBINE_BS) k_combine_level(const uint32_t* __
     }
 }
 
+__global__ void __launch_bounds__(COMBINE_BS) k_combine_level(const uint32_t* __restrict__ dep_nodes,
+                                                              const UpsweepIndex* ix, int depth, const unsigned* counts,
+                                                              const float4* __restrict__ nd_geo, Moments mo,
+                                                              float inv_theta, const float* __restrict__ inv_theta_sys,
+                                                              const uint32_t* __restrict__ sys, unsigned* err) {
+    if (!build_ok(counts)) return;
+    combine_depth<false>(dep_nodes, ix, depth, counts[2], nd_geo, mo, inv_theta, inv_theta_sys, sys,
+                         (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5, err);
+}
+
+// The depths from `depth` up to the root in one launch of one cluster of 16 blocks (one warp per
+// scheduler of 16 SMs), a cluster barrier between depths: a depth of up to 512 nodes is one round of
+// the FP64 chain (about 4 us) whether it has its own launch or not, and the barrier costs less than
+// the launch.
+constexpr int TOP_BLOCKS = 16, TOP_NODES = TOP_BLOCKS * COMBINE_NODES;
+__global__ void __launch_bounds__(COMBINE_BS) k_combine_top(const uint32_t* __restrict__ dep_nodes, const UpsweepIndex* ix,
+                                                            int depth, const unsigned* counts,
+                                                            const float4* __restrict__ nd_geo, Moments mo, float inv_theta,
+                                                            const float* __restrict__ inv_theta_sys,
+                                                            const uint32_t* __restrict__ sys, unsigned* err) {
+    if (!build_ok(counts)) return;  // the same word for all blocks
+    for (; depth >= 0; --depth) {
+        combine_depth<true>(dep_nodes, ix, depth, counts[2], nd_geo, mo, inv_theta, inv_theta_sys, sys,
+                            (blockIdx.x * blockDim.x + threadIdx.x) >> 5, TOP_BLOCKS * COMBINE_BS / 32, err);
+        __threadfence();
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+
 #undef DADD
 #undef DMUL
 #undef DSUB
 
-
-__global__ void k_lid(uint32_t* lid, const uint32_t* flag, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) lid[i] = lid[i] + flag[i] - 1;
-}
-
-__global__ void k_leaf_tail(uint32_t* leaf_first, const unsigned* K, int n) { leaf_first[*K] = static_cast<uint32_t>(n); }
-
-__global__ void k_gflag(const uint16_t* pn_meta, uint32_t Tcap, const unsigned* Tdev, uint32_t* gflag) {
-    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < Tcap) gflag[v] = v < eff(Tdev, Tcap) ? (pn_meta[v] >> 9) & 1u : 0u;
-}
 
 __global__ void k_probe() {}
 
@@ -1438,6 +1660,9 @@ void scan_u32(Engine& e, TreeState& t, const uint32_t* in, uint32_t* out, int n,
     LG_LAUNCHED();
     ++e.launches;
 }
+
+// k_leaves' look-back words and its tile counter.
+size_t leaf_state_words(int n) { return (static_cast<size_t>(leaf_tiles(n)) * 8 + 16 + 15) / 16; }
 
 int sort_tiles(int n) { return (n + SORT_TILE - 1) / SORT_TILE; }
 
@@ -1484,6 +1709,7 @@ void reserve_sort(TreeState& t, int n) {
     t.hist.reserve(hist_words() * 16);
     t.lookback.reserve(lookback_words(n, PASSES) * 16);
     t.counts.reserve(64);
+    t.leaf_state.reserve(leaf_state_words(n) * 16);
 }
 
 // Octal digits to sort by when no earlier build says how deep the tree is: one and a half times
@@ -1504,6 +1730,8 @@ int bits_for(int count) {
 }  // namespace
 
 std::unique_ptr<TreeState, void (*)(TreeState*)> make_tree_state() {
+    // Clusters of 16 blocks are an opt-in size.
+    LG_CK(cudaFuncSetAttribute(k_combine_top, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     return std::unique_ptr<TreeState, void (*)(TreeState*)>(new TreeState, destroy_tree);
 }
 
@@ -1548,6 +1776,7 @@ void tree_sort(Engine& e) {
         z.span[0] = {t.counts.as<uint4>(), 4};
         z.span[1] = {t.hist.as<uint4>(), hist_words()};
         z.span[2] = {t.lookback.as<uint4>(), lookback_words(n, passes)};
+        z.span[3] = {t.leaf_state.as<uint4>(), leaf_state_words(n)};
         if (sys) {
             k_frame_sys<<<t.nsys, BS, 0, s>>>(e.bodies(e.cur), t.sys_off, t.frame.as<double>(), z);
         } else {
@@ -1673,49 +1902,31 @@ void tree_build(Engine& e, double theta) {
     const uint64_t* k0 = t.skey.as<uint64_t>();
     const FrameTable* ft = t.restarted ? t.ftab.as<FrameTable>() : nullptr;
     unsigned* counts = t.counts.as<unsigned>();
-    const unsigned* Kdev = counts + 1;
-    const unsigned* Tdev = counts + 2;
     const size_t n1 = static_cast<size_t>(n) + 1;
-    t.bdepth.reserve(n1 * 2);
-    t.flag.reserve(n1 * 4);
     t.leafid.reserve(n1 * 4);
     t.leaf_first.reserve(n1 * 4);
     t.leaf_depth.reserve(n1);
+    t.leaf_gdepth.reserve(n1);
     t.leaf_c.reserve(n1);
-    t.leaf_cnt.reserve(n1 * 4);
     t.leaf_pre.reserve(n1 * 4);
     t.leaf_node.reserve(n1 * 4);
-    const int gb = grid_for(n, BS);
     if (t.group_max > GMAX_LIMIT) fail(kRuntime, "cuda tree build: group size above 1024");
-    k_body_depth<<<grid_for(n, DEPTH_BS), DEPTH_BS, 0, s>>>(sys, k0, ft, n, t.group_max,
-                                                            t.bdepth.as<uint16_t>());
-    LG_LAUNCHED();
-    k_leaf_flags<<<gb, BS, 0, s>>>(sys, k0, ft, t.bdepth.as<uint16_t>(), n, t.flag.as<uint32_t>());
-    LG_LAUNCHED();
-    e.launches += 2;
-    scan_u32(e, t, t.flag.as<uint32_t>(), t.leafid.as<uint32_t>(), n, counts + 1);
-    LG_CK(cudaMemsetAsync(t.leaf_cnt.as<char>(), 0, n1 * 4, s));
-    k_leaf_info<<<gb, BS, 0, s>>>(sys, k0, ft, t.bdepth.as<uint16_t>(), t.flag.as<uint32_t>(), t.leafid.as<uint32_t>(), n,
-                                  t.leaf_first.as<uint32_t>(), t.leaf_depth.as<uint8_t>(), t.leaf_c.as<int8_t>(),
-                                  t.leaf_cnt.as<uint32_t>(), reinterpret_cast<int*>(counts + 4));
-    LG_LAUNCHED();
-    k_lid<<<gb, BS, 0, s>>>(t.leafid.as<uint32_t>(), t.flag.as<uint32_t>(), n);
-    LG_LAUNCHED();
-    k_leaf_tail<<<1, 1, 0, s>>>(t.leaf_first.as<uint32_t>(), counts + 1, n);
-    LG_LAUNCHED();
-    e.launches += 3;
-    scan_u32(e, t, t.leaf_cnt.as<uint32_t>(), t.leaf_pre.as<uint32_t>(), n + 1, counts + 2);
     // Sizes: exact (one host read) for the first build and after a miss; otherwise the previous
-    // build's with headroom, checked by tree_verify once the force call synchronises.
-    size_t K, T;
-    int depth;
+    // build's with headroom, checked by tree_verify once the force call synchronises. On a miss the
+    // kernels after k_leaves do nothing (counts[8]).
     const bool spec = t.have_guess && (t.speculative || t.restarted);
-    if (spec) {
-        K = t.K;
-        T = t.T;
-        depth = t.max_depth;
-        t.speculative = true;
-    } else {
+    const LeafOut leaf{t.leafid.as<uint32_t>(), t.leaf_first.as<uint32_t>(), t.leaf_pre.as<uint32_t>(),
+                       t.leaf_depth.as<uint8_t>(), t.leaf_gdepth.as<uint8_t>(), t.leaf_c.as<int8_t>()};
+    auto leaves = [&](unsigned Kcap, unsigned Tcap, const ZeroList& z) {
+        const int tiles = leaf_tiles(n);
+        k_leaves<<<tiles, LEAF_BS, 0, s>>>(sys, k0, ft, n, t.group_max, leaf, t.leaf_state.as<unsigned long long>(),
+                                           t.leaf_state.as<unsigned>() + 2 * static_cast<size_t>(tiles), counts, Kcap,
+                                           Tcap, z, e.err_word());
+        LG_LAUNCHED();
+        ++e.launches;
+    };
+    if (!spec) {
+        leaves(0xffffffffu, 0xffffffffu, ZeroList{});
         LG_CK(cudaMemcpyAsync(e.pinned_small, counts, 32, cudaMemcpyDeviceToHost, s));
         LG_CK(cudaStreamSynchronize(s));
         const size_t Kx = e.pinned_small[1], Tx = e.pinned_small[2];
@@ -1727,131 +1938,137 @@ void tree_build(Engine& e, double theta) {
         size_t pct = 25;
         if (const char* h = std::getenv("LETTUCE_GB300_TREE_HEADROOM")) pct = static_cast<size_t>(std::atoi(h));
         const size_t slack = pct ? 1024 : 0;
-        K = std::min(static_cast<size_t>(n), Kx + Kx * pct / 100 + slack);
-        T = Tx + Tx * pct / 100 + slack;
-        depth = std::min(dx + (pct ? 2 : 0), MAX_DEPTH + 1);
-        t.K = K;
-        t.T = T;
-        t.max_depth = depth;
+        t.K = std::min(static_cast<size_t>(n), Kx + Kx * pct / 100 + slack);
+        t.T = Tx + Tx * pct / 100 + slack;
+        t.max_depth = std::min(dx + (pct ? 2 : 0), MAX_DEPTH + 1);
         t.have_guess = true;
         ++t.generation;
-        t.speculative = false;
     }
+    t.speculative = spec;
+    const size_t K = t.K, T = t.T;
+    const int depth = t.max_depth;
+    // What has to be zero before the node kernels, in one buffer: the upsweep's buckets, the group
+    // classes, the scan's look-back words and tile counter, the child masks. Cleared by k_leaves when
+    // the sizes are known before it.
+    const int scan_tiles = grid_for(static_cast<long long>(T), NSCAN_TILE);
+    const size_t z_ix = (sizeof(UpsweepIndex) + 15) / 16 * 16, z_cls = 2 * GCLASS * 4,
+                 z_state = static_cast<size_t>(scan_tiles) * 8 + 16;
+    const size_t z_mask = (z_ix + z_cls + z_state + 15) / 16 * 16, z_all = z_mask + (T * 4 + 15) / 16 * 16;
+    t.node_zero.reserve(z_all);
     t.pn_lohi.reserve(T * 8);
     t.pn_meta.reserve(T * 2);
-    t.pn_nchild.reserve(T * 4);
-    t.pn_cb.reserve(T * 4);
-    t.pn_cpu.reserve(T * 4);
-    t.gflag.reserve(T * 4);
-    t.gidx.reserve(T * 4);
+    t.pn_parent.reserve(T * 4);
+    t.pn_first.reserve(T * 4);
     t.grp_node.reserve(T * 4);
     t.grp_range.reserve(T * 8);
     t.grp_box.reserve(T * 32);
     t.grp_order.reserve(T * 4);
-    t.grp_class.reserve(2 * GCLASS * 4);
     t.nd_test.reserve(T * sizeof(NodeTest));
     t.nd_cell.reserve(T * sizeof(NodeCell));
     t.nd_geo.reserve(T * 16);
     t.nd_parent.reserve(T * 4);
-    const uint32_t Tc = static_cast<uint32_t>(T), Kc = static_cast<uint32_t>(K);
-    NodeCtx c{sys, k0, ft, t.leaf_first.as<uint32_t>(), t.leaf_depth.as<uint8_t>(), t.leaf_c.as<int8_t>(),
-              t.leaf_pre.as<uint32_t>(), t.leafid.as<uint32_t>(), t.bdepth.as<uint16_t>(), n, Kdev, Kc,
-              static_cast<unsigned>(sys ? t.nsys : 1)};
-    const int tb = grid_for(static_cast<long long>(T), BS);
-    // Index arrays start out of range (0xff..): a slot the construction fails to fill is caught by
-    // the range checks below instead of being followed.
-    LG_CK(cudaMemsetAsync(t.pn_cpu.as<char>(), 0xff, T * 4, s));
-    LG_CK(cudaMemsetAsync(t.grp_node.as<char>(), 0xff, T * 4, s));
-    LG_CK(cudaMemsetAsync(t.leaf_node.as<char>(), 0xff, K * 4, s));
-    LG_CK(cudaMemsetAsync(t.nd_parent.as<char>(), 0xff, T * 4, s));
-    LG_CK(cudaMemsetAsync(t.nd_test.as<char>(), 0, T * sizeof(NodeTest), s));
-    LG_CK(cudaMemsetAsync(t.grp_range.as<char>(), 0, T * 8, s));
-    k_nodes_pre<<<tb, BS, 0, s>>>(c, Tc, Tdev, t.pn_lohi.as<uint2>(), t.pn_meta.as<uint16_t>());
+    t.dep_nodes.reserve(T * 4);
+    t.leaf_order.reserve(K * 4);
+    char* zero = t.node_zero.as<char>();
+    if (spec) {
+        ZeroList z{};
+        z.span[0] = {t.node_zero.as<uint4>(), z_all / 16};
+        leaves(static_cast<unsigned>(std::min<size_t>(K, 0xffffffffu)), static_cast<unsigned>(std::min<size_t>(T, 0xffffffffu)), z);
+    } else {
+        LG_CK(cudaMemsetAsync(zero, 0, z_all, s));
+    }
+    UpsweepIndex* ix = reinterpret_cast<UpsweepIndex*>(zero);
+    unsigned* cls = reinterpret_cast<unsigned*>(zero + z_ix);
+    unsigned long long* scan_state = reinterpret_cast<unsigned long long*>(zero + z_ix + z_cls);
+    const PreNodes pn{t.pn_lohi.as<uint2>(), t.pn_meta.as<uint16_t>(), t.pn_parent.as<uint32_t>(),
+                      reinterpret_cast<uint32_t*>(zero + z_mask), t.pn_first.as<uint32_t>()};
+    const NodeCtx x{sys, k0, ft, leaf, n, counts, static_cast<unsigned>(sys ? t.nsys : 1)};
+    const uint32_t Tc = static_cast<uint32_t>(T);
+    const int tb = grid_for(static_cast<long long>(T), NODE_BS);
+    k_nodes<<<tb, NODE_BS, 0, s>>>(x, pn);
     LG_LAUNCHED();
-    k_nchild<<<tb, BS, 0, s>>>(c, Tc, Tdev, t.pn_lohi.as<uint2>(), t.pn_meta.as<uint16_t>(), t.pn_nchild.as<uint32_t>());
+    k_node_scan<<<scan_tiles, NSCAN_BS, 0, s>>>(x, pn, scan_state, reinterpret_cast<unsigned*>(scan_state + scan_tiles),
+                                                counts, ix, t.grp_node.as<uint32_t>(), e.err_word());
     LG_LAUNCHED();
     e.launches += 2;
-    scan_u32(e, t, t.pn_nchild.as<uint32_t>(), t.pn_cb.as<uint32_t>(), static_cast<int>(T), nullptr);
-    k_gflag<<<tb, BS, 0, s>>>(t.pn_meta.as<uint16_t>(), Tc, Tdev, t.gflag.as<uint32_t>());
-    LG_LAUNCHED();
-    ++e.launches;
-    scan_u32(e, t, t.gflag.as<uint32_t>(), t.gidx.as<uint32_t>(), static_cast<int>(T), counts + 3);
-    k_cpu_index<<<tb, BS, 0, s>>>(c, Tc, Tdev, t.pn_lohi.as<uint2>(), t.pn_meta.as<uint16_t>(), t.pn_cb.as<uint32_t>(),
-                                  t.pn_cpu.as<uint32_t>());
-    LG_LAUNCHED();
-    k_nodes_out<<<tb, BS, 0, s>>>(c, Tc, Tdev, t.pn_lohi.as<uint2>(), t.pn_meta.as<uint16_t>(),
-                                  t.pn_nchild.as<uint32_t>(), t.pn_cb.as<uint32_t>(), t.pn_cpu.as<uint32_t>(),
-                                  t.frame.as<double>(), t.nd_test.as<NodeTest>(), t.nd_geo.as<float4>(),
-                                  t.nd_parent.as<uint32_t>(), t.leaf_node.as<uint32_t>(), t.gidx.as<uint32_t>(),
-                                  t.grp_node.as<uint32_t>(), reinterpret_cast<int*>(counts + 4), e.err_word());
-    LG_LAUNCHED();
+    // The group boxes depend neither on the nodes' order nor on the moments: with the reference groups
+    // they are computed on the side stream from here on, and joined back before the build returns.
     t.merged = e.walk_merge && !sys;
-    // The group boxes do not depend on the moments: with the reference groups they are computed on
-    // the side stream while the FP64 upsweep runs, and joined back before the build returns.
     cudaStream_t gs = s;
     if (!t.merged) {
         LG_CK(cudaEventRecord(e.fork_ev, s));
         LG_CK(cudaStreamWaitEvent(e.side, e.fork_ev, 0));
         gs = e.side;
     }
-    LG_CK(cudaMemsetAsync(t.grp_class.as<unsigned>(), 0, 2 * GCLASS * 4, gs));
-    k_groups<<<tb, BS, 0, gs>>>(t.grp_node.as<uint32_t>(), t.pn_lohi.as<uint2>(), Tc, Tdev, e.bodies(e.cur), counts + 3,
-                                t.grp_range.as<uint2>(), t.grp_box.as<float4>(), t.grp_class.as<unsigned>());
+    const int gb = grid_for(static_cast<long long>(std::min<size_t>(T, K)), BS);  // a group holds at least one leaf
+    k_groups<<<gb, BS, 0, gs>>>(t.grp_node.as<uint32_t>(), t.pn_lohi.as<uint2>(), Tc, counts, e.bodies(e.cur),
+                                t.grp_range.as<uint2>(), t.grp_box.as<float4>(), cls);
     LG_LAUNCHED();
+    ++e.launches;
     if (!t.merged) {
-        k_group_order<<<tb, BS, 0, gs>>>(t.grp_range.as<uint2>(), Tc, counts + 3, t.grp_class.as<unsigned>(),
-                                         t.grp_order.as<uint32_t>());
+        k_group_order<<<gb, BS, 0, gs>>>(t.grp_range.as<uint2>(), Tc, counts + 3, cls, t.grp_order.as<uint32_t>());
         LG_LAUNCHED();
         ++e.launches;
+        LG_CK(cudaEventRecord(e.join_ev, e.side));
     }
-    if (!t.merged) LG_CK(cudaEventRecord(e.join_ev, e.side));
-    e.launches += 3;
+    k_nodes_out<<<tb, NODE_BS, 0, s>>>(x, pn, t.frame.as<double>(), t.nd_test.as<NodeTest>(), t.nd_geo.as<float4>(),
+                                       t.nd_parent.as<uint32_t>(), t.leaf_node.as<uint32_t>(), ix,
+                                       t.dep_nodes.as<uint32_t>(), t.leaf_order.as<uint32_t>(), e.err_word());
+    LG_LAUNCHED();
+    ++e.launches;
     if (t.merged) {
         t.mcount.reserve(T * 4 + 4);
         t.moff.reserve(T * 4 + 4);
         t.mrange.reserve(T * 8 + 8);
         t.mbox.reserve(T * 32 + 32);
-        k_merge_groups<false><<<tb, BS, 0, s>>>(t.grp_node.as<uint32_t>(), t.pn_cpu.as<uint32_t>(),
-                                                t.nd_parent.as<uint32_t>(), t.grp_range.as<uint2>(), counts + 3, Tc,
-                                                Tdev, std::min(e.merge_cap, t.group_max), t.mcount.as<uint32_t>(),
+        k_merge_groups<false><<<tb, BS, 0, s>>>(t.grp_node.as<uint32_t>(), t.pn_parent.as<uint32_t>(),
+                                                t.grp_range.as<uint2>(), counts + 3, Tc, counts + 2, std::min(e.merge_cap, t.group_max), t.mcount.as<uint32_t>(),
                                                 nullptr, nullptr);
         LG_LAUNCHED();
         scan_u32(e, t, t.mcount.as<uint32_t>(), t.moff.as<uint32_t>(), static_cast<int>(T), counts + 5);
-        k_merge_groups<true><<<tb, BS, 0, s>>>(t.grp_node.as<uint32_t>(), t.pn_cpu.as<uint32_t>(),
-                                               t.nd_parent.as<uint32_t>(), t.grp_range.as<uint2>(), counts + 3, Tc,
-                                               Tdev, std::min(e.merge_cap, t.group_max), nullptr,
+        k_merge_groups<true><<<tb, BS, 0, s>>>(t.grp_node.as<uint32_t>(), t.pn_parent.as<uint32_t>(),
+                                               t.grp_range.as<uint2>(), counts + 3, Tc, counts + 2, std::min(e.merge_cap, t.group_max), nullptr,
                                                t.moff.as<uint32_t>(), t.mrange.as<uint2>());
         LG_LAUNCHED();
         k_merged_boxes<<<tb, BS, 0, s>>>(t.mrange.as<uint2>(), counts + 5, Tc, e.bodies(e.cur), t.mbox.as<float4>());
         LG_LAUNCHED();
         e.launches += 3;
     }
-    // Upsweep: leaves (by size), then internal nodes level by level from the deepest.
-    t.ups.reserve(sizeof(UpsweepIndex));
-    t.dep_nodes.reserve(T * 4);
-    t.leaf_order.reserve(K * 4);
-    UpsweepIndex* ix = t.ups.as<UpsweepIndex>();
-    LG_CK(cudaMemsetAsync(ix, 0, sizeof(UpsweepIndex), s));
-    k_upsweep_bucket<<<tb, BS, 0, s>>>(t.pn_lohi.as<uint2>(), t.pn_meta.as<uint16_t>(), t.pn_cpu.as<uint32_t>(), Tc, Tdev,
-                                       ix, 0, nullptr, nullptr);
-    LG_LAUNCHED();
-    k_upsweep_offsets<<<1, 32, 0, s>>>(ix);
-    LG_LAUNCHED();
-    k_upsweep_bucket<<<tb, BS, 0, s>>>(t.pn_lohi.as<uint2>(), t.pn_meta.as<uint16_t>(), t.pn_cpu.as<uint32_t>(), Tc, Tdev,
-                                       ix, 1, t.dep_nodes.as<uint32_t>(), t.leaf_order.as<uint32_t>());
-    LG_LAUNCHED();
+    // Upsweep: leaves (by size), then internal nodes level by level from the deepest; the depths of at
+    // most TOP_NODES nodes (by the eight-way branching, or because the whole tree is small) together.
     const float inv_theta = theta > 0 ? static_cast<float>(1.0 / theta) : FLT_MAX;
     Moments mo{t.nd_test.as<NodeTest>(), t.nd_cell.as<NodeCell>()};
     k_leaf_moments<<<grid_for(static_cast<long long>(K), 128), 128, 0, s>>>(
-        t.leaf_order.as<uint32_t>(), Kc, Kdev, Tc, Tdev, t.nd_geo.as<float4>(), e.bodies(e.cur),
-        mo, inv_theta, t.inv_theta_sys, sys, e.err_word());
+        t.leaf_order.as<uint32_t>(), counts, t.nd_geo.as<float4>(), e.bodies(e.cur), mo, inv_theta, t.inv_theta_sys, sys,
+        e.err_word());
     LG_LAUNCHED();
-    e.launches += 4;
+    ++e.launches;
+    int top = -1;
+    if (T <= 8 * TOP_NODES) top = depth - 1;
+    else
+        for (size_t width = x.nroots; width <= TOP_NODES && top < depth - 1; width *= 8) ++top;
     const int cb = std::max(1, std::min(2 * e.sms, grid_for(static_cast<long long>(T), COMBINE_NODES)));
-    for (int d = depth - 1; d >= 0; --d) {
-        k_combine_level<<<cb, COMBINE_BS, 0, s>>>(t.dep_nodes.as<uint32_t>(), ix, d, Tc, Tdev,
-                                           t.nd_geo.as<float4>(), mo, inv_theta, t.inv_theta_sys, sys, e.err_word());
+    for (int d = depth - 1; d > top; --d) {
+        k_combine_level<<<cb, COMBINE_BS, 0, s>>>(t.dep_nodes.as<uint32_t>(), ix, d, counts, t.nd_geo.as<float4>(), mo,
+                                                  inv_theta, t.inv_theta_sys, sys, e.err_word());
         LG_LAUNCHED();
+        ++e.launches;
+    }
+    if (top >= 0) {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = TOP_BLOCKS;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(TOP_BLOCKS);
+        cfg.blockDim = dim3(COMBINE_BS);
+        cfg.stream = s;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        LG_CK(cudaLaunchKernelEx(&cfg, k_combine_top, static_cast<const uint32_t*>(t.dep_nodes.as<uint32_t>()),
+                                 static_cast<const UpsweepIndex*>(ix), top, static_cast<const unsigned*>(counts),
+                                 static_cast<const float4*>(t.nd_geo.as<float4>()), mo, inv_theta, t.inv_theta_sys, sys,
+                                 e.err_word()));
         ++e.launches;
     }
     if (!t.merged) LG_CK(cudaStreamWaitEvent(s, e.join_ev, 0));
@@ -2036,10 +2253,11 @@ size_t tree_held_bytes(const Engine& e) {
     const TreeState& t = *e.tree;
     size_t h = 0;
     for (const DevBuf* d : {&t.keysA, &t.keysB, &t.valsA, &t.valsB, &t.hist, &t.lookback, &t.mkeys, &t.skey, &t.key1tmp,
-                            &t.nfr, &t.ftab, &t.bdepth, &t.flag, &t.leafid, &t.frame, &t.runs, &t.counts,
-                            &t.leaf_first, &t.leaf_depth, &t.leaf_c, &t.leaf_pre, &t.leaf_node, &t.pn_lohi,
-                            &t.pn_meta, &t.pn_nchild, &t.pn_cb, &t.pn_cpu, &t.nd_test, &t.nd_cell, &t.nd_geo, &t.nd_parent, &t.gflag, &t.gidx, &t.grp_node, &t.leaf_cnt, &t.ups, &t.dep_nodes, &t.leaf_order,
-                            &t.grp_range, &t.grp_box, &t.grp_order, &t.grp_class, &t.scan_state, &t.scan_ctr})
+                            &t.nfr, &t.ftab, &t.leafid, &t.frame, &t.runs, &t.counts, &t.leaf_first, &t.leaf_depth,
+                            &t.leaf_gdepth, &t.leaf_c, &t.leaf_pre, &t.leaf_node, &t.leaf_state, &t.pn_lohi,
+                            &t.pn_meta, &t.pn_parent, &t.pn_first, &t.node_zero, &t.nd_test, &t.nd_cell, &t.nd_geo,
+                            &t.nd_parent, &t.grp_node, &t.dep_nodes, &t.leaf_order, &t.grp_range, &t.grp_box,
+                            &t.grp_order, &t.scan_state, &t.scan_ctr})
         h += d->capacity();
     for (int f = 1; f < FRAMES; ++f) h += t.fkey[f].capacity() + t.frunid[f].capacity() + t.fcube[f].capacity();
     return h;

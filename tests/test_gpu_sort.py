@@ -1,7 +1,7 @@
-"""The tree's body sort where its short form can go wrong: sorted by the leading digits of the Morton
+"""The tree's body sort where its short form can go wrong (sorted by the leading digits of the Morton
 keys only, ties ordered where the bodies are gathered, redone with every digit when the tree is
-deeper than that. Keys and permutation equal the oracle's (a stable sort by the whole keys) bit for
-bit."""
+deeper than that), and the build's scans at the edges of their tiles. Keys, permutation, nodes,
+moments and groups equal the oracle's bit for bit."""
 import numpy as np
 import pytest
 
@@ -28,10 +28,18 @@ def same_as_oracle(be, b):
     assert np.array_equal(be.tree_keys(), port.keys())
     assert np.array_equal(be.download().id, port.download().id)
     assert be.times().interactions == port.times()["interactions"] - len(b)
+    rng, mom, geo = be.tree_nodes()
+    pn = port.nodes()
+    assert np.array_equal(rng, np.stack([pn[f] for f in ("lo", "hi", "first", "nchild")], 1))
+    for k, f in enumerate(("cx", "cy", "cz", "m", "qxx", "qxy", "qxz", "qyy", "qyz", "qzz", "rcrit2")):
+        assert np.array_equal(mom[:, k], pn[f]), f
+    box, lohi = be.tree_groups()
+    pg = port.groups()
+    assert np.array_equal(lohi, np.stack([pg["lo"], pg["hi"]], 1))
 
 
-# Around a sort tile (2048) and a histogram block, and where a fixed number of passes ends.
-@pytest.mark.parametrize("n", [1, 2, 17, 255, 257, 511, 513, 2047, 2048, 2049, 4097, 33000])
+# Around the tiles of the sort (2048 bodies), the leaves (1024) and the nodes (256, 1024).
+@pytest.mark.parametrize("n", [1, 2, 17, 255, 257, 1023, 1024, 1025, 2047, 2048, 2049, 4097, 33000])
 def test_sizes(be, n):
     b = zero_v(S.cube(n, 11))
     be.upload(b)
