@@ -28,13 +28,13 @@ namespace lg {
 
 namespace {
 
-#ifndef LG_DIRECT_UNROLL
-#define LG_DIRECT_UNROLL 2  // j-pair iterations unrolled in the inner loop (measured best on GB300)
-#endif
 #ifndef LG_DIRECT_MINB
 #define LG_DIRECT_MINB 1    // resident blocks per SM the register budget is sized for
 #endif
-constexpr int DUNROLL = LG_DIRECT_UNROLL;
+// j-pair iterations unrolled in the inner loop: as many as give eight packed pairs in flight per
+// thread (two i-bodies with four: N = 65537 1.52 ms against 1.66 with two; four i-bodies with two:
+// 1.53 against 1.61 with four).
+constexpr int direct_unroll(int ipt) { return ipt <= 2 ? 4 : 2; }
 constexpr int DBS = 256;   // threads per block
 constexpr int TILE = 256;  // j-bodies per stage (default; 128 is the other compiled shape)
 
@@ -149,6 +149,7 @@ __device__ __forceinline__ void direct_block(DirectSmem<TL>& sm, const float4* _
         const int jt0 = j0 + t * TL;
         auto tile_pairs = [&](auto masked) {
             constexpr bool MASK = decltype(masked)::value;
+            constexpr int DUNROLL = direct_unroll(IPT);
 #pragma unroll DUNROLL
             for (int k = 0; k < cnt8; k += 2) {
                 const f2x X = *reinterpret_cast<const f2x*>(rx + k), Y = *reinterpret_cast<const f2x*>(ry + k);
@@ -290,9 +291,12 @@ int blocks_per_sm(int ipt) {
 
 // Default shape: i-bodies per thread by size, and a split-j count that makes the grid a whole
 // number of waves (blocks resident at once = SMs x blocks per SM), so no partial wave idles SMs.
+// Two i-bodies per thread from 2048 bodies on: as fast as four at every size without the potential
+// (N = 16384: 106 us both, 65537: 1.52 and 1.53 ms), and far faster with it, where four run out of
+// registers for the masked tiles (16384: 130 against 186 us; 5001: 27 against 30).
 DirectShape default_direct_shape(int n, int sms) {
     DirectShape sh;
-    sh.ipt = n >= 8 * 1024 ? 4 : (n >= 2048 ? 2 : 1);
+    sh.ipt = n >= 2048 ? 2 : 1;
     sh.tile = TILE;
     const int iblocks = (n + DBS * sh.ipt - 1) / (DBS * sh.ipt);
     const int wave = blocks_per_sm(sh.ipt) * sms;
