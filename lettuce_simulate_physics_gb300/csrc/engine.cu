@@ -284,10 +284,15 @@ void Engine::compute_forces_with(const lg_force_params& p, bool potential, const
     const float G = static_cast<float>(p.G);
     const float e2 = static_cast<float>(p.eps * p.eps);
     const bool eps0 = !(e2 >= 1.17549435e-38f);  // zero or denormal: guarded pair kernel
-    LG_CK(cudaMemsetAsync(small.as<char>(), 0, 128, stream));
     // Remote trees (other ranks' locally-essential trees) go to the device before the timed part.
     const LetView let = nremote > 0 ? let_upload(*this, remote, nremote) : LetView{};
     const bool have_let = let.ntrees > 0;
+    // The kernels hand what the host reads to page-locked memory themselves and leave the counters
+    // at zero (a clear before and one or two copies after them cost a few us a call): the walk at its
+    // end, the direct kernels only a wait that ran out. The direct method's remote part, two
+    // launches, is copied and cleared here.
+    const bool report = tree_m || !have_let;
+    pinned_small[0] = 0;
     LG_CK(cudaEventRecord(events[EV_WALK0], stream));
     BodyArrays b = bodies(cur);
     NvtxRange walk_range(tree_m ? "lettuce walk" : "lettuce direct");
@@ -295,17 +300,19 @@ void Engine::compute_forces_with(const lg_force_params& p, bool potential, const
         DirectShape sh = direct_shape_override.ipt ? direct_shape_override : default_direct_shape(n, sms);
         int slices = std::max(1, sh.slices);
         if (slices > 1) partial.reserve(static_cast<size_t>(slices) * n * 16 + 16 * 1024);
-        launch_direct(b, n, G, e2, potential, eps0, sh, acc.as<float4>(), partial.as<float4>(), err_word(), stream,
-                      b.cost);
+        launch_direct(b, n, G, e2, potential, eps0, sh, acc.as<float4>(), partial.as<float4>(),
+                      report ? pinned_small : err_word(), stream, b.cost);
         launches += slices > 1 ? 2 : 1;
         // Remote trees per block of 128 consecutive bodies (src/cpu_backend.cpp:695-717).
         if (have_let) tree_walk_remote_blocks(*this, G, e2, potential, eps0, let, let_body_blocks(*this, 128));
     } else {
-        tree_walk(*this, G, e2, potential, eps0, nullptr, nullptr, have_let ? &let : nullptr);
+        tree_walk(*this, G, e2, potential, eps0, nullptr, nullptr, have_let ? &let : nullptr, pinned_small);
     }
     LG_CK(cudaEventRecord(events[EV_WALK1], stream));
-    LG_CK(cudaMemcpyAsync(pinned_small, small.as<char>(), 128, cudaMemcpyDeviceToHost, stream));
-    if (tree_m) LG_CK(cudaMemcpyAsync(pinned_small + 64, tree_counts_device(*this), 32, cudaMemcpyDeviceToHost, stream));
+    if (!report) {
+        LG_CK(cudaMemcpyAsync(pinned_small, small.as<char>(), 128, cudaMemcpyDeviceToHost, stream));
+        LG_CK(cudaMemsetAsync(small.as<char>() + 32, 0, 64, stream));
+    }
     LG_CK(cudaStreamSynchronize(stream));
     if (tree_m && !tree_verify(*this, pinned_small + 64)) {
         // A sync-free build guessed its sizes wrong (or missed a key restart): rebuild exactly and
@@ -324,8 +331,9 @@ void Engine::compute_forces_with(const lg_force_params& p, bool potential, const
     const unsigned long long* cnt = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(pinned_small) + 64);
     // Walk: [0] body pairs (own entry excluded), [1] cell terms; the direct method adds its
     // remote walk's entries to its n (n - 1) pairs.
-    last_body_pairs = tree_m ? cnt[0] : static_cast<uint64_t>(n) * static_cast<uint64_t>(n - 1) + cnt[0];
-    last_cell_terms = cnt[1];
+    const uint64_t walked[2] = {tree_m || have_let ? cnt[0] : 0ull, tree_m || have_let ? cnt[1] : 0ull};
+    last_body_pairs = tree_m ? walked[0] : static_cast<uint64_t>(n) * static_cast<uint64_t>(n - 1) + walked[0];
+    last_cell_terms = walked[1];
     times.interactions = last_body_pairs + last_cell_terms;
     has_pe = potential;
     acc_ok = true;

@@ -197,8 +197,11 @@ const void* probe_kernel();
 // walk.cu
 // sys/e2_sys: forest walk (per-body system, per-system squared softening); nullptr for one tree.
 // let: remote trees walked after the local one (nullptr: none).
+// report: page-locked host memory that receives the error word, the interaction counters (at byte 64)
+// and the tree's counts (at byte 256); the launch then leaves the group and interaction counters at
+// zero, as it needs them. nullptr: the caller clears and reads them.
 void tree_walk(Engine& e, float G, float e2, bool potential, bool eps0, const uint32_t* sys = nullptr,
-               const float* e2_sys = nullptr, const LetView* let = nullptr);
+               const float* e2_sys = nullptr, const LetView* let = nullptr, unsigned* report = nullptr);
 // Remote trees only, for groups given by `blocks` (grp_range, grp_box, ngroups); adds to acc and
 // cost (the direct method's remote part).
 void tree_walk_remote_blocks(Engine& e, float G, float e2, bool potential, bool eps0, const LetView& let,

@@ -95,7 +95,7 @@ struct ZeroSpan {
     uint4* p;
     size_t words;
 };
-constexpr int ZSPANS = 4;
+constexpr int ZSPANS = 5;
 struct ZeroList {
     ZeroSpan span[ZSPANS];
 };
@@ -1777,6 +1777,7 @@ void tree_sort(Engine& e) {
         z.span[1] = {t.hist.as<uint4>(), hist_words()};
         z.span[2] = {t.lookback.as<uint4>(), lookback_words(n, passes)};
         z.span[3] = {t.leaf_state.as<uint4>(), leaf_state_words(n)};
+        z.span[4] = {reinterpret_cast<uint4*>(e.err_word()), 1};  // (the frame kernel's ticket lies behind it)
         if (sys) {
             k_frame_sys<<<t.nsys, BS, 0, s>>>(e.bodies(e.cur), t.sys_off, t.frame.as<double>(), z);
         } else {

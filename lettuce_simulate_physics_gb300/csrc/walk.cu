@@ -105,6 +105,10 @@ struct WalkArgs {
     unsigned* group_ctr;
     unsigned long long* inter;
     unsigned* err;
+    // What the last block to finish hands to the host (see tree_walk), or null.
+    unsigned* report;
+    unsigned* done;
+    const unsigned* counts;
     float G, e2;
     // Forest (ensemble) walk: body -> system (nullptr: one tree rooted at node 0) and the
     // per-system squared softening; system s's tree is rooted at node s.
@@ -591,6 +595,19 @@ __device__ __forceinline__ void build_lists(const WalkArgs& w, WalkSmem& s) {
         if (inter_b) atomicAdd(w.inter, inter_b);
         if (inter_c) atomicAdd(w.inter + 1, inter_c);
     }
+    if (w.report && lane == 0) {
+        __threadfence();
+        if (atomicAdd(w.done, 1u) == gridDim.x - 1u) {  // every list warp has taken its last group
+            unsigned long long* inter = reinterpret_cast<unsigned long long*>(w.report + 16);
+            inter[0] = atomicExch(w.inter, 0ull);
+            inter[1] = atomicExch(w.inter + 1, 0ull);
+            for (int k = 0; k < 8; ++k) w.report[64 + k] = w.counts[k];
+            w.report[0] = atomicOr(w.err, 0u);
+            *w.group_ctr = 0u;
+            *w.done = 0u;
+            __threadfence_system();
+        }
+    }
 }
 
 // ---- the evaluating warps --------------------------------------------------------------------------
@@ -798,8 +815,11 @@ void tree_walk_remote_blocks(Engine& e, float G, float e2, bool potential, bool 
 }
 
 void tree_walk(Engine& e, float G, float e2, bool potential, bool eps0, const uint32_t* sys, const float* e2_sys,
-               const LetView* let) {
+               const LetView* let, unsigned* report) {
     WalkArgs w{};
+    w.report = report;
+    w.done = e.small.as<unsigned>() + 13;
+    w.counts = tree_counts_device(e);
     w.sys = sys;
     w.e2_sys = e2_sys;
     if (let) w.let = *let;

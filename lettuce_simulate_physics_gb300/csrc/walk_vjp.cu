@@ -469,7 +469,7 @@ void tree_walk_vjp(Engine& e, const float4* w, float e2, bool eps0, double* g) {
     e.vjp_scratch.reserve(T * NADJ * 8);
     double* nadj = e.vjp_scratch.as<double>();
     LG_CK(cudaMemsetAsync(nadj, 0, T * NADJ * 8, e.stream));
-    LG_CK(cudaMemsetAsync(e.small.as<char>() + 32, 0, 4, e.stream));
+    LG_CK(cudaMemsetAsync(e.small.as<char>() + 40, 0, 4, e.stream));
     const int blocks = eps0 ? vjp_blocks<true>(e.sms) : vjp_blocks<false>(e.sms);
     e.walk_stack.reserve(static_cast<size_t>(blocks) * VWARPS * SCAP * 4);
     BodyArrays b = e.bodies(e.cur);
@@ -484,7 +484,7 @@ void tree_walk_vjp(Engine& e, const float4* w, float e2, bool eps0, double* g) {
     a.gm = g + 3 * static_cast<size_t>(n);
     a.nadj = nadj;
     a.stack = e.walk_stack.as<uint32_t>();
-    a.group_ctr = reinterpret_cast<unsigned*>(e.small.as<char>() + 32);
+    a.group_ctr = reinterpret_cast<unsigned*>(e.small.as<char>() + 40);
     a.err = e.err_word();
     a.e2 = e2;
     if (eps0) k_walk_vjp<true><<<blocks, VWBS, 0, e.stream>>>(a);
