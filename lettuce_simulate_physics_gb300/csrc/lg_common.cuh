@@ -80,6 +80,31 @@ enum : unsigned {
 constexpr unsigned kSpinCap = 1u << 22;
 
 #ifdef __CUDACC__
+// ---- programmatic dependent launch ----------------------------------------------------------
+// With `overlap`, launches a kernel that may be scheduled while the kernel before it in the stream
+// still runs. Every kernel launched this way begins with pdl_wait(), which lets the next one be
+// scheduled and then waits until the one before has completed with its writes visible: the order of
+// all memory accesses is that of plain launches, only the launch latency is hidden (1 to 2 us a
+// kernel). Without, a plain launch.
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... P, class... A>
+inline void launch_pdl(bool overlap, void (*kernel)(P...), int grid, int block, cudaStream_t s, const A&... args) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.blockDim = dim3(static_cast<unsigned>(block));
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    LG_CK(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 // ---- PTX: MUFU reciprocal square root ------------------------------------------------------
 __device__ __forceinline__ float rsqrt_mufu(float x) {
     float y;

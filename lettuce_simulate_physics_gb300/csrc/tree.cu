@@ -75,6 +75,12 @@ struct FrameTable {
 
 inline int grid_for(long long n, int bs) { return static_cast<int>((n + bs - 1) / bs); }
 
+// Whether a build's kernels overlap their launches. It hides 1 to 2 us a kernel where the kernels are
+// that short, and costs where they run in several waves, as the waiting blocks take the place of
+// running ones. Sort + build, plain -> overlapped, Plummer: 8191 bodies 198 -> 176 us, 65536 242 ->
+// 210, 131072 277 -> 250, 262144 304 -> 337, 4e5 351 -> 412, 1.6e7 5370 -> 6170.
+inline bool overlap(int n) { return n <= 160000; }
+
 // ---- sort control --------------------------------------------------------------------------
 constexpr int RADIX = 256;
 constexpr int PASSES = 8;
@@ -291,6 +297,7 @@ __device__ __forceinline__ void zero_spans(const ZeroList& z) {
 }
 
 __global__ void k_frame(const BodyArrays b, int n, long long* partial, unsigned* ticket, double* frame, ZeroList z) {
+    pdl_wait();
     zero_spans(z);
     __shared__ long long sh[6][BS / 32];
     __shared__ bool last;
@@ -328,6 +335,7 @@ __global__ void k_frame(const BodyArrays b, int n, long long* partial, unsigned*
 __global__ void k_keys(const uint32_t* __restrict__ sys, const BodyArrays b, int n, const double* __restrict__ frame,
                        uint64_t* __restrict__ mkeys, uint64_t* __restrict__ keys, int levels, int passes, int sys_key,
                        unsigned* __restrict__ hist) {
+    pdl_wait();
     __shared__ unsigned h[PASSES * RADIX];
     for (int k = threadIdx.x; k < passes * RADIX; k += blockDim.x) h[k] = 0;
     __syncthreads();
@@ -348,6 +356,7 @@ __global__ void k_keys(const uint32_t* __restrict__ sys, const BodyArrays b, int
 
 // Forest: one block per system computes its key frame over its body range [off[s], off[s + 1]).
 __global__ void k_frame_sys(const BodyArrays b, const uint32_t* __restrict__ off, double* frame, ZeroList z) {
+    pdl_wait();
     zero_spans(z);
     __shared__ long long sh[6][BS / 32];
     const uint32_t lo = off[blockIdx.x], hi = off[blockIdx.x + 1];
@@ -407,6 +416,7 @@ __global__ void __launch_bounds__(SORT_BS) k_sort_pass(const uint64_t* __restric
                                                        int shift, const unsigned* __restrict__ hist,
                                                        unsigned* __restrict__ lookback, unsigned* tile_ctr,
                                                        unsigned* err) {
+    pdl_wait();
     __shared__ unsigned warp_hist[SORT_BS / 32][RADIX];
     __shared__ unsigned gbase[RADIX];       // global start of each digit for this tile
     __shared__ unsigned tstart[RADIX];      // start of each digit in the staged tile
@@ -537,6 +547,7 @@ __global__ void k_permute(const BodyArrays src, BodyArrays dst, const uint64_t* 
                           const uint32_t* __restrict__ vals, const uint64_t* __restrict__ mkeys,
                           uint64_t* __restrict__ skey, const uint64_t* __restrict__ key1_in,
                           uint64_t* __restrict__ key1_out, int n, int n_total, int partial, unsigned* long_run) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_total) return;
     int to = i;
@@ -884,6 +895,7 @@ __global__ void __launch_bounds__(LEAF_BS) k_leaves(const uint32_t* __restrict__
                                                     const FrameTable* ft, int n, int gmax, LeafOut out,
                                                     unsigned long long* state, unsigned* tile_ctr, unsigned* counts,
                                                     unsigned Kcap, unsigned Tcap, ZeroList z, unsigned* err) {
+    pdl_wait();
     // Common prefixes of every window of LEAF_MAX + 1 and of gmax + 1 sorted keys that holds one of
     // the tile's bodies or the one before them; then their maxima over a body's windows.
     __shared__ int8_t c16[LEAF_TILE + 1 + LEAF_MAX];
@@ -1040,6 +1052,7 @@ __device__ __forceinline__ int last_sharing(int a, int end, F&& share) {
 // c[l] that also holds the body before the leaf.
 constexpr int NODE_BS = 256;
 __global__ void __launch_bounds__(NODE_BS) k_nodes(NodeCtx x, PreNodes pn) {
+    pdl_wait();
     __shared__ int l_first;
     if (!build_ok(x.counts)) return;
     const uint32_t T = x.counts[2];
@@ -1113,6 +1126,7 @@ constexpr int NSCAN_BS = 256, NSCAN_IPT = 4, NSCAN_TILE = NSCAN_BS * NSCAN_IPT;
 __global__ void __launch_bounds__(NSCAN_BS) k_node_scan(NodeCtx x, PreNodes pn, unsigned long long* state,
                                                         unsigned* tile_ctr, unsigned* counts, UpsweepIndex* ix,
                                                         uint32_t* grp_node, unsigned* err) {
+    pdl_wait();
     __shared__ unsigned long long warp_sum[NSCAN_BS / 32], prefix_s;
     __shared__ unsigned tile_s, bucket[NBUCKET];
     if (!build_ok(x.counts)) return;
@@ -1198,6 +1212,7 @@ __global__ void __launch_bounds__(NODE_BS) k_nodes_out(NodeCtx x, PreNodes pn, c
                                                        float4* nd_geo, uint32_t* nd_parent, uint32_t* leaf_node,
                                                        UpsweepIndex* ix, uint32_t* dep_nodes, uint32_t* leaf_order,
                                                        unsigned* err) {
+    pdl_wait();
     __shared__ unsigned start[NBUCKET], count[NBUCKET];
     if (!build_ok(x.counts)) return;
     const uint32_t T = x.counts[2], K = x.counts[1];
@@ -1455,6 +1470,7 @@ __device__ void store_moments(Moments mo, uint32_t node, double M, double cx, do
 __global__ void k_leaf_moments(const uint32_t* __restrict__ leaf_order, const unsigned* counts,
                                const float4* __restrict__ nd_geo, const BodyArrays b, Moments mo, float inv_theta,
                                const float* __restrict__ inv_theta_sys, const uint32_t* __restrict__ sys, unsigned* err) {
+    pdl_wait();
     const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
     if (!build_ok(counts)) return;
     const uint32_t T = counts[2];
@@ -1615,6 +1631,7 @@ __global__ void __launch_bounds__(COMBINE_BS) k_combine_level(const uint32_t* __
                                                               const float4* __restrict__ nd_geo, Moments mo,
                                                               float inv_theta, const float* __restrict__ inv_theta_sys,
                                                               const uint32_t* __restrict__ sys, unsigned* err) {
+    pdl_wait();
     if (!build_ok(counts)) return;
     combine_depth<false>(dep_nodes, ix, depth, counts[2], nd_geo, mo, inv_theta, inv_theta_sys, sys,
                          (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5, err);
@@ -1630,6 +1647,7 @@ __global__ void __launch_bounds__(COMBINE_BS) k_combine_top(const uint32_t* __re
                                                             const float4* __restrict__ nd_geo, Moments mo, float inv_theta,
                                                             const float* __restrict__ inv_theta_sys,
                                                             const uint32_t* __restrict__ sys, unsigned* err) {
+    pdl_wait();
     if (!build_ok(counts)) return;  // the same word for all blocks
     for (; depth >= 0; --depth) {
         combine_depth<true>(dep_nodes, ix, depth, counts[2], nd_geo, mo, inv_theta, inv_theta_sys, sys,
@@ -1678,11 +1696,10 @@ int sort_passes(Engine& e, TreeState& t, int n, int passes, bool iota, int pass0
     const int tiles = sort_tiles(n);
     unsigned* hist = t.hist.as<unsigned>();
     for (int p = pass0; p < passes; ++p, from ^= 1) {
-        k_sort_pass<<<tiles, SORT_BS, 0, e.stream>>>(k[from], iota && p == 0 ? nullptr : v[from], k[from ^ 1], v[from ^ 1], n,
-                                                     8 * p, hist + p * RADIX,
-                                                     t.lookback.as<unsigned>() + static_cast<size_t>(p) * tiles * RADIX,
-                                                     hist + PASSES * RADIX + p, e.err_word());
-        LG_LAUNCHED();
+        launch_pdl(overlap(n), k_sort_pass, tiles, SORT_BS, e.stream, k[from],
+                   iota && p == 0 ? nullptr : v[from], k[from ^ 1], v[from ^ 1], n, 8 * p, hist + p * RADIX,
+                   t.lookback.as<unsigned>() + static_cast<size_t>(p) * tiles * RADIX,
+                   hist + PASSES * RADIX + p, e.err_word());
         ++e.launches;
     }
     return from;
@@ -1779,19 +1796,19 @@ void tree_sort(Engine& e) {
         z.span[3] = {t.leaf_state.as<uint4>(), leaf_state_words(n)};
         z.span[4] = {reinterpret_cast<uint4*>(e.err_word()), 1};  // (the frame kernel's ticket lies behind it)
         if (sys) {
-            k_frame_sys<<<t.nsys, BS, 0, s>>>(e.bodies(e.cur), t.sys_off, t.frame.as<double>(), z);
+            launch_pdl(overlap(n), k_frame_sys, t.nsys, BS, s, e.bodies(e.cur), t.sys_off,
+                       t.frame.as<double>(), z);
         } else {
             const int fb = std::min(2 * e.sms, grid_for(n, BS));
             e.diag_partial.reserve(static_cast<size_t>(fb) * 12 * 8);
-            k_frame<<<fb, BS, 0, s>>>(e.bodies(e.cur), n, e.diag_partial.as<long long>(), e.ticket(),
-                                      t.frame.as<double>(), z);
+            launch_pdl(overlap(n), k_frame, fb, BS, s, e.bodies(e.cur), n, e.diag_partial.as<long long>(),
+                       e.ticket(), t.frame.as<double>(), z);
         }
         LG_LAUNCHED();
         // With every digit sorted the system index does not fit beside them: it is sorted on its own.
-        k_keys<<<std::min(2 * e.sms, grid_for(n, 512)), 512, 0, s>>>(
-            sys, e.bodies(e.cur), n, t.frame.as<double>(), t.mkeys.as<uint64_t>(), t.keysA.as<uint64_t>(), levels, passes,
-            sys && !full ? 1 : 0, t.hist.as<unsigned>());
-        LG_LAUNCHED();
+        launch_pdl(overlap(n), k_keys, std::min(2 * e.sms, grid_for(n, 512)), 512, s, sys, e.bodies(e.cur),
+                   n, t.frame.as<double>(), t.mkeys.as<uint64_t>(), t.keysA.as<uint64_t>(), levels, passes,
+                   sys && !full ? 1 : 0, t.hist.as<unsigned>());
         e.launches += 2;
         int at = sort_passes(e, t, n, passes, true);
         if (full && sys) {
@@ -1802,11 +1819,10 @@ void tree_sort(Engine& e) {
             at = 0;
         }
         const int other = e.cur ^ 1;
-        k_permute<<<grid_for(n_total, BS), BS, 0, s>>>(
-            e.bodies(e.cur), e.bodies(other), at ? t.keysB.as<uint64_t>() : t.keysA.as<uint64_t>(),
-            at ? t.valsB.as<uint32_t>() : t.valsA.as<uint32_t>(), t.mkeys.as<uint64_t>(), t.skey.as<uint64_t>(), nullptr,
-            nullptr, n, n_total, full ? 0 : 1, counts + 7);
-        LG_LAUNCHED();
+        launch_pdl(overlap(n), k_permute, grid_for(n_total, BS), BS, s, e.bodies(e.cur), e.bodies(other),
+                   at ? t.keysB.as<uint64_t>() : t.keysA.as<uint64_t>(),
+                   at ? t.valsB.as<uint32_t>() : t.valsA.as<uint32_t>(), t.mkeys.as<uint64_t>(),
+                   t.skey.as<uint64_t>(), nullptr, nullptr, n, n_total, full ? 0 : 1, counts + 7);
         ++e.launches;
         e.cur = other;
         if (full) {
@@ -1867,10 +1883,9 @@ void tree_sort(Engine& e) {
         LG_LAUNCHED();
         sort_pairs(e, t, n, false);
         const int other = e.cur ^ 1;
-        k_permute<<<grid_for(n_total, BS), BS, 0, s>>>(e.bodies(e.cur), e.bodies(other), t.keysA.as<uint64_t>(),
-                                                       t.valsA.as<uint32_t>(), nullptr, nullptr, key1,
-                                                       t.fkey[f].as<uint64_t>(), n, n_total, 0, nullptr);
-        LG_LAUNCHED();
+        launch_pdl(overlap(n), k_permute, grid_for(n_total, BS), BS, s, e.bodies(e.cur), e.bodies(other),
+                   t.keysA.as<uint64_t>(), t.valsA.as<uint32_t>(), nullptr, nullptr, key1,
+                   t.fkey[f].as<uint64_t>(), n, n_total, 0, nullptr);
         e.cur = other;
         ft.key[f] = t.fkey[f].as<uint64_t>();
         ft.runid[f] = runid;
@@ -1920,10 +1935,10 @@ void tree_build(Engine& e, double theta) {
                        t.leaf_depth.as<uint8_t>(), t.leaf_gdepth.as<uint8_t>(), t.leaf_c.as<int8_t>()};
     auto leaves = [&](unsigned Kcap, unsigned Tcap, const ZeroList& z) {
         const int tiles = leaf_tiles(n);
-        k_leaves<<<tiles, LEAF_BS, 0, s>>>(sys, k0, ft, n, t.group_max, leaf, t.leaf_state.as<unsigned long long>(),
-                                           t.leaf_state.as<unsigned>() + 2 * static_cast<size_t>(tiles), counts, Kcap,
-                                           Tcap, z, e.err_word());
-        LG_LAUNCHED();
+        launch_pdl(overlap(n), k_leaves, tiles, LEAF_BS, s, sys, k0, ft, n, t.group_max, leaf,
+                   t.leaf_state.as<unsigned long long>(),
+                   t.leaf_state.as<unsigned>() + 2 * static_cast<size_t>(tiles), counts, Kcap, Tcap, z,
+                   e.err_word());
         ++e.launches;
     };
     if (!spec) {
@@ -1986,11 +2001,10 @@ void tree_build(Engine& e, double theta) {
     const NodeCtx x{sys, k0, ft, leaf, n, counts, static_cast<unsigned>(sys ? t.nsys : 1)};
     const uint32_t Tc = static_cast<uint32_t>(T);
     const int tb = grid_for(static_cast<long long>(T), NODE_BS);
-    k_nodes<<<tb, NODE_BS, 0, s>>>(x, pn);
-    LG_LAUNCHED();
-    k_node_scan<<<scan_tiles, NSCAN_BS, 0, s>>>(x, pn, scan_state, reinterpret_cast<unsigned*>(scan_state + scan_tiles),
-                                                counts, ix, t.grp_node.as<uint32_t>(), e.err_word());
-    LG_LAUNCHED();
+    launch_pdl(overlap(n), k_nodes, tb, NODE_BS, s, x, pn);
+    launch_pdl(overlap(n), k_node_scan, scan_tiles, NSCAN_BS, s, x, pn, scan_state,
+               reinterpret_cast<unsigned*>(scan_state + scan_tiles), counts, ix, t.grp_node.as<uint32_t>(),
+               e.err_word());
     e.launches += 2;
     // The group boxes depend neither on the nodes' order nor on the moments: with the reference groups
     // they are computed on the side stream from here on, and joined back before the build returns.
@@ -2012,10 +2026,10 @@ void tree_build(Engine& e, double theta) {
         ++e.launches;
         LG_CK(cudaEventRecord(e.join_ev, e.side));
     }
-    k_nodes_out<<<tb, NODE_BS, 0, s>>>(x, pn, t.frame.as<double>(), t.nd_test.as<NodeTest>(), t.nd_geo.as<float4>(),
-                                       t.nd_parent.as<uint32_t>(), t.leaf_node.as<uint32_t>(), ix,
-                                       t.dep_nodes.as<uint32_t>(), t.leaf_order.as<uint32_t>(), e.err_word());
-    LG_LAUNCHED();
+    launch_pdl(overlap(n), k_nodes_out, tb, NODE_BS, s, x, pn, t.frame.as<double>(),
+               t.nd_test.as<NodeTest>(), t.nd_geo.as<float4>(), t.nd_parent.as<uint32_t>(),
+               t.leaf_node.as<uint32_t>(), ix, t.dep_nodes.as<uint32_t>(), t.leaf_order.as<uint32_t>(),
+               e.err_word());
     ++e.launches;
     if (t.merged) {
         t.mcount.reserve(T * 4 + 4);
@@ -2039,10 +2053,9 @@ void tree_build(Engine& e, double theta) {
     // most TOP_NODES nodes (by the eight-way branching, or because the whole tree is small) together.
     const float inv_theta = theta > 0 ? static_cast<float>(1.0 / theta) : FLT_MAX;
     Moments mo{t.nd_test.as<NodeTest>(), t.nd_cell.as<NodeCell>()};
-    k_leaf_moments<<<grid_for(static_cast<long long>(K), 128), 128, 0, s>>>(
-        t.leaf_order.as<uint32_t>(), counts, t.nd_geo.as<float4>(), e.bodies(e.cur), mo, inv_theta, t.inv_theta_sys, sys,
-        e.err_word());
-    LG_LAUNCHED();
+    launch_pdl(overlap(n), k_leaf_moments, grid_for(static_cast<long long>(K), 128), 128, s,
+               t.leaf_order.as<uint32_t>(), counts, t.nd_geo.as<float4>(), e.bodies(e.cur), mo, inv_theta,
+               t.inv_theta_sys, sys, e.err_word());
     ++e.launches;
     int top = -1;
     if (T <= 8 * TOP_NODES) top = depth - 1;
@@ -2050,22 +2063,23 @@ void tree_build(Engine& e, double theta) {
         for (size_t width = x.nroots; width <= TOP_NODES && top < depth - 1; width *= 8) ++top;
     const int cb = std::max(1, std::min(2 * e.sms, grid_for(static_cast<long long>(T), COMBINE_NODES)));
     for (int d = depth - 1; d > top; --d) {
-        k_combine_level<<<cb, COMBINE_BS, 0, s>>>(t.dep_nodes.as<uint32_t>(), ix, d, counts, t.nd_geo.as<float4>(), mo,
-                                                  inv_theta, t.inv_theta_sys, sys, e.err_word());
-        LG_LAUNCHED();
+        launch_pdl(overlap(n), k_combine_level, cb, COMBINE_BS, s, t.dep_nodes.as<uint32_t>(), ix, d,
+                   counts, t.nd_geo.as<float4>(), mo, inv_theta, t.inv_theta_sys, sys, e.err_word());
         ++e.launches;
     }
     if (top >= 0) {
         cudaLaunchConfig_t cfg{};
-        cudaLaunchAttribute at{};
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = TOP_BLOCKS;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchAttribute at[2] = {};
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = TOP_BLOCKS;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.gridDim = dim3(TOP_BLOCKS);
         cfg.blockDim = dim3(COMBINE_BS);
         cfg.stream = s;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = overlap(n) ? 2 : 1;
         LG_CK(cudaLaunchKernelEx(&cfg, k_combine_top, static_cast<const uint32_t*>(t.dep_nodes.as<uint32_t>()),
                                  static_cast<const UpsweepIndex*>(ix), top, static_cast<const unsigned*>(counts),
                                  static_cast<const float4*>(t.nd_geo.as<float4>()), mo, inv_theta, t.inv_theta_sys, sys,
