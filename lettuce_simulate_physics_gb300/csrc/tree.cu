@@ -1508,159 +1508,306 @@ __global__ void k_leaf_moments(const uint32_t* __restrict__ leaf_order, const un
     store_moments(mo, node, M, cx, cy, cz, qxx, qxy, qxz, qyy, qyz, qzz, g, inv_theta);
 }
 
-// Internal nodes of one depth: combine the children (already final) in index order, FP64, the
-// parallel-axis theorem for the traceless quadrupole (src/cpu_backend.cpp:642-663).
-// Four lanes per node, eight nodes per warp. Lane j forms the terms of children j and j + 4 (the
-// per-child FP64 work runs in parallel); each of the reference's sequential child-order sums is
-// then folded by one lane only, from terms shuffled in child order: M, sx, sy, sz by lanes 0..3;
-// qxx and qyy by lane 0, qzz and qxy by lane 1, qxz by lane 2, qyz by lane 3. Lanes 1..3 divide
-// their first sum by M together. Every FP64 operation of the reference, as its compiler forms it
-// (fused multiply-adds included), is done once, in its order, so the moments are the reference's
-// bit for bit. (On this part an FP64 warp instruction holds a
-// scheduler's FP64 unit for about 64 cycles: the form keeps the number of FP64 warp instructions
-// per node low and spreads the nodes of a level over all schedulers.)
-__device__ __forceinline__ double shfl_d(double v, int src_lane) { return __shfl_sync(0xffffffffu, v, src_lane); }
+// Eight lanes per node or leaf, four of them per warp: lane j holds child (or body) j's terms, lays
+// them out in rows of the warp's shared memory, one row per sum, and folds row j in order. On this
+// part an FP64 warp instruction holds a scheduler's FP64 unit for about 64 cycles whatever its active
+// lanes, so the chain that counts is that of FP64 warp instructions: the terms are formed once, side
+// by side, the sums that must be sequential run beside each other, one per lane, and each lane
+// rounds and stores its own results. A row is 10 doubles long: 16-byte reads without conflicts.
+constexpr int WIDE = 8, ROW = 10;
 
-constexpr int COMBINE_BS = 128;
-constexpr int COMBINE_NODES = COMBINE_BS / 4;  // nodes per block and round
-
-// The nodes of one depth, taken by `warps` warps of which this is number wid. FAR: the children were
-// written by other SMs in the same launch and are read past the L1 cache.
-template <bool FAR>
-__device__ __forceinline__ void combine_depth(const uint32_t* __restrict__ dep_nodes, const UpsweepIndex* ix, int depth,
-                                              uint32_t T, const float4* __restrict__ nd_geo, const Moments& mo,
-                                              float inv_theta, const float* __restrict__ inv_theta_sys,
-                                              const uint32_t* __restrict__ sys, unsigned wid, unsigned warps, unsigned* err) {
-    const unsigned lo = ix->off[depth], hi = depth + 1 < NDEP ? ix->off[depth + 1] : lo;
-    const int lane = threadIdx.x & 31, j = lane & 3, base = lane & ~3;
-    for (unsigned k0 = lo + 8 * wid; k0 < hi; k0 += 8 * warps) {  // warp-uniform
-        const unsigned k = k0 + static_cast<unsigned>(lane >> 2);
-        bool valid = k < hi;
-        uint32_t p = valid ? dep_nodes[k] : 0u;
-        uint4 r = make_uint4(0, 0, 0, 0);
-        if (valid) {
-            if (p >= T) {
-                if (j == 0) atomicOr(err, kErrNodeOverflow);
-                valid = false;
-            } else {
-                r = mo.test[p].range;
-                if (r.w == 0 || r.w > 8 || r.z + r.w > T) {
-                    if (j == 0) atomicOr(err, kErrNodeOverflow);
-                    valid = false;
-                }
-            }
-        }
-        const int nch = valid ? static_cast<int>(r.w) : 0;
-        // Terms of the lane's children c = j + 4 sl (zeros past the last child: never added).
-        double m[2], ccx[2], ccy[2], ccz[2], mx[2], my[2], mz[2];
-        float4 qa[2], qb[2];
+__device__ __forceinline__ void load_row(const double* row, double (&v)[WIDE]) {
+    const double2* p = reinterpret_cast<const double2*>(row);
 #pragma unroll
-        for (int sl = 0; sl < 2; ++sl) {
-            const int c = j + 4 * sl;
-            float4 cm = make_float4(0.f, 0.f, 0.f, 0.f);
-            qa[sl] = cm;
-            qb[sl] = cm;
-            if (c < nch) {
-                const NodeCell* ch = mo.cell + r.z + c;
-                cm = FAR ? __ldcg(&ch->com) : ch->com;
-                qa[sl] = FAR ? __ldcg(&ch->q0) : ch->q0;
-                qb[sl] = FAR ? __ldcg(&ch->q1) : ch->q1;
-            }
-            m[sl] = cm.w;
-            ccx[sl] = cm.x;
-            ccy[sl] = cm.y;
-            ccz[sl] = cm.z;
-            mx[sl] = DMUL(m[sl], ccx[sl]);
-            my[sl] = DMUL(m[sl], ccy[sl]);
-            mz[sl] = DMUL(m[sl], ccz[sl]);
-        }
-        // Monopole sums in child order: lane j folds M (0), sx (1), sy (2), sz (3).
-        double f1 = 0;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int src = base + (q & 3), sl = q >> 2;
-            const double vm = shfl_d(m[sl], src), vx = shfl_d(mx[sl], src), vy = shfl_d(my[sl], src),
-                         vz = shfl_d(mz[sl], src);
-            const double v = j == 0 ? vm : j == 1 ? vx : j == 2 ? vy : vz;
-            if (q < nch) f1 = DADD(f1, v);
-        }
-        const double M = shfl_d(f1, base);
-        const float4 g = valid ? nd_geo[p] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float gj = j == 1 ? g.x : j == 2 ? g.y : g.z;
-        const double cj = M > 0 ? __ddiv_rn(f1, M) : static_cast<double>(gj);  // lane 0's is unused
-        const double cx = shfl_d(cj, base + 1), cy = shfl_d(cj, base + 2), cz = shfl_d(cj, base + 3);
-        // Quadrupole terms of the lane's children about the new centre.
-        double txx[2], tyy[2], tzz[2], txy[2], txz[2], tyz[2];
-#pragma unroll
-        for (int sl = 0; sl < 2; ++sl) {
-            const double dx = DSUB(ccx[sl], cx), dy = DSUB(ccy[sl], cy), dz = DSUB(ccz[sl], cz);
-            const double r2 = DFMA(dz, dz, DFMA(dx, dx, DMUL(dy, dy)));
-            const double m3 = DMUL(m[sl], 3.0);
-            txx[sl] = DFMA(m[sl], DFMA(DMUL(3.0, dx), dx, -r2), static_cast<double>(qa[sl].x));
-            tyy[sl] = DFMA(m[sl], DFMA(DMUL(3.0, dy), dy, -r2), static_cast<double>(qa[sl].w));
-            tzz[sl] = DFMA(m[sl], DFMA(DMUL(3.0, dz), dz, -r2), static_cast<double>(qb[sl].y));
-            txy[sl] = DFMA(DMUL(m3, dx), dy, static_cast<double>(qa[sl].y));
-            txz[sl] = DFMA(DMUL(m3, dx), dz, static_cast<double>(qa[sl].z));
-            tyz[sl] = DFMA(DMUL(m3, dy), dz, static_cast<double>(qb[sl].x));
-        }
-        // Quadrupole sums in child order: lane 0 folds qxx and qyy, lane 1 qzz and qxy, lane 2 qxz,
-        // lane 3 qyz.
-        double fa = 0, fb = 0;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int src = base + (q & 3), sl = q >> 2;
-            const double vxx = shfl_d(txx[sl], src), vyy = shfl_d(tyy[sl], src), vzz = shfl_d(tzz[sl], src),
-                         vxy = shfl_d(txy[sl], src), vxz = shfl_d(txz[sl], src), vyz = shfl_d(tyz[sl], src);
-            const double va = j == 0 ? vxx : j == 1 ? vzz : j == 2 ? vxz : vyz;
-            const double vb = j == 0 ? vyy : vxy;
-            if (q < nch) {
-                fa = DADD(fa, va);
-                if (j < 2) fb = DADD(fb, vb);
-            }
-        }
-        const double qzz = shfl_d(fa, base + 1), qxy = shfl_d(fb, base + 1), qxz = shfl_d(fa, base + 2),
-                     qyz = shfl_d(fa, base + 3);
-        if (valid && j == 0)
-            store_moments(mo, p, M, cx, cy, cz, fa, qxy, qxz, fb, qyz, qzz, g,
-                          inv_theta_sys ? inv_theta_sys[sys_of(sys, static_cast<int>(r.x))] : inv_theta);
+    for (int q = 0; q < WIDE / 2; ++q) {
+        const double2 d = p[q];
+        v[2 * q] = d.x;
+        v[2 * q + 1] = d.y;
     }
 }
 
+__device__ __forceinline__ double shfl_d(double v, int src_lane) { return __shfl_sync(0xffffffffu, v, src_lane); }
+
+// A node's floats from its eight lanes: f1 / M, that is the centre's coordinate j, on lanes 1..3 (lane
+// 0: M itself); the quadrupole's sum j on lanes 0..5. The opening radius is stored by store_rcrit.
+__device__ __forceinline__ void store_wide(const Moments& mo, uint32_t node, int j, double M, double cj, double q) {
+    float* c = reinterpret_cast<float*>(mo.cell + node);  // com.xyz m, lo.xyz 0, q0, q1
+    const double v = j == 0 ? M : cj;
+    const float f = static_cast<float>(v);
+    const float l = static_cast<float>(__dsub_rn(v, static_cast<double>(f)));
+    const float fq = static_cast<float>(q);
+    if (j < 4) {
+        c[(j + 3) & 3] = f;
+        c[4 + ((j + 3) & 3)] = j ? l : 0.f;
+    }
+    if (j != 6) c[8 + j] = j < 6 ? fq : 0.f;  // q1.z is the opening radius
+}
+
+__device__ __forceinline__ void store_rcrit(const Moments& mo, uint32_t node, float4 com, float4 g, float inv_theta) {
+    const float rc2 = rcrit2_of(com.x, com.y, com.z, g, inv_theta);
+    mo.test[node].com = make_float4(com.x, com.y, com.z, rc2);
+    mo.cell[node].q1.z = rc2;
+}
+
+// k_leaf_moments for the trees whose leaves are too few to fill the FP64 units one to a thread, where
+// a leaf's chain of about 40 FP64 instructions per body is the time (8191 bodies: 27 -> 10 us). Bodies
+// in rounds of eight. The two folds of a body leave lanes idle, so more FP64 work is issued in all,
+// hence the line (build phase with a thread -> eight lanes per leaf: 8191 bodies 108 -> 90 us, 25000, of 4e3
+// leaves, 129 -> 123, 40000, of 6.4e3, 141 -> 147).
+constexpr int LEAFW_BS = 128;
+constexpr size_t LEAFW_MAX = 4096;
+__global__ void __launch_bounds__(LEAFW_BS) k_leaf_moments_wide(const uint32_t* __restrict__ leaf_order,
+                                                                const unsigned* counts,
+                                                                const float4* __restrict__ nd_geo,
+                                                                const BodyArrays b, Moments mo, float inv_theta,
+                                                                const float* __restrict__ inv_theta_sys,
+                                                                const uint32_t* __restrict__ sys, unsigned* err) {
+    __shared__ __align__(16) double rows[LEAFW_BS / WIDE][8][ROW];
+    pdl_wait();
+    if (!build_ok(counts)) return;
+    const uint32_t T = counts[2], K = counts[1];
+    const int lane = threadIdx.x & 31, j = lane & 7, base = lane & ~7;
+    double(*row)[ROW] = rows[threadIdx.x / WIDE];
+    const uint32_t l = (blockIdx.x * LEAFW_BS + threadIdx.x) / WIDE;
+    uint32_t node = l < K ? leaf_order[l] : 0u;
+    bool valid = l < K;
+    if (valid && node >= T) {
+        if (j == 0) atomicOr(err, kErrNodeOverflow);
+        valid = false;
+        node = 0;
+    }
+    uint4 r = make_uint4(0, 0, 0, 0);
+    float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (valid) {
+        r = mo.test[node].range;
+        g = nd_geo[node];
+    }
+    const int nb = static_cast<int>(r.y - r.x);
+    const int rounds = __reduce_max_sync(0xffffffffu, (nb + WIDE - 1) / WIDE);
+    double f1 = 0;
+    double v[WIDE];
+    for (int q0 = 0; q0 < rounds; ++q0) {
+        const int at = WIDE * q0 + j;
+        const uint32_t i = r.x + at;
+        const bool on = at < nb;
+        const double m = on ? b.m[i] : 0.f, x = on ? b.x[i] : 0.f, y = on ? b.y[i] : 0.f, z = on ? b.z[i] : 0.f;
+        row[0][j] = m;
+        row[1][j] = DMUL(m, x);
+        row[2][j] = DMUL(m, y);
+        row[3][j] = DMUL(m, z);
+        __syncwarp();
+        load_row(row[j & 3], v);
+#pragma unroll
+        for (int q = 0; q < WIDE; ++q)
+            if (WIDE * q0 + q < nb) f1 = DADD(f1, v[q]);
+        __syncwarp();
+    }
+    const double M = shfl_d(f1, base);
+    const double cj = M > 0 ? __ddiv_rn(f1, M) : static_cast<double>(j == 1 ? g.x : j == 2 ? g.y : g.z);
+    const double cx = shfl_d(cj, base + 1), cy = shfl_d(cj, base + 2), cz = shfl_d(cj, base + 3);
+    // Each sum is a chain of fused multiply-adds: its factors are laid out, m or m3 dx or m3 dy, and
+    // the axis terms or dy or dz.
+    const int ra = j == 1 || j == 2 ? 1 : j == 4 ? 2 : 0;
+    const int rb = j == 0 ? 3 : j == 1 ? 6 : j == 3 ? 4 : j == 5 ? 5 : 7;
+    double fq = 0;
+    for (int q0 = 0; q0 < rounds; ++q0) {
+        const int at = WIDE * q0 + j;
+        const uint32_t i = r.x + at;
+        const bool on = at < nb;
+        const double m = on ? b.m[i] : 0.f, dx = DSUB(on ? b.x[i] : 0.f, cx), dy = DSUB(on ? b.y[i] : 0.f, cy),
+                     dz = DSUB(on ? b.z[i] : 0.f, cz);
+        const double r2 = DFMA(dz, dz, DFMA(dx, dx, DMUL(dy, dy)));
+        const double m3 = DMUL(m, 3.0);
+        row[0][j] = m;
+        row[1][j] = DMUL(m3, dx);
+        row[2][j] = DMUL(m3, dy);
+        row[3][j] = DFMA(DMUL(3.0, dx), dx, -r2);
+        row[4][j] = DFMA(DMUL(3.0, dy), dy, -r2);
+        row[5][j] = DFMA(DMUL(3.0, dz), dz, -r2);
+        row[6][j] = dy;
+        row[7][j] = dz;
+        __syncwarp();
+        double u[WIDE];
+        load_row(row[ra], u);
+        load_row(row[rb], v);
+#pragma unroll
+        for (int q = 0; q < WIDE; ++q)
+            if (WIDE * q0 + q < nb) fq = DFMA(u[q], v[q], fq);
+        __syncwarp();
+    }
+    if (!valid) return;
+    store_wide(mo, node, j, M, cj, fq);
+    if (j == 0) {
+        if (inv_theta_sys) inv_theta = inv_theta_sys[sys_of(sys, static_cast<int>(r.x))];
+        store_rcrit(mo, node,
+                    make_float4(static_cast<float>(cx), static_cast<float>(cy), static_cast<float>(cz), 0.f), g,
+                    inv_theta);
+    }
+}
+
+// Internal nodes of one depth: combine the children (already final) in index order, FP64, the
+// parallel-axis theorem for the traceless quadrupole (src/cpu_backend.cpp:642-663). Lane j forms the
+// terms of child j; each of the reference's sequential child-order sums is then folded by one lane:
+// M, sx, sy, sz by lanes 0..3, which divide by M together, the quadrupole's by lanes 0..5. Every FP64
+// operation of the reference, as its compiler forms it (fused multiply-adds included), is done once,
+// in its order, so the moments are the reference's bit for bit. The opening radius, which no parent
+// reads, costs a square root: it is left to rcrit_range, a lane per node.
+constexpr int COMBINE_BS = 128, TOP_BS = 256;
+constexpr int COMBINE_NODES = COMBINE_BS / WIDE;  // nodes per block and round
+
+// What a lane needs of its node before the children are final.
+struct CombineNode {
+    uint32_t p, first;
+    int nch;  // 0: nothing to do
+    float4 g;
+};
+
+__device__ __forceinline__ CombineNode combine_fetch(const uint32_t* __restrict__ dep_nodes, unsigned k, unsigned hi,
+                                                     uint32_t T, const float4* __restrict__ nd_geo, const Moments& mo,
+                                                     unsigned* err) {
+    CombineNode c{0u, 0u, 0, make_float4(0.f, 0.f, 0.f, 0.f)};
+    if (k >= hi) return c;
+    c.p = dep_nodes[k];
+    if (c.p < T) {
+        const uint4 r = mo.test[c.p].range;
+        c.g = nd_geo[c.p];
+        if (r.w != 0 && r.w <= 8 && r.z + r.w <= T) {
+            c.first = r.z;
+            c.nch = static_cast<int>(r.w);
+            return c;
+        }
+    }
+    if ((threadIdx.x & 7) == 0) atomicOr(err, kErrNodeOverflow);
+    return c;
+}
+
+// One node per eight lanes; row: their ten rows. FAR: the children were written by other SMs in the
+// same launch and are read past the L1 cache.
+template <bool FAR>
+__device__ __forceinline__ void combine_node(const CombineNode& n, double (*row)[ROW], const Moments& mo) {
+    const int lane = threadIdx.x & 31, j = lane & 7, base = lane & ~7;
+    float4 cm = make_float4(0.f, 0.f, 0.f, 0.f), qa = cm, qb = cm;  // zeros past the last child: never added
+    if (j < n.nch) {
+        const NodeCell* ch = mo.cell + n.first + j;
+        cm = FAR ? __ldcg(&ch->com) : ch->com;
+        qa = FAR ? __ldcg(&ch->q0) : ch->q0;
+        qb = FAR ? __ldcg(&ch->q1) : ch->q1;
+    }
+    const double m = cm.w, x = cm.x, y = cm.y, z = cm.z;
+    row[0][j] = m;
+    row[1][j] = DMUL(m, x);
+    row[2][j] = DMUL(m, y);
+    row[3][j] = DMUL(m, z);
+    __syncwarp();
+    double v[WIDE];
+    load_row(row[j & 3], v);
+    double f1 = 0;
+#pragma unroll
+    for (int q = 0; q < WIDE; ++q)
+        if (q < n.nch) f1 = DADD(f1, v[q]);
+    const double M = shfl_d(f1, base);
+    const double cj = M > 0 ? __ddiv_rn(f1, M) : static_cast<double>(j == 1 ? n.g.x : j == 2 ? n.g.y : n.g.z);
+    const double cx = shfl_d(cj, base + 1), cy = shfl_d(cj, base + 2), cz = shfl_d(cj, base + 3);
+    // The child's quadrupole about the new centre.
+    const double dx = DSUB(x, cx), dy = DSUB(y, cy), dz = DSUB(z, cz);
+    const double r2 = DFMA(dz, dz, DFMA(dx, dx, DMUL(dy, dy)));
+    const double m3 = DMUL(m, 3.0);
+    row[4][j] = DFMA(m, DFMA(DMUL(3.0, dx), dx, -r2), static_cast<double>(qa.x));
+    row[5][j] = DFMA(DMUL(m3, dx), dy, static_cast<double>(qa.y));
+    row[6][j] = DFMA(DMUL(m3, dx), dz, static_cast<double>(qa.z));
+    row[7][j] = DFMA(m, DFMA(DMUL(3.0, dy), dy, -r2), static_cast<double>(qa.w));
+    row[8][j] = DFMA(DMUL(m3, dy), dz, static_cast<double>(qb.x));
+    row[9][j] = DFMA(m, DFMA(DMUL(3.0, dz), dz, -r2), static_cast<double>(qb.y));
+    __syncwarp();
+    load_row(row[4 + min(j, 5)], v);
+    double fq = 0;
+#pragma unroll
+    for (int q = 0; q < WIDE; ++q)
+        if (q < n.nch) fq = DADD(fq, v[q]);
+    if (n.nch) store_wide(mo, n.p, j, M, cj, fq);
+    __syncwarp();  // the rows are free again
+}
+
+// Opening radii of the internal nodes dep_nodes[lo, hi), a lane each, once their centres are final.
+__device__ __forceinline__ void rcrit_range(const uint32_t* __restrict__ dep_nodes, unsigned lo, unsigned hi, uint32_t T,
+                                            const float4* __restrict__ nd_geo, const Moments& mo, float inv_theta,
+                                            const float* __restrict__ inv_theta_sys, const uint32_t* __restrict__ sys,
+                                            unsigned tid, unsigned threads) {
+    for (unsigned k = lo + tid; k < hi; k += threads) {
+        const uint32_t p = dep_nodes[k];
+        if (p >= T) continue;  // reported by combine_fetch
+        const float th = inv_theta_sys ? inv_theta_sys[sys_of(sys, static_cast<int>(mo.test[p].range.x))] : inv_theta;
+        store_rcrit(mo, p, __ldcg(&mo.cell[p].com), nd_geo[p], th);
+    }
+}
+
+__device__ __forceinline__ unsigned dep_begin(const UpsweepIndex* ix, int depth) {  // of a depth's list
+    return ix->off[min(depth, NDEP - 1)];
+}
+
+// One depth, and the opening radii of the depth below it.
 __global__ void __launch_bounds__(COMBINE_BS) k_combine_level(const uint32_t* __restrict__ dep_nodes,
                                                               const UpsweepIndex* ix, int depth, const unsigned* counts,
                                                               const float4* __restrict__ nd_geo, Moments mo,
                                                               float inv_theta, const float* __restrict__ inv_theta_sys,
                                                               const uint32_t* __restrict__ sys, unsigned* err) {
+    __shared__ __align__(16) double rows[COMBINE_NODES][ROW][ROW];
     pdl_wait();
     if (!build_ok(counts)) return;
-    combine_depth<false>(dep_nodes, ix, depth, counts[2], nd_geo, mo, inv_theta, inv_theta_sys, sys,
-                         (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5, err);
+    const uint32_t T = counts[2];
+    const unsigned lo = dep_begin(ix, depth), hi = dep_begin(ix, depth + 1), end = dep_begin(ix, depth + 2);
+    const unsigned sub = threadIdx.x / WIDE, of = gridDim.x * COMBINE_NODES;
+    for (unsigned k = lo + blockIdx.x * COMBINE_NODES; k < hi; k += of)
+        combine_node<false>(combine_fetch(dep_nodes, k + sub, hi, T, nd_geo, mo, err), rows[sub], mo);
+    rcrit_range(dep_nodes, hi, end, T, nd_geo, mo, inv_theta, inv_theta_sys, sys,
+                blockIdx.x * COMBINE_BS + threadIdx.x, gridDim.x * COMBINE_BS);
 }
 
-// The depths from `depth` up to the root in one launch of one cluster of 16 blocks (one warp per
-// scheduler of 16 SMs), a cluster barrier between depths: a depth of up to 512 nodes is one round of
-// the FP64 chain (about 4 us) whether it has its own launch or not, and the barrier costs less than
-// the launch.
-constexpr int TOP_BLOCKS = 16, TOP_NODES = TOP_BLOCKS * COMBINE_NODES;
-__global__ void __launch_bounds__(COMBINE_BS) k_combine_top(const uint32_t* __restrict__ dep_nodes, const UpsweepIndex* ix,
-                                                            int depth, const unsigned* counts,
-                                                            const float4* __restrict__ nd_geo, Moments mo, float inv_theta,
-                                                            const float* __restrict__ inv_theta_sys,
-                                                            const uint32_t* __restrict__ sys, unsigned* err) {
+// The depths from `depth` up to the root in one launch of one cluster of 16 blocks, a cluster barrier
+// between depths: a depth of up to 512 nodes is one round of the FP64 chain whether it has its own
+// launch or not, and the barrier costs less than the launch. What is known of a depth's nodes before
+// their children are final is read ahead of the barrier, and all opening radii are formed at the end:
+// 4.9 us a depth (8.7 with four lanes to a node, the radii inside and all loads after the barrier).
+constexpr int TOP_BLOCKS = 16, TOP_NODES = TOP_BLOCKS * (TOP_BS / WIDE);
+__global__ void __launch_bounds__(TOP_BS) k_combine_top(const uint32_t* __restrict__ dep_nodes, const UpsweepIndex* ix,
+                                                        int depth, const unsigned* counts,
+                                                        const float4* __restrict__ nd_geo, Moments mo, float inv_theta,
+                                                        const float* __restrict__ inv_theta_sys,
+                                                        const uint32_t* __restrict__ sys, unsigned* err) {
+    __shared__ __align__(16) double rows[TOP_BS / WIDE][ROW][ROW];
     pdl_wait();
     if (!build_ok(counts)) return;  // the same word for all blocks
+    const uint32_t T = counts[2];
+    const unsigned sub = threadIdx.x / WIDE;
+    // Nodes in order go to the blocks' first warps, then to their second: a narrow depth is spread
+    // over all FP64 units.
+    const unsigned at = (threadIdx.x / 32 * TOP_BLOCKS + blockIdx.x) * (32 / WIDE) + (threadIdx.x % 32) / WIDE;
+    const unsigned warp0 = at - (threadIdx.x % 32) / WIDE;
+    const unsigned end = dep_begin(ix, depth + 2);
+    unsigned lo = dep_begin(ix, depth), hi = dep_begin(ix, depth + 1);
+    CombineNode n = combine_fetch(dep_nodes, lo + at, hi, T, nd_geo, mo, err);
     for (; depth >= 0; --depth) {
-        combine_depth<true>(dep_nodes, ix, depth, counts[2], nd_geo, mo, inv_theta, inv_theta_sys, sys,
-                            (blockIdx.x * blockDim.x + threadIdx.x) >> 5, TOP_BLOCKS * COMBINE_BS / 32, err);
-        __threadfence();
+        for (unsigned k = lo; k + warp0 < hi; k += TOP_NODES) {  // warp-uniform
+            if (k != lo) n = combine_fetch(dep_nodes, k + at, hi, T, nd_geo, mo, err);
+            combine_node<true>(n, rows[sub], mo);
+        }
+        if (depth > 0) {
+            hi = lo;
+            lo = dep_begin(ix, depth - 1);
+            n = combine_fetch(dep_nodes, lo + at, hi, T, nd_geo, mo, err);
+        }
         __syncwarp();
+        // Releases this thread's writes to the cluster and acquires the others'.
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
+    rcrit_range(dep_nodes, dep_begin(ix, 0), end, T, nd_geo, mo, inv_theta, inv_theta_sys, sys,
+                blockIdx.x * TOP_BS + threadIdx.x, TOP_BLOCKS * TOP_BS);
 }
 
 #undef DADD
 #undef DMUL
 #undef DSUB
+#undef DFMA
 
 
 __global__ void k_probe() {}
@@ -2053,7 +2200,9 @@ void tree_build(Engine& e, double theta) {
     // most TOP_NODES nodes (by the eight-way branching, or because the whole tree is small) together.
     const float inv_theta = theta > 0 ? static_cast<float>(1.0 / theta) : FLT_MAX;
     Moments mo{t.nd_test.as<NodeTest>(), t.nd_cell.as<NodeCell>()};
-    launch_pdl(overlap(n), k_leaf_moments, grid_for(static_cast<long long>(K), 128), 128, s,
+    const bool wide = K <= LEAFW_MAX;
+    launch_pdl(overlap(n), wide ? k_leaf_moments_wide : k_leaf_moments,
+               grid_for(static_cast<long long>(K), wide ? LEAFW_BS / WIDE : 128), wide ? LEAFW_BS : 128, s,
                t.leaf_order.as<uint32_t>(), counts, t.nd_geo.as<float4>(), e.bodies(e.cur), mo, inv_theta,
                t.inv_theta_sys, sys, e.err_word());
     ++e.launches;
@@ -2061,7 +2210,7 @@ void tree_build(Engine& e, double theta) {
     if (T <= 8 * TOP_NODES) top = depth - 1;
     else
         for (size_t width = x.nroots; width <= TOP_NODES && top < depth - 1; width *= 8) ++top;
-    const int cb = std::max(1, std::min(2 * e.sms, grid_for(static_cast<long long>(T), COMBINE_NODES)));
+    const int cb = std::max(1, std::min(4 * e.sms, grid_for(static_cast<long long>(T), COMBINE_NODES)));
     for (int d = depth - 1; d > top; --d) {
         launch_pdl(overlap(n), k_combine_level, cb, COMBINE_BS, s, t.dep_nodes.as<uint32_t>(), ix, d,
                    counts, t.nd_geo.as<float4>(), mo, inv_theta, t.inv_theta_sys, sys, e.err_word());
@@ -2076,7 +2225,7 @@ void tree_build(Engine& e, double theta) {
         at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.gridDim = dim3(TOP_BLOCKS);
-        cfg.blockDim = dim3(COMBINE_BS);
+        cfg.blockDim = dim3(TOP_BS);
         cfg.stream = s;
         cfg.attrs = at;
         cfg.numAttrs = overlap(n) ? 2 : 1;

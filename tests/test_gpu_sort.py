@@ -89,3 +89,16 @@ def test_deeper_later(be):
         other.compute_forces(p, False)
         assert np.array_equal(other.tree_keys(), keys) and np.array_equal(other.download().id, ids)
         assert np.array_equal(other.accel(), a)
+
+
+# The moments on both sides of the leaf counts and depth widths at which they are formed by more lanes
+# or in other launches (about 6 bodies a leaf: 4096 leaves, 512 and 4096 nodes), the second call with
+# the sizes of the first; a corner of the cube holds no mass (the centre is the cell's).
+@pytest.mark.parametrize("n", [3000, 12000, 20000, 25000, 27000, 31000, 60000])
+def test_moment_widths(be, n):
+    b = zero_v(S.cube(n, n))
+    b.m[(b.x < 0) & (b.y < 0) & (b.z < 0)] = 0.0
+    be.upload(b)
+    for _ in range(2):
+        be.compute_forces(params(1, 0.01), False)
+        same_as_oracle(be, b)
