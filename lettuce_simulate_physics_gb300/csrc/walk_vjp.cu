@@ -19,7 +19,7 @@
 //   and dx_i -= gd, dX_entry += gd (X = x_j or the cell's centre of mass).
 // The self pair (j == i) is skipped: d is identically zero, so it has no derivative.
 // The cell adjoints (dM, dcom, dQ) then reach the bodies through the moment definitions
-// (k_moment_chain): for every ancestor cell c of body b, with e = x_b - com_c,
+// (k_leaf_field, k_body_field): for every ancestor cell c of body b, with e = x_b - com_c,
 //   dx_b += (m_b/M) dcom + m_b [6 dQ_diag e - 2 tr(dQ) e + 3 offdiag terms]
 //   dm_b += dM + e . dcom / M + sum_kl dQ_kl (3 e_k e_l - |e|^2 delta_kl)  (stored components)
 // (the derivative of Q through com vanishes because sum_b m_b e_b = 0).
@@ -328,47 +328,87 @@ __global__ void __launch_bounds__(WBS, VMINB) k_walk_vjp(VjpArgs a) {
     else vjp_evaluate<EPS0>(a, s);
 }
 
-// Cell adjoints to bodies through the moment definitions (every ancestor of the body's leaf).
-__global__ void k_moment_chain(TreeView tv, const BodyArrays b, int n, const double* __restrict__ nadj, double* gx,
-                               double* gy, double* gz, double* gm, unsigned* err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const size_t T = tv.T;
-    const uint32_t leaf = tv.body_leaf[i];
-    if (leaf >= min(static_cast<size_t>(*tv.nleaves), tv.K)) {
+// Cell adjoints to bodies through the moment definitions. What a cell gives a body at x is, for dm,
+//   dM + p.e + 1/2 e.H e,  and for dx m times its gradient p + H e,
+// with e = x - com, p = dcom / M, H_kk = 6 dQ_kk - 2 tr dQ, H_kl = 3 dQ_kl: a quadratic, and so is the
+// sum over a leaf's ancestors. A thread per leaf sums it about the leaf's centre of mass, and the
+// bodies evaluate their leaf's (FP64 both; the chain from every body cost 355 us a pass for the
+// 200 000-body collision, the two kernels 60 and 20).
+constexpr int NFIELD = 10;  // per leaf: the value, the gradient (3), H (xx, xy, xz, yy, yz, zz)
+
+__device__ __forceinline__ void cell_centre(const NodeCell& c, double& x, double& y, double& z) {
+    x = static_cast<double>(c.com.x) + c.lo.x;
+    y = static_cast<double>(c.com.y) + c.lo.y;
+    z = static_cast<double>(c.com.z) + c.lo.z;
+}
+
+__global__ void k_leaf_field(TreeView tv, const double* __restrict__ nadj, double* __restrict__ field, unsigned* err) {
+    const size_t l = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x, T = tv.T, K = tv.K;
+    if (l >= min(static_cast<size_t>(*tv.nleaves), K)) return;
+    uint32_t node = tv.leaf_node[l];
+    if (node >= T) {
         atomicOr(err, kErrNodeOverflow);
         return;
     }
-    uint32_t node = tv.leaf_node[leaf];
-    const double xb = b.x[i], yb = b.y[i], zb = b.z[i], mb = b.m[i];
-    double ax = 0, ay = 0, az = 0, am = 0;
+    double x0, y0, z0;
+    cell_centre(tv.nd_cell[node], x0, y0, z0);
+    double A = 0, Bx = 0, By = 0, Bz = 0, Hxx = 0, Hxy = 0, Hxz = 0, Hyy = 0, Hyz = 0, Hzz = 0;
     for (int guard = 0; node < T && guard < 128; ++guard) {
-        const double dM = nadj[node], dcx = nadj[T + node], dcy = nadj[2 * T + node], dcz = nadj[3 * T + node];
-        const double qxx = nadj[4 * T + node], qxy = nadj[5 * T + node], qxz = nadj[6 * T + node];
-        const double qyy = nadj[7 * T + node], qyz = nadj[8 * T + node], qzz = nadj[9 * T + node];
-        const float4 c = tv.nd_cell[node].com, cl = tv.nd_cell[node].lo;
-        const double M = c.w;
-        const double ex = xb - (static_cast<double>(c.x) + cl.x);
-        const double ey = yb - (static_cast<double>(c.y) + cl.y);
-        const double ez = zb - (static_cast<double>(c.z) + cl.z);
-        if (M > 0) {
-            ax += mb / M * dcx;
-            ay += mb / M * dcy;
-            az += mb / M * dcz;
-            am += (ex * dcx + ey * dcy + ez * dcz) / M;
-        }
-        const double tr = qxx + qyy + qzz, e2 = ex * ex + ey * ey + ez * ez;
-        ax += mb * (6 * qxx * ex - 2 * tr * ex + 3 * qxy * ey + 3 * qxz * ez);
-        ay += mb * (6 * qyy * ey - 2 * tr * ey + 3 * qxy * ex + 3 * qyz * ez);
-        az += mb * (6 * qzz * ez - 2 * tr * ez + 3 * qxz * ex + 3 * qyz * ey);
-        am += dM + qxx * (3 * ex * ex - e2) + qyy * (3 * ey * ey - e2) + qzz * (3 * ez * ez - e2) +
-              3 * (qxy * ex * ey + qxz * ex * ez + qyz * ey * ez);
+        const double qxx = nadj[4 * T + node], qyy = nadj[7 * T + node], qzz = nadj[9 * T + node];
+        const double hxy = 3 * nadj[5 * T + node], hxz = 3 * nadj[6 * T + node], hyz = 3 * nadj[8 * T + node];
+        const double t2 = 2 * (qxx + qyy + qzz), hxx = 6 * qxx - t2, hyy = 6 * qyy - t2, hzz = 6 * qzz - t2;
+        const NodeCell c = tv.nd_cell[node];
+        double ex, ey, ez;
+        cell_centre(c, ex, ey, ez);
+        ex = x0 - ex;
+        ey = y0 - ey;
+        ez = z0 - ez;
+        const double iM = c.com.w > 0 ? 1.0 / c.com.w : 0.0;
+        const double px = nadj[T + node] * iM, py = nadj[2 * T + node] * iM, pz = nadj[3 * T + node] * iM;
+        const double vx = hxx * ex + hxy * ey + hxz * ez, vy = hxy * ex + hyy * ey + hyz * ez,
+                     vz = hxz * ex + hyz * ey + hzz * ez;
+        A += nadj[node] + (px * ex + py * ey + pz * ez) + 0.5 * (vx * ex + vy * ey + vz * ez);
+        Bx += px + vx;
+        By += py + vy;
+        Bz += pz + vz;
+        Hxx += hxx;
+        Hxy += hxy;
+        Hxz += hxz;
+        Hyy += hyy;
+        Hyz += hyz;
+        Hzz += hzz;
         node = tv.nd_parent[node];
     }
-    gx[i] += ax;
-    gy[i] += ay;
-    gz[i] += az;
-    gm[i] += am;
+    const double f[NFIELD] = {A, Bx, By, Bz, Hxx, Hxy, Hxz, Hyy, Hyz, Hzz};
+#pragma unroll
+    for (int k = 0; k < NFIELD; ++k) field[k * K + l] = f[k];
+}
+
+__global__ void k_body_field(TreeView tv, const BodyArrays b, int n, const double* __restrict__ field, double* gx,
+                             double* gy, double* gz, double* gm, unsigned* err) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const size_t K = tv.K;
+    const uint32_t l = tv.body_leaf[i];
+    if (l >= min(static_cast<size_t>(*tv.nleaves), K) || tv.leaf_node[l] >= tv.T) {
+        atomicOr(err, kErrNodeOverflow);
+        return;
+    }
+    double ex, ey, ez;
+    cell_centre(tv.nd_cell[tv.leaf_node[l]], ex, ey, ez);
+    ex = b.x[i] - ex;
+    ey = b.y[i] - ey;
+    ez = b.z[i] - ez;
+    double f[NFIELD];
+#pragma unroll
+    for (int k = 0; k < NFIELD; ++k) f[k] = field[k * K + l];
+    const double vx = f[4] * ex + f[5] * ey + f[6] * ez, vy = f[5] * ex + f[7] * ey + f[8] * ez,
+                 vz = f[6] * ex + f[8] * ey + f[9] * ez;
+    const double m = b.m[i];
+    gx[i] += m * (f[1] + vx);
+    gy[i] += m * (f[2] + vy);
+    gz[i] += m * (f[3] + vz);
+    gm[i] += f[0] + (f[1] * ex + f[2] * ey + f[3] * ez) + 0.5 * (vx * ex + vy * ey + vz * ez);
 }
 
 template <bool EPS0>
@@ -396,7 +436,7 @@ void tree_walk_vjp(Engine& e, const float4* w, float e2, bool eps0, double* g) {
     if (n == 0) return;
     TreeView tv = tree_view(e);
     const size_t T = tv.T;
-    e.vjp_scratch.reserve(T * NADJ * 8);
+    e.vjp_scratch.reserve((T * NADJ + tv.K * NFIELD) * 8);
     double* nadj = e.vjp_scratch.as<double>();
     LG_CK(cudaMemsetAsync(nadj, 0, T * NADJ * 8, e.stream));
     LG_CK(cudaMemsetAsync(e.small.as<char>() + 40, 0, 4, e.stream));
@@ -417,9 +457,12 @@ void tree_walk_vjp(Engine& e, const float4* w, float e2, bool eps0, double* g) {
     a.e2 = e2;
     if (eps0) launch_vjp<true>(e, a);
     else launch_vjp<false>(e, a);
-    k_moment_chain<<<(n + 255) / 256, 256, 0, e.stream>>>(tv, b, n, nadj, a.gx, a.gy, a.gz, a.gm, e.err_word());
+    double* field = nadj + T * NADJ;
+    k_leaf_field<<<static_cast<int>((tv.K + 63) / 64), 64, 0, e.stream>>>(tv, nadj, field, e.err_word());
     LG_LAUNCHED();
-    ++e.launches;
+    k_body_field<<<(n + 255) / 256, 256, 0, e.stream>>>(tv, b, n, field, a.gx, a.gy, a.gz, a.gm, e.err_word());
+    LG_LAUNCHED();
+    e.launches += 2;
 }
 
 }  // namespace lg
