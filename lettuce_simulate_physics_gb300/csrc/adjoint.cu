@@ -215,12 +215,18 @@ __global__ void k_vjp_apply(const float4* __restrict__ partial, int n, int slice
 //   S1 += w_k / s^3,  S2 += m_k / s^3,  S3 -= cc d,  h -= (w_k . d) / s^3,
 // which is 34 FP32 operations for two ordered pairs instead of 52. Work units are pairs of
 // STILE-body tiles (I, J), J >= I; a block takes a strip of SSTRIP J tiles (or fewer) for one I tile,
-// its threads holding SIPT i-bodies each. The i side sums in registers over the strip. The j side
-// of each pair of j-bodies is summed over a warp's lanes by a transposed butterfly (16 values over
-// 32 lanes: each exchange sends half of what a lane holds), over the block's warps in shared
-// memory (warp order), and stored per unit. A diagonal unit (J == I) masks the pairs j <= k. All
-// sums run in a fixed order, so results do not depend on scheduling; k_vjp_sym_apply adds the
-// strips' and units' partial sums per body in FP64.
+// its threads holding SIPT i-bodies each. The i side sums in registers over the strip. The j side of
+// a warp: its lanes hold different pairs of j-bodies, 32 pairs at a time, and the pairs' sums move on
+// by one lane after each step, so that after 32 steps every pair has met every lane's i-bodies. Only
+// what the body's gradient needs travels, four sums per body: with m_j and w_j at hand the lane adds
+//   o = m_j S1 - w_j S2 - 3 S3  (its i-bodies' share of S1, S2, S3)  and h.
+// The block's warps are added in shared memory (warp order), and stored per unit. A diagonal unit
+// (J == I) masks the pairs j <= k. All sums run in a fixed order, so results do not depend on
+// scheduling; k_vjp_sym_apply adds the strips' and units' partial sums per body in FP64.
+// Bound by the FMA pipe: 146 packed instructions per step of a warp. With all lanes on one pair of
+// j-bodies and a butterfly of 16 values after it (62 instructions) 65 536 bodies took 2.99 ms and the
+// partial sums, twice as many, 0.27 ms; now 2.55 and 0.11 (two resident blocks instead of three: 2.52, two
+// i-bodies per thread: 3.0).
 #ifndef LG_VJPS_BS
 #define LG_VJPS_BS 128
 #endif
@@ -242,25 +248,12 @@ constexpr int STILE = SBS * SIPT;      // bodies per tile
 constexpr int SSUB = LG_VJPS_SUB;      // j-bodies between cross-warp reductions
 constexpr int SSTRIP = LG_VJPS_STRIP;  // J tiles per block
 constexpr int SWARPS = SBS / 32;
-static_assert(STILE % SSUB == 0 && SSUB % 2 == 0, "sub-tiles hold whole j pairs");
+static_assert(STILE % SSUB == 0 && SSUB % 64 == 0, "sub-tiles hold whole turns of 32 j pairs");
 
 struct __align__(16) SymSmem {
     float jx[STILE], jy[STILE], jz[STILE], jnm[STILE], jwx[STILE], jwy[STILE], jwz[STILE];
-    float red[SWARPS][SSUB][8];
+    float4 red[SWARPS][SSUB];
 };
-
-// One exchange of the transposed butterfly: lanes with bit O keep the upper H of their 2H values
-// and send the lower H, the others the reverse; each kept value adds the partner's sent one.
-template <int O, int H>
-__device__ __forceinline__ void tr_level(float (&v)[16], int lane) {
-    const bool up = (lane & O) != 0;
-#pragma unroll
-    for (int t = 0; t < H; ++t) {
-        const float send = up ? v[t] : v[t + H];
-        const float keep = up ? v[t + H] : v[t];
-        v[t] = keep + __shfl_xor_sync(0xffffffffu, send, O);
-    }
-}
 
 constexpr float kFarV = 1e18f;  // a far, massless, zero-weight body: adds nothing to either side
 
@@ -271,13 +264,12 @@ __device__ __forceinline__ size_t jrow(int I, int npad) {
 
 // units[b] = (I, J0, J1, strip): block b evaluates tile I against tiles [J0, J1) and writes its i
 // sums to row `strip` of ipart (the tile's STILE bodies); the j sums of unit (I, J) go to row I of
-// jpart. Entries are 8 floats: S1 (3), -S2, S3 (3), h, where jpart holds the j side's -S2, S3 and
-// h with the opposite sign.
+// jpart. Entries are o and h of the body, both with the opposite sign.
 template <bool EPS0>
 __global__ void __launch_bounds__(SBS, LG_VJPS_MINB) k_vjp_sym(const float4* __restrict__ hm, const float4* __restrict__ lo,
                                                    const float4* __restrict__ wv, int n, int npad, float e2,
-                                                   const int4* __restrict__ units, float* __restrict__ ipart,
-                                                   float* __restrict__ jpart) {
+                                                   const int4* __restrict__ units, float4* __restrict__ ipart,
+                                                   float4* __restrict__ jpart) {
     __shared__ SymSmem sm;
     const int4 un = units[blockIdx.x];
     const int I = un.x, J0 = un.y, J1 = un.z, strip = un.w;
@@ -308,8 +300,7 @@ __global__ void __launch_bounds__(SBS, LG_VJPS_MINB) k_vjp_sym(const float4* __r
         for (int q = 0; q < 8; ++q) a[u][q] = 0ull;
     }
     const f2x E2 = f2_bcast(e2);
-    // The (j, component) a lane holds after the butterfly: lane bits 4..1 select halves in turn.
-    const int qsel = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+    const f2x CN3 = f2_bcast(-3.f);
     for (int J = J0; J < J1; ++J) {
         const int jb = J * STILE;
         __syncthreads();  // the previous tile's readers are done
@@ -333,7 +324,11 @@ __global__ void __launch_bounds__(SBS, LG_VJPS_MINB) k_vjp_sym(const float4* __r
         auto tile = [&](auto diag_tag) {
         constexpr bool DIAG = decltype(diag_tag)::value;
         for (int s0 = 0; s0 < STILE; s0 += SSUB) {
-            for (int jp = s0; jp < s0 + SSUB; jp += 2) {
+          for (int c0 = s0; c0 < s0 + SSUB; c0 += 64) {
+            f2x ox = 0ull, oy = 0ull, oz = 0ull, oh = 0ull;  // the pair's sums, of opposite sign
+#pragma unroll 1
+            for (int st = 0; st < 32; ++st) {
+                const int jp = c0 + 2 * ((lane + st) & 31);
                 const f2x X = ld2(sm.jx + jp), Y = ld2(sm.jy + jp), Z = ld2(sm.jz + jp), NM = ld2(sm.jnm + jp);
                 const f2x WX = ld2(sm.jwx + jp), WY = ld2(sm.jwy + jp), WZ = ld2(sm.jwz + jp);
                 f2x b[8];
@@ -377,26 +372,32 @@ __global__ void __launch_bounds__(SBS, LG_VJPS_MINB) k_vjp_sym(const float4* __r
                     b[6] = f2_fma(cc, dz, b[6]);
                     b[7] = f2_fma(dwk, inv3, b[7]);
                 }
-                // v[2c + h] = component c of j-body jp + h, summed over the lane's i-bodies.
-                float v[16];
-#pragma unroll
-                for (int c = 0; c < 8; ++c) f2_unpack(b[c], v[2 * c], v[2 * c + 1]);
-                tr_level<16, 8>(v, lane);
-                tr_level<8, 4>(v, lane);
-                tr_level<4, 2>(v, lane);
-                tr_level<2, 1>(v, lane);
-                v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-                if (!(lane & 1)) sm.red[warp][jp - s0 + (qsel & 1)][qsel >> 1] = v[0];
+                // Every sum goes to the lane that meets the pair next: after 32 steps to lane l pair l.
+                const int from = (lane + 1) & 31;
+                ox = __shfl_sync(0xffffffffu, f2_fma(NM, b[0], f2_fma(WX, b[3], f2_fma(CN3, b[4], ox))), from);
+                oy = __shfl_sync(0xffffffffu, f2_fma(NM, b[1], f2_fma(WY, b[3], f2_fma(CN3, b[5], oy))), from);
+                oz = __shfl_sync(0xffffffffu, f2_fma(NM, b[2], f2_fma(WZ, b[3], f2_fma(CN3, b[6], oz))), from);
+                oh = __shfl_sync(0xffffffffu, f2_add(oh, b[7]), from);
             }
+            float4 r0, r1;
+            f2_unpack(ox, r0.x, r1.x);
+            f2_unpack(oy, r0.y, r1.y);
+            f2_unpack(oz, r0.z, r1.z);
+            f2_unpack(oh, r0.w, r1.w);
+            sm.red[warp][c0 - s0 + 2 * lane] = r0;
+            sm.red[warp][c0 - s0 + 2 * lane + 1] = r1;
+          }
             __syncthreads();
             // The sub-tile's j sums over the block's warps, in warp order.
-            for (int t = tid; t < SSUB * 8; t += SBS) {
-                const int jj = t >> 3, c = t & 7;
-                float sum = sm.red[0][jj][c];
+            for (int jj = tid; jj < SSUB; jj += SBS) {
+                float4 sum = sm.red[0][jj];
 #pragma unroll
-                for (int w = 1; w < SWARPS; ++w) sum += sm.red[w][jj][c];
+                for (int w = 1; w < SWARPS; ++w) {
+                    const float4 r = sm.red[w][jj];
+                    sum = make_float4(sum.x + r.x, sum.y + r.y, sum.z + r.z, sum.w + r.w);
+                }
                 const int j = jb + s0 + jj;
-                if (j < n) jpart[(jrow(I, npad) + (j - ib)) * 8 + c] = sum;
+                if (j < n) jpart[jrow(I, npad) + (j - ib)] = sum;
             }
             __syncthreads();  // red is rewritten by the next sub-tile
         }
@@ -407,43 +408,56 @@ __global__ void __launch_bounds__(SBS, LG_VJPS_MINB) k_vjp_sym(const float4* __r
 #pragma unroll
     for (int u = 0; u < SIPT; ++u) {
         if (iidx[u] >= n) continue;
-        float* o = ipart + (static_cast<size_t>(strip) * STILE + (iidx[u] - ib)) * 8;
-        const float4 p0 = make_float4(f2_sum(a[u][0]), f2_sum(a[u][1]), f2_sum(a[u][2]), f2_sum(a[u][3]));
-        const float4 p1 = make_float4(f2_sum(a[u][4]), f2_sum(a[u][5]), f2_sum(a[u][6]), f2_sum(a[u][7]));
-        reinterpret_cast<float4*>(o)[0] = p0;
-        reinterpret_cast<float4*>(o)[1] = p1;
+        // -(m S1 - w S2 - 3 S3), -h; a[u][3] holds -S2
+        const float m = hm[iidx[u]].w, s2 = f2_sum(a[u][3]);
+        const float4 w = wv[iidx[u]];
+        ipart[static_cast<size_t>(strip) * STILE + (iidx[u] - ib)] =
+            make_float4(fmaf(-m, f2_sum(a[u][0]), fmaf(-w.x, s2, 3.f * f2_sum(a[u][4]))),
+                        fmaf(-m, f2_sum(a[u][1]), fmaf(-w.y, s2, 3.f * f2_sum(a[u][5]))),
+                        fmaf(-m, f2_sum(a[u][2]), fmaf(-w.z, s2, 3.f * f2_sum(a[u][6]))), -f2_sum(a[u][7]));
     }
 }
 
-// Per body k of tile K: the i sums of K's strips and the j sums of units (I, K), I <= K, in that
-// order in FP64; then lx += G (m_k S1 - w_k S2 - 3 S3), lm -= G h.
-__global__ void k_vjp_sym_apply(const float* __restrict__ ipart, const float* __restrict__ jpart,
-                                const int* __restrict__ strip_base, const float4* __restrict__ hm,
-                                const float4* __restrict__ wv, int n, int npad, double G, double* lx, double* ly,
-                                double* lz, double* lm) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const int K = k / STILE;
-    double S[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int st = strip_base[K]; st < strip_base[K + 1]; ++st) {
-        const float4* p = reinterpret_cast<const float4*>(ipart + (static_cast<size_t>(st) * STILE + (k - K * STILE)) * 8);
-        const float4 p0 = p[0], p1 = p[1];
-        S[0] += p0.x; S[1] += p0.y; S[2] += p0.z; S[3] += p0.w;
-        S[4] += p1.x; S[5] += p1.y; S[6] += p1.z; S[7] += p1.w;
+// Per body k of tile K: the i sums of K's strips and the j sums of units (I, K), I <= K, in FP64; then
+// lx += G o, lm -= G h. APARTS threads per body take every APARTS-th row (a thread per body had up to
+// 192 dependent reads), and their sums are added in order.
+constexpr int ABODIES = 32, APARTS = 8;  // 65 536 bodies: 0.27 -> 0.11 ms, FP64 additions
+__global__ void __launch_bounds__(ABODIES * APARTS) k_vjp_sym_apply(const float4* __restrict__ ipart,
+                                                                    const float4* __restrict__ jpart,
+                                                                    const int* __restrict__ strip_base, int n,
+                                                                    int npad, double G, double* lx, double* ly,
+                                                                    double* lz, double* lm) {
+    __shared__ double sums[APARTS][4][ABODIES];
+    const int lane = threadIdx.x % ABODIES, part = threadIdx.x / ABODIES;
+    const int k = blockIdx.x * ABODIES + lane;
+    double S[4] = {0, 0, 0, 0};
+    if (k < n) {
+        const int K = k / STILE;
+        auto add = [&](const float4 p) {
+            S[0] += p.x;
+            S[1] += p.y;
+            S[2] += p.z;
+            S[3] += p.w;
+        };
+        const int st1 = strip_base[K + 1];
+#pragma unroll 4
+        for (int st = strip_base[K] + part; st < st1; st += APARTS)
+            add(ipart[static_cast<size_t>(st) * STILE + (k - K * STILE)]);
+#pragma unroll 4
+        for (int I = part; I <= K; I += APARTS) add(jpart[jrow(I, npad) + (k - I * STILE)]);
     }
-    for (int I = 0; I <= K; ++I) {
-        const float4* p = reinterpret_cast<const float4*>(jpart + (jrow(I, npad) + (k - I * STILE)) * 8);
-        const float4 p0 = p[0], p1 = p[1];
-        S[0] += p0.x; S[1] += p0.y; S[2] += p0.z; S[3] -= p0.w;
-        S[4] -= p1.x; S[5] -= p1.y; S[6] -= p1.z; S[7] -= p1.w;
-    }
-    const double m = hm[k].w;
-    const float4 w = wv[k];
-    // m_k S1 - w_k S2 - 3 S3 (S[3] holds -S2)
-    lx[k] += G * (m * S[0] + w.x * S[3] - 3.0 * S[4]);
-    ly[k] += G * (m * S[1] + w.y * S[3] - 3.0 * S[5]);
-    lz[k] += G * (m * S[2] + w.z * S[3] - 3.0 * S[6]);
-    lm[k] -= G * S[7];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) sums[part][c][lane] = S[c];
+    __syncthreads();
+    if (part != 0 || k >= n) return;
+#pragma unroll
+    for (int p = 1; p < APARTS; ++p)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) S[c] += sums[p][c][lane];
+    lx[k] -= G * S[0];
+    ly[k] -= G * S[1];
+    lz[k] -= G * S[2];
+    lm[k] += G * S[3];
 }
 
 // lv += dt lx; w = c lv (FP32 for the VJP), with the body's mass alongside.
@@ -789,14 +803,14 @@ double adjoint_backward(Engine& e, AdjointState& a, const double* tx, const doub
     slices = (n + jslice - 1) / jslice;
     // Symmetric VJP (each unordered pair once) when there are enough tile units to fill the GPU
     // (at least four per SM: about 26k bodies and up; below that the one-sided kernel's split-j
-    // grid fills it better) and its partial sums stay within 4 GB (about 250k bodies).
+    // grid fills it better) and its partial sums stay within 2 GB (about 250k bodies).
     // LETTUCE_GB300_VJP=pairs or =symmetric overrides the size rule (not the memory bound).
     const int T = (n + STILE - 1) / STILE;
     const int npad = T * STILE;
-    const size_t jbytes = static_cast<size_t>(STILE) * T * (T + 1) / 2 * 32;
+    const size_t jbytes = static_cast<size_t>(STILE) * T * (T + 1) / 2 * 16;
     long long units_needed = 0;  // one block per strip of up to SSTRIP tiles: sum over I of ceil((T - I) / SSTRIP)
     for (int I = 0; I < T; ++I) units_needed += (T - I + SSTRIP - 1) / SSTRIP;
-    const bool fits = jbytes + static_cast<size_t>(units_needed) * STILE * 32 <= (size_t(4) << 30);
+    const bool fits = jbytes + static_cast<size_t>(units_needed) * STILE * 16 <= (size_t(2) << 30);
     bool sym = !tree && fits && units_needed >= 4LL * e.sms;
     if (const char* v = std::getenv("LETTUCE_GB300_VJP")) {
         const std::string m = v;
@@ -823,7 +837,7 @@ double adjoint_backward(Engine& e, AdjointState& a, const double* tx, const doub
                               cudaMemcpyHostToDevice, s));
         LG_CK(cudaMemcpyAsync(a.sym_sbase.as<int>(), a.sym_sbase_h.data(), a.sym_sbase_h.size() * sizeof(int),
                               cudaMemcpyHostToDevice, s));
-        a.ipart.reserve(static_cast<size_t>(strip) * STILE * 32);
+        a.ipart.reserve(static_cast<size_t>(strip) * STILE * 16);
         a.jpart.reserve(jbytes);
     } else if (!tree) {
         a.partial.reserve(static_cast<size_t>(slices) * n * 16);
@@ -907,16 +921,16 @@ double adjoint_backward(Engine& e, AdjointState& a, const double* tx, const doub
                 if (sym) {
                     if (eps0)
                         k_vjp_sym<true><<<nunits, SBS, 0, vs>>>(hm, lo, a.w.as<float4>(), n, npad, e2,
-                                                                a.sym_units.as<int4>(), a.ipart.as<float>(),
-                                                                a.jpart.as<float>());
+                                                                a.sym_units.as<int4>(), a.ipart.as<float4>(),
+                                                                a.jpart.as<float4>());
                     else
                         k_vjp_sym<false><<<nunits, SBS, 0, vs>>>(hm, lo, a.w.as<float4>(), n, npad, e2,
-                                                                 a.sym_units.as<int4>(), a.ipart.as<float>(),
-                                                                 a.jpart.as<float>());
+                                                                 a.sym_units.as<int4>(), a.ipart.as<float4>(),
+                                                                 a.jpart.as<float4>());
                     LG_LAUNCHED();
-                    k_vjp_sym_apply<<<gb, 256, 0, vs>>>(a.ipart.as<float>(), a.jpart.as<float>(), a.sym_sbase.as<int>(),
-                                                        hm, a.w.as<float4>(), n, npad, a.p.G, a.lx.as<double>(),
-                                                        a.ly.as<double>(), a.lz.as<double>(), a.lm.as<double>());
+                    k_vjp_sym_apply<<<grid_for(n, ABODIES), ABODIES * APARTS, 0, vs>>>(
+                        a.ipart.as<float4>(), a.jpart.as<float4>(), a.sym_sbase.as<int>(), n, npad, a.p.G,
+                        a.lx.as<double>(), a.ly.as<double>(), a.lz.as<double>(), a.lm.as<double>());
                     LG_LAUNCHED();
                     e.launches += 3;
                     continue;
