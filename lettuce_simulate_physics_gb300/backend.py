@@ -547,7 +547,7 @@ class CudaBackend:
         ptr = [out[k].ctypes.data_as(_d) for k in range(7)]
         _check(self._lib.lg_adjoint_backward(self._h, t[0].ctypes.data_as(_d), t[1].ctypes.data_as(_d),
                                              t[2].ctypes.data_as(_d), C.byref(loss), *ptr))
-        return float(loss.value), out[0:3].T.copy(), out[3:6].T.copy(), out[6].copy()
+        return float(loss.value), _rows(out[0:3]), _rows(out[3:6]), out[6].copy()
 
     def adjoint_backward_seeded(self, dldx):
         """Gradients for a caller's loss of the final positions: dldx (n, 3) = dL/dx(T) by body id.
@@ -558,12 +558,20 @@ class CudaBackend:
         ptr = [out[k].ctypes.data_as(_d) for k in range(7)]
         _check(self._lib.lg_adjoint_backward_seeded(self._h, t[0].ctypes.data_as(_d), t[1].ctypes.data_as(_d),
                                                     t[2].ctypes.data_as(_d), *ptr))
-        return out[0:3].T.copy(), out[3:6].T.copy(), out[6].copy()
+        return _rows(out[0:3]), _rows(out[3:6]), out[6].copy()
 
     def launch_count(self) -> int:
         c = C.c_uint64()
         _check(self._lib.lg_launch_count(self._h, C.byref(c)))
         return int(c.value)
+
+
+def _rows(columns: np.ndarray) -> np.ndarray:
+    """(3, n) columns as an (n, 3) array, a column at a time (columns.T.copy() runs along rows of three)."""
+    out = np.empty(columns.shape[::-1])
+    for k, c in enumerate(columns):
+        out[:, k] = c
+    return out
 
 
 class PinnedBodies:

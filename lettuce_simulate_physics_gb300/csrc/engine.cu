@@ -10,7 +10,11 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
+
+#include <unistd.h>
 
 #include "../../include/lettuce_gb300.h"
 #include "engine.cuh"
@@ -106,6 +110,52 @@ Engine::~Engine() {
     if (stream) cudaStreamDestroy(stream);
 }
 
+int adjacent_columns(void* const* dst, int c, int columns, size_t bytes) {
+    int k = 1;
+    while (c + k < columns && dst[c] && dst[c + k] == static_cast<char*>(dst[c]) + bytes * static_cast<size_t>(k)) ++k;
+    return k;
+}
+
+void map_host_pages(void* const* dst, int columns, size_t bytes) {
+    constexpr size_t kShare = size_t(4) << 20;  // per thread
+    const size_t page = static_cast<size_t>(sysconf(_SC_PAGESIZE));
+    std::vector<std::pair<char*, char*>> parts;
+    size_t total = 0;
+    for (int c = 0, k; c < columns && bytes; c += k) {
+        k = adjacent_columns(dst, c, columns, bytes);
+        char *p = static_cast<char*>(dst[c]), *end = p + bytes * static_cast<size_t>(k);
+        if (!p) continue;
+        // To ask whether it is page-locked takes 10 us, as long as to write to 2 MB of pages that are.
+        if (end - p > (2 << 20)) {
+            cudaPointerAttributes at{};
+            if (cudaPointerGetAttributes(&at, p) != cudaSuccess) cudaGetLastError();
+            else if (at.type != cudaMemoryTypeUnregistered) continue;
+        }
+        total += static_cast<size_t>(end - p);
+        for (char* q = p; q < end; q += kShare) parts.emplace_back(q, std::min(q + kShare, end));
+    }
+    // Written, not read first: a page read before it is written is mapped twice, and the second mapping
+    // takes the first back from the device as well (10 times the time).
+    auto map = [&](size_t first, size_t step) {
+        for (size_t k = first; k < parts.size(); k += step) {
+            for (volatile char* q = parts[k].first; q < parts[k].second; q += page) *q = 0;
+            parts[k].second[-1] = 0;
+        }
+    };
+    if (total < 2 * kShare) return map(0, 1);
+    const size_t threads = std::min<size_t>({8, total / kShare, std::max(1u, std::thread::hardware_concurrency())});
+    std::vector<std::thread> pool;
+    pool.reserve(threads);
+    size_t started = 1;
+    try {
+        for (; started < threads; ++started) pool.emplace_back(map, started, threads);
+    } catch (const std::system_error&) {  // no more threads to be had: this one does their parts
+    }
+    for (size_t k = started; k < threads; ++k) map(k, threads);
+    map(0, threads);
+    for (std::thread& t : pool) t.join();
+}
+
 BodyArrays Engine::bodies(int which) const {
     const BodySet& s = set[which];
     BodyArrays b;
@@ -124,7 +174,7 @@ void Engine::reserve_bodies(size_t count) {
         s.cost.reserve(count * 4); s.id.reserve(count * 4); s.level.reserve(count + 16);
     }
     acc.reserve(count * 16);
-    staging.reserve(count * 4 * 4);
+    staging.reserve(count * 16);
 }
 
 void Engine::upload(size_t count, const float* x, const float* y, const float* z, const float* vx, const float* vy,
@@ -183,17 +233,27 @@ void Engine::upload64(size_t count, const double* x, const double* y, const doub
     LG_CK(cudaStreamSynchronize(stream));
 }
 
+void Engine::read_columns(Columns set, const PlaceMap& map, void* const* dst, int columns, int mapped) {
+    float* st = staging.as<float>();
+    launch_columns(bodies(cur), acc.as<float4>(), set, map, st, n, stream);
+    ++launches;
+    const size_t fb = static_cast<size_t>(n) * 4;
+    map_host_pages(dst, std::max(columns, mapped), fb);
+    for (int c = 0, k; c < columns; c += k) {
+        k = adjacent_columns(dst, c, columns, fb);
+        if (dst[c])
+            LG_CK(cudaMemcpyAsync(dst[c], st + static_cast<size_t>(n) * static_cast<size_t>(c),
+                                  fb * static_cast<size_t>(k), cudaMemcpyDeviceToHost, stream));
+    }
+}
+
 void Engine::download(float* x, float* y, float* z, float* vx, float* vy, float* vz, float* m, uint32_t* id) {
     LG_CK(cudaSetDevice(dev));
     if (n == 0) return;
-    const size_t count = static_cast<size_t>(n), fb = count * 4;
-    BodyArrays b = bodies(cur);
-    float* st = staging.as<float>();
-    launch_round_pos(b, st, st + count, st + 2 * count, n, stream);
-    ++launches;
-    LG_CK(cudaMemcpyAsync(x, st, fb, cudaMemcpyDeviceToHost, stream));
-    LG_CK(cudaMemcpyAsync(y, st + count, fb, cudaMemcpyDeviceToHost, stream));
-    LG_CK(cudaMemcpyAsync(z, st + 2 * count, fb, cudaMemcpyDeviceToHost, stream));
+    void* const dst[8] = {x, y, z, vx, vy, vz, m, id};
+    const size_t fb = static_cast<size_t>(n) * 4;
+    const BodyArrays b = bodies(cur);
+    read_columns(Columns::kPos, PlaceMap{}, dst, 3, 8);
     LG_CK(cudaMemcpyAsync(vx, b.vx, fb, cudaMemcpyDeviceToHost, stream));
     LG_CK(cudaMemcpyAsync(vy, b.vy, fb, cudaMemcpyDeviceToHost, stream));
     LG_CK(cudaMemcpyAsync(vz, b.vz, fb, cudaMemcpyDeviceToHost, stream));
@@ -440,13 +500,9 @@ bool Engine::body_costs(float* cost, size_t count) {
 void Engine::read_accel(float* ax, float* ay, float* az, float* pot) {
     LG_CK(cudaSetDevice(dev));
     if (n == 0) return;
-    std::vector<float4> h(static_cast<size_t>(n));
-    LG_CK(cudaMemcpyAsync(h.data(), acc.as<float4>(), h.size() * 16, cudaMemcpyDeviceToHost, stream));
+    void* const dst[4] = {ax, ay, az, pot};
+    read_columns(Columns::kAcc, PlaceMap{}, dst, 4);
     LG_CK(cudaStreamSynchronize(stream));
-    for (size_t i = 0; i < h.size(); ++i) {
-        ax[i] = h[i].x; ay[i] = h[i].y; az[i] = h[i].z;
-        if (pot) pot[i] = h[i].w;
-    }
 }
 
 void Engine::read_pos64(double* x, double* y, double* z) {

@@ -76,6 +76,14 @@ struct BodySet {
     DevBuf x, y, z, hm, lo, vx, vy, vz, m, cost, id, level;
 };
 
+// Has the CPU give memory to those pages of host arrays (null ones are left out) that have none yet,
+// before a copy fills them: a caller's new arrays, whose pages the copy would fault in from the device
+// (83 MB took 70 ms that way; one thread maps them in 2.7 ms, several, where there are many, in 1, and
+// the copy then takes 0.6). `columns` arrays of `bytes` each; those that follow one another count as one.
+void map_host_pages(void* const* dst, int columns, size_t bytes);
+// Columns c .. of dst that follow column c in memory, itself included.
+int adjacent_columns(void* const* dst, int c, int columns, size_t bytes);
+
 struct Engine {
     explicit Engine(int device);
     ~Engine();
@@ -86,6 +94,10 @@ struct Engine {
     void upload64(size_t count, const double* x, const double* y, const double* z, const float* vx, const float* vy,
                   const float* vz, const float* m, const uint32_t* id);
     void download(float* x, float* y, float* z, float* vx, float* vy, float* vz, float* m, uint32_t* id);
+    // Lays `set` out in the staging buffer and copies its columns to dst (a null one is left out), as
+    // one copy where the host's arrays follow one another; their pages, and those of further columns up
+    // to `mapped`, are mapped first.
+    void read_columns(Columns set, const PlaceMap& map, void* const* dst, int columns, int mapped = 0);
     void build_tree(const lg_force_params& p);
     void compute_forces_with(const lg_force_params& p, bool potential, const lg_let_tree* remote, size_t nremote);
     void kick(double dt);

@@ -46,13 +46,42 @@ __global__ void k_refresh_hilo(BodyArrays b, int n) {
     store_hilo(b, i, b.x[i], b.y[i], b.z[i], b.m[i]);
 }
 
-__global__ void k_round_pos(const BodyArrays b, float* __restrict__ x, float* __restrict__ y, float* __restrict__ z,
-                            int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Columns of 4-byte values as the host takes them, column c at out + c n, body i at the place the map
+// gives it (an ensemble's systems in the caller's order) or at i.
+__global__ void k_columns(const BodyArrays b, const float4* __restrict__ acc, Columns set, PlaceMap map,
+                          float* __restrict__ out, size_t n) {
+    const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
     if (i >= n) return;
-    x[i] = __double2float_rn(b.x[i]);
-    y[i] = __double2float_rn(b.y[i]);
-    z[i] = __double2float_rn(b.z[i]);
+    size_t at = i;
+    if (map.nsys) {
+        int lo = 0, hi = map.nsys;  // the last system that begins at or before body i
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (map.off[mid] <= i) lo = mid;
+            else hi = mid;
+        }
+        at = map.dst[lo] + (i - map.off[lo]);
+    }
+    float* o = out + at;
+    if (set == Columns::kAcc) {
+        const float4 a = acc[i];
+        o[0] = a.x;
+        o[n] = a.y;
+        o[2 * n] = a.z;
+        o[3 * n] = a.w;
+        return;
+    }
+    if (set != Columns::kRest) {
+        o[0] = __double2float_rn(b.x[i]);
+        o[n] = __double2float_rn(b.y[i]);
+        o[2 * n] = __double2float_rn(b.z[i]);
+        if (set == Columns::kFirst) o[3 * n] = b.vx[i];
+        return;
+    }
+    o[0] = b.vy[i];
+    o[n] = b.vz[i];
+    o[2 * n] = b.m[i];
+    reinterpret_cast<uint32_t*>(o)[3 * n] = b.id[i];
 }
 
 // v += a dt in FP32 (src/cpu_backend.cpp:279-290).
@@ -374,9 +403,10 @@ void launch_refresh_hilo(BodyArrays b, int n, cudaStream_t s) {
     LG_LAUNCHED();
 }
 
-void launch_round_pos(const BodyArrays b, float* x, float* y, float* z, int n, cudaStream_t s) {
+void launch_columns(const BodyArrays b, const float4* acc, Columns set, const PlaceMap& map, float* out, int n,
+                    cudaStream_t s) {
     if (n <= 0) return;
-    k_round_pos<<<grid_for(n, BS), BS, 0, s>>>(b, x, y, z, n);
+    k_columns<<<grid_for(n, BS), BS, 0, s>>>(b, acc, set, map, out, static_cast<size_t>(n));
     LG_LAUNCHED();
 }
 

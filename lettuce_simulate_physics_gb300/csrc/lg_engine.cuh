@@ -44,7 +44,16 @@ void launch_widen(const float* x, const float* y, const float* z, const float* m
                   cudaStream_t s);
 // hm/lo from the FP64 positions and masses already stored in b.
 void launch_refresh_hilo(BodyArrays b, int n, cudaStream_t s);
-void launch_round_pos(const BodyArrays b, float* x, float* y, float* z, int n, cudaStream_t s);
+// Columns of one readback: x y z (rounded); x y z vx; vy vz m id; the accelerations and the potential.
+enum class Columns { kPos, kFirst, kRest, kAcc };
+// Body i of system s (bodies [off[s], off[s + 1])) goes to dst[s] + i - off[s]; nsys == 0: to i.
+struct PlaceMap {
+    const uint32_t* off = nullptr;
+    const uint32_t* dst = nullptr;
+    int nsys = 0;
+};
+void launch_columns(const BodyArrays b, const float4* acc, Columns set, const PlaceMap& map, float* out, int n,
+                    cudaStream_t s);
 void launch_kick(BodyArrays b, const float4* acc, float dt, int n, cudaStream_t s);
 void launch_drift(BodyArrays b, double dt, int n, cudaStream_t s);
 // Ensemble step opening (kick by hdt, then drift by dt; the same arithmetic as the two kernels).
