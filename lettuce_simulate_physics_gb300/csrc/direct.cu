@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(DBS, LG_DIRECT_MINB) k_direct(const float4* __
                                                 int jslice, float G, float e2, float4* __restrict__ out, int write_final,
                                                 unsigned* err, float* cost) {
     __shared__ DirectSmem<TL> sm;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the partials' sum may be scheduled
     const int j0 = blockIdx.y * jslice;
     direct_block<IPT, TL, POT, EPS0>(sm, hm, lo, blockIdx.x * (DBS * IPT), n, j0, min(n, j0 + jslice), G, e2,
                                  write_final ? out : out + static_cast<size_t>(blockIdx.y) * n, write_final != 0, err,
@@ -233,20 +234,35 @@ __global__ void __launch_bounds__(DBS, LG_DIRECT_MINB) k_direct_batch(const floa
     direct_block<IPT, TL, POT, EPS0>(sm, hm, lo, w.base, w.iend, w.j0, w.j1, G, w.e2, acc, true, err);
 }
 
-// Sums the split-j partials in slice order (Kahan) and scales by G.
-__global__ void k_direct_reduce(const float4* __restrict__ partial, int n, int slices, float G, float4* __restrict__ acc,
-                                float* __restrict__ cost) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (cost) cost[i] = static_cast<float>(n - 1);
+// Sums the split-j partials (Kahan) and scales by G: `parts` threads per body take every parts-th slice
+// in order, and their sums are added in order. One thread per body read up to 40 slices one after
+// another on a few SMs; see launch_direct for what it measured.
+constexpr int RBS = 256;
+__global__ void __launch_bounds__(RBS) k_direct_reduce(const float4* __restrict__ partial, int n, int slices, int parts,
+                                                       float G, float4* __restrict__ acc, float* __restrict__ cost) {
+    __shared__ float4 sums[RBS];
+    pdl_wait();
+    const int bodies = RBS / parts, part = threadIdx.x / bodies, lane = threadIdx.x - part * bodies;
+    const int i = blockIdx.x * bodies + lane;
     float s[4] = {0, 0, 0, 0}, c[4] = {0, 0, 0, 0};
-    for (int k = 0; k < slices; ++k) {
-        const float4 p = partial[static_cast<size_t>(k) * n + i];
+    auto add = [&](const float4 p) {
         kahan_add(s[0], c[0], p.x);
         kahan_add(s[1], c[1], p.y);
         kahan_add(s[2], c[2], p.z);
         kahan_add(s[3], c[3], p.w);
+    };
+    if (i < n) {
+#pragma unroll 4
+        for (int k = part; k < slices; k += parts) add(partial[static_cast<size_t>(k) * n + i]);
     }
+    if (parts > 1) {
+        sums[threadIdx.x] = make_float4(s[0] - c[0], s[1] - c[1], s[2] - c[2], s[3] - c[3]);
+        __syncthreads();
+        if (part) return;
+        for (int p = 1; p < parts; ++p) add(sums[p * bodies + lane]);
+    }
+    if (i >= n) return;
+    if (cost) cost[i] = static_cast<float>(n - 1);
     acc[i] = make_float4(G * (s[0] - c[0]), G * (s[1] - c[1]), G * (s[2] - c[2]), -G * (s[3] - c[3]));
 }
 
@@ -300,7 +316,9 @@ DirectShape default_direct_shape(int n, int sms) {
     sh.tile = TILE;
     const int iblocks = (n + DBS * sh.ipt - 1) / (DBS * sh.ipt);
     const int wave = blocks_per_sm(sh.ipt) * sms;
-    const int max_slices = std::max(1, n / 128);
+    // Slices of 128 j-bodies at least, 64 for the smallest sets, which fill few SMs (300 bodies 9.5 -> 7.7
+    // us, 1000 with the potential 11.8 -> 10.1; 2000 without 9.9 -> 11.2).
+    const int max_slices = std::max(1, n / (n <= 1024 ? 64 : 128));
     int best = 1;
     double best_eff = 0;
     for (int waves = 1; waves <= 8; ++waves) {
@@ -343,8 +361,13 @@ void launch_direct(const BodyArrays b, int n, float G, float e2, bool potential,
         }
     }
     if (!final_out) {
-        k_direct_reduce<<<(n + 255) / 256, 256, 0, s>>>(partial, n, slices, G, acc, cost);
-        LG_LAUNCHED();
+        // Two slices per thread or more, up to eight threads per body, and the launch overlaps the end of
+        // the pairs' kernel (both kernels: 1000 bodies 12.7 -> 10.6 us, 5001 27.0 -> 22.8, 16 384 106.7 ->
+        // 102.9).
+        int parts = 1;
+        while (parts < 8 && slices >= 4 * parts) parts *= 2;
+        launch_pdl(true, k_direct_reduce, (n + RBS / parts - 1) / (RBS / parts), RBS, s, partial, n, slices, parts, G,
+                   acc, cost);
     }
 }
 
