@@ -2207,7 +2207,11 @@ void tree_build(Engine& e, double theta) {
                t.inv_theta_sys, sys, e.err_word());
     ++e.launches;
     int top = -1;
-    if (T <= 8 * TOP_NODES) top = depth - 1;
+    // The whole tree where that is no slower than a launch per depth on all SMs: up to 32 768 nodes (build
+    // phase, from 4096 nodes on by depths -> all in one: 25 000 bodies 136 -> 117 us, 65 536 163 -> 140,
+    // 100 003 176 -> 152; at 40 000 nodes, 131 072 bodies, 182 -> 172 and 155 -> 164 for a disk and a
+    // Plummer sphere, at 200 000 bodies 186 -> 215).
+    if (T <= 64 * TOP_NODES) top = depth - 1;
     else
         for (size_t width = x.nroots; width <= TOP_NODES && top < depth - 1; width *= 8) ++top;
     const int cb = std::max(1, std::min(4 * e.sms, grid_for(static_cast<long long>(T), COMBINE_NODES)));

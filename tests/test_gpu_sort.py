@@ -92,9 +92,9 @@ def test_deeper_later(be):
 
 
 # The moments on both sides of the leaf counts and depth widths at which they are formed by more lanes
-# or in other launches (about 6 bodies a leaf: 4096 leaves, 512 and 4096 nodes), the second call with
+# or in other launches (about 6 bodies a leaf: 4096 leaves, 512 and 32 768 nodes), the second call with
 # the sizes of the first; a corner of the cube holds no mass (the centre is the cell's).
-@pytest.mark.parametrize("n", [3000, 12000, 20000, 25000, 27000, 31000, 60000])
+@pytest.mark.parametrize("n", [3000, 12000, 20000, 25000, 27000, 31000, 60000, 110000, 160000])
 def test_moment_widths(be, n):
     b = zero_v(S.cube(n, n))
     b.m[(b.x < 0) & (b.y < 0) & (b.z < 0)] = 0.0
