@@ -32,9 +32,9 @@
 // TP pairs of i-bodies, and summed there by lanes that hold i-bodies, with Kahan sums over the tiles.
 // Every pair is so evaluated once for both sides: 86 packed instructions for two cell pairs and 27 for
 // two body pairs, where an evaluation for each side (lanes over i-bodies, then over entries) took 153
-// and 40; the tile costs a tenth of them. One pass over the 200 000-body collision: 2.25 -> 0.99 ms against
+// and 40; the tile costs a tenth of them. One pass over the 200 000-body collision: 2.25 -> 0.91 ms against
 // one warp per group (which ended on the few largest groups, with the SMs idle for a third of it). The
-// FMA pipe is now 55% busy: three blocks of 120 registers per SM leave it waiting for latencies.
+// FMA pipe is now 60% busy: three blocks of 126 registers per SM leave it waiting for latencies.
 #include "engine.cuh"
 #include "walk_common.cuh"
 
@@ -200,61 +200,82 @@ __device__ __forceinline__ void vjp_cells(const VjpArgs& a, VjpSmem& s, const Pa
     }
 }
 
-// 32 bodies of the packet from e0 on: per pair e = w / r^3 - 3 u d / r^5, dx_j += m_j e, dm_j += u / r^3
-// and dx_i -= m_j e. The self pair is taken out by zeroing its half of the weight.
-template <bool EPS0>
+// 32 NE bodies of the packet from e0 on, NE per lane: per pair e = w / r^3 - 3 u d / r^5, dx_j += m_j e,
+// dm_j += u / r^3 and dx_i -= m_j e. The self pair is taken out by zeroing its half of the weight. Two
+// per lane share the loads of the i-bodies and the tile, whose shared-memory traffic (16 cycles a step
+// of each of four warps) would otherwise take longer than the 27 packed instructions of a pair.
+template <int NE, bool EPS0>
 __device__ __forceinline__ void vjp_bodies(const VjpArgs& a, VjpSmem& s, const Packet& k, int warp, int e0, int pairs) {
     const int lane = threadIdx.x & 31, nb = k.nb;
     const float4 o = k.centre;
     const f2x E2 = f2_bcast(a.e2), CN3 = f2_bcast(-3.f);
-    const bool on = e0 + lane < nb;
-    const int p = min(e0 + lane, nb - 1);
-    const uint32_t j = k.base[range_of(k, p)] + static_cast<uint32_t>(p);
-    const float4 h = a.hm[j], l = a.lo[j];
-    const int js = j - k.plo < k.np ? static_cast<int>(j - k.plo) : -2;
-    const float mj = on ? h.w : 0.f;
-    const f2x X = f2_bcast((h.x - o.x) + l.x), Y = f2_bcast((h.y - o.y) + l.y), Z = f2_bcast((h.z - o.z) + l.z),
-              M = f2_bcast(mj);
-    f2x GX = f2_bcast(0.f), GY = GX, GZ = GX, GM = GX;
+    uint32_t j[NE];
+    int js[NE];
+    float mj[NE];
+    f2x X[NE], Y[NE], Z[NE], M[NE], GX[NE], GY[NE], GZ[NE], GM[NE];
+#pragma unroll
+    for (int v = 0; v < NE; ++v) {
+        const int p = min(e0 + 32 * v + lane, nb - 1);
+        j[v] = k.base[range_of(k, p)] + static_cast<uint32_t>(p);
+        const float4 h = a.hm[j[v]], l = a.lo[j[v]];
+        js[v] = j[v] - k.plo < k.np ? static_cast<int>(j[v] - k.plo) : -2;
+        mj[v] = e0 + 32 * v + lane < nb ? h.w : 0.f;
+        X[v] = f2_bcast((h.x - o.x) + l.x);
+        Y[v] = f2_bcast((h.y - o.y) + l.y);
+        Z[v] = f2_bcast((h.z - o.z) + l.z);
+        M[v] = f2_bcast(mj[v]);
+        GX[v] = GY[v] = GZ[v] = GM[v] = f2_bcast(0.f);
+    }
     for (int q0 = 0; q0 < pairs; q0 += TP) {
         const int q1 = min(pairs, q0 + TP);
-#pragma unroll 2
+#pragma unroll 1
         for (int q = q0; q < q1; ++q) {
-            IPair i = load_pair(s, q);
-            const unsigned off = static_cast<unsigned>(js - 2 * q);
-            if (off <= 1u) {
-                const f2x msk = off == 0 ? f2_pack(0.f, 1.f) : f2_pack(1.f, 0.f);
-                i.wx = f2_mul(i.wx, msk);
-                i.wy = f2_mul(i.wy, msk);
-                i.wz = f2_mul(i.wz, msk);
+            const IPair ip = load_pair(s, q);
+            f2x tx = 0ull, ty = 0ull, tz = 0ull;
+#pragma unroll
+            for (int v = 0; v < NE; ++v) {
+                IPair i = ip;
+                const unsigned off = static_cast<unsigned>(js[v] - 2 * q);
+                if (off <= 1u) {
+                    const f2x msk = off == 0 ? f2_pack(0.f, 1.f) : f2_pack(1.f, 0.f);
+                    i.wx = f2_mul(i.wx, msk);
+                    i.wy = f2_mul(i.wy, msk);
+                    i.wz = f2_mul(i.wz, msk);
+                }
+                const f2x dx = f2_sub(X[v], i.x), dy = f2_sub(Y[v], i.y), dz = f2_sub(Z[v], i.z);
+                const f2x inv = inv_r2<EPS0>(f2_fma(dx, dx, f2_fma(dy, dy, f2_fma(dz, dz, E2))));
+                const f2x inv2 = f2_mul(inv, inv), inv3 = f2_mul(inv, inv2), inv5 = f2_mul(inv3, inv2);
+                const f2x u = f2_fma(i.wx, dx, f2_fma(i.wy, dy, f2_mul(i.wz, dz)));
+                const f2x t = f2_mul(f2_mul(CN3, u), inv5);
+                const f2x ex = f2_fma(i.wx, inv3, f2_mul(t, dx)), ey = f2_fma(i.wy, inv3, f2_mul(t, dy)),
+                          ez = f2_fma(i.wz, inv3, f2_mul(t, dz));
+                tx = v ? f2_fma(M[v], ex, tx) : f2_mul(M[v], ex);
+                ty = v ? f2_fma(M[v], ey, ty) : f2_mul(M[v], ey);
+                tz = v ? f2_fma(M[v], ez, tz) : f2_mul(M[v], ez);
+                GX[v] = f2_add(GX[v], ex);
+                GY[v] = f2_add(GY[v], ey);
+                GZ[v] = f2_add(GZ[v], ez);
+                GM[v] = f2_fma(u, inv3, GM[v]);
             }
-            const f2x dx = f2_sub(X, i.x), dy = f2_sub(Y, i.y), dz = f2_sub(Z, i.z);
-            const f2x inv = inv_r2<EPS0>(f2_fma(dx, dx, f2_fma(dy, dy, f2_fma(dz, dz, E2))));
-            const f2x inv2 = f2_mul(inv, inv), inv3 = f2_mul(inv, inv2), inv5 = f2_mul(inv3, inv2);
-            const f2x u = f2_fma(i.wx, dx, f2_fma(i.wy, dy, f2_mul(i.wz, dz)));
-            const f2x t = f2_mul(f2_mul(CN3, u), inv5);
-            const f2x ex = f2_fma(i.wx, inv3, f2_mul(t, dx)), ey = f2_fma(i.wy, inv3, f2_mul(t, dy)),
-                      ez = f2_fma(i.wz, inv3, f2_mul(t, dz));
-            s.tile[warp][0][q - q0][lane] = f2_mul(M, ex);
-            s.tile[warp][1][q - q0][lane] = f2_mul(M, ey);
-            s.tile[warp][2][q - q0][lane] = f2_mul(M, ez);
-            GX = f2_add(GX, ex);
-            GY = f2_add(GY, ey);
-            GZ = f2_add(GZ, ez);
-            GM = f2_fma(u, inv3, GM);
+            s.tile[warp][0][q - q0][lane] = tx;
+            s.tile[warp][1][q - q0][lane] = ty;
+            s.tile[warp][2][q - q0][lane] = tz;
         }
         sum_tile(s, warp, q0, pairs);
     }
-    if (!on) return;
-    atomicAdd(a.gx + j, static_cast<double>(mj * f2_sum(GX)));
-    atomicAdd(a.gy + j, static_cast<double>(mj * f2_sum(GY)));
-    atomicAdd(a.gz + j, static_cast<double>(mj * f2_sum(GZ)));
-    atomicAdd(a.gm + j, static_cast<double>(f2_sum(GM)));
+#pragma unroll
+    for (int v = 0; v < NE; ++v) {
+        if (e0 + 32 * v + lane >= nb) continue;
+        atomicAdd(a.gx + j[v], static_cast<double>(mj[v] * f2_sum(GX[v])));
+        atomicAdd(a.gy + j[v], static_cast<double>(mj[v] * f2_sum(GY[v])));
+        atomicAdd(a.gz + j[v], static_cast<double>(mj[v] * f2_sum(GZ[v])));
+        atomicAdd(a.gm + j[v], static_cast<double>(f2_sum(GM[v])));
+    }
 }
 
-// The evaluating warps. They take a packet's cells 32 at a time in turn, then its bodies: as 32 cells
-// cost what four times 32 bodies do, the warps that had one turn of cells less begin with four of
-// bodies.
+// The evaluating warps. They take a packet's cells 32 at a time in turn, then its bodies, 64 at a time:
+// as 32 cells cost what two times 64 bodies do, the warps that had one turn of cells less begin with
+// two of bodies.
 template <bool EPS0>
 __device__ __forceinline__ void vjp_evaluate(const VjpArgs& a, VjpSmem& s) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -287,13 +308,15 @@ __device__ __forceinline__ void vjp_evaluate(const VjpArgs& a, VjpSmem& s) {
             __syncwarp();
             bar_sync(kBarEval, EVAL);
         }
-        const int tc = (k.nc + 31) >> 5, tb = (k.nb + 31) >> 5;
+        const int tc = (k.nc + 31) >> 5, tb = (k.nb + 63) >> 6;
         for (int t = warp; t < tc; t += EWARPS) vjp_cells<EPS0>(a, s, k, warp, 32 * t, pairs);
         const int ahead = tc % EWARPS, behind = EWARPS - ahead;
-        const int lead = ahead ? 4 * behind : 0;  // turns of bodies for the warps behind
+        const int lead = ahead ? 2 * behind : 0;  // turns of bodies for the warps behind
         for (int t = 0; t < tb; ++t) {
             const int who = t < lead ? ahead + t % behind : (t - lead) % EWARPS;
-            if (who == warp) vjp_bodies<EPS0>(a, s, k, warp, 32 * t, pairs);
+            if (who != warp) continue;
+            if (k.nb - 64 * t > 32) vjp_bodies<2, EPS0>(a, s, k, warp, 64 * t, pairs);
+            else vjp_bodies<1, EPS0>(a, s, k, warp, 64 * t, pairs);
         }
         __syncwarp();
         bar_arrive(kBarEmpty + sl, WBS);  // the packet is read
