@@ -111,6 +111,7 @@ struct ZeroList {
 struct TreeState {
     // sort
     DevBuf keysA, keysB, valsA, valsB, hist, lookback;
+    bool clusters_of_16 = false;  // k_combine_top may be launched as one
     bool sort_full = false;  // a partial sort met a run too long to order locally: all key bits from now on
     // sorted frame-0 keys, per-body tree data
     DevBuf skey, leafid;
@@ -1894,8 +1895,6 @@ int bits_for(int count) {
 }  // namespace
 
 std::unique_ptr<TreeState, void (*)(TreeState*)> make_tree_state() {
-    // Clusters of 16 blocks are an opt-in size.
-    LG_CK(cudaFuncSetAttribute(k_combine_top, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     return std::unique_ptr<TreeState, void (*)(TreeState*)>(new TreeState, destroy_tree);
 }
 
@@ -2221,6 +2220,11 @@ void tree_build(Engine& e, double theta) {
         ++e.launches;
     }
     if (top >= 0) {
+        // Clusters of 16 blocks are an opt-in size, for the current device.
+        if (!t.clusters_of_16) {
+            LG_CK(cudaFuncSetAttribute(k_combine_top, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            t.clusters_of_16 = true;
+        }
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute at[2] = {};
         at[0].id = cudaLaunchAttributeClusterDimension;

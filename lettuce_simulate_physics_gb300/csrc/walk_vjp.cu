@@ -437,8 +437,9 @@ __global__ void k_body_field(TreeView tv, const BodyArrays b, int n, const doubl
 template <bool EPS0>
 void launch_vjp(Engine& e, VjpArgs& a) {
     static int per_sm = 0;
+    // On each launch: it holds for the current device only.
+    LG_CK(cudaFuncSetAttribute(k_walk_vjp<EPS0>, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(VjpSmem)));
     if (!per_sm) {
-        LG_CK(cudaFuncSetAttribute(k_walk_vjp<EPS0>, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(VjpSmem)));
         int fit = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_walk_vjp<EPS0>, WBS, sizeof(VjpSmem)) != cudaSuccess)
             cudaGetLastError();
