@@ -630,12 +630,13 @@ def run_reference(args, w, world, rank, dist):
 
 
 # Algorithmic bytes per body of the tree step's memory-side phases (this engine's layout):
-#   sort:  bounding box (read FP64 x, y, z: 24), keys (read 24, write key 8 + index 4), histogram
-#          (read keys 8), eight onesweep passes (read and write key + index: 24 each), permute (read
-#          and write the body arrays, 81 B each way, plus the index 4);
+#   sort:  bounding box (read FP64 x, y, z: 24), keys (read 24, write the whole key and the sorted
+#          digits, 8 each), five onesweep passes (the 1e6 disk's depth: read and write key + index, 24
+#          each; the first reads no index), permute (read and write the body arrays, 81 B each way,
+#          plus the index 4 and both keys 16);
 #   build: keys read once (8), positions and masses read once by the leaf moments (32), node
 #          records written once (about N/4 nodes x 96 B: range, geometry, moments).
-SORT_BYTES_PER_BODY = 24 + 36 + 8 + 8 * 24 + 2 * 81 + 4
+SORT_BYTES_PER_BODY = 24 + 40 + 5 * 24 - 4 + 2 * 81 + 4 + 16
 BUILD_BYTES_PER_BODY = 8 + 32 + 24
 
 
@@ -656,9 +657,9 @@ def phase_roofline(n, sort_ms, build_ms):
         out[name] = {"bound": "hbm", "bytes_per_body": per, "achieved": round(gbs, 1) if gbs else None,
                      "peak": peak, "unit": "GB/s", "frac": round(gbs / peak, 4) if gbs else None,
                      "peak_source": src}
-    out["build"]["note"] = ("FP64-latency bound in practice: the moments upsweep (leaf moments and one "
-                            "launch per tree level) is about half of the phase")
-    out["sort"]["note"] = "eight dependent onesweep passes, each limited by its decoupled look-back"
+    out["build"]["note"] = ("FP64-latency bound in practice: the moments upsweep (leaf moments, one launch "
+                            "per wide tree level, one for the narrow ones) is about 60% of the phase")
+    out["sort"]["note"] = "five dependent onesweep passes, each limited by its decoupled look-back"
     return out
 
 
