@@ -33,12 +33,12 @@
 //     child of v = 1 + exclusive scan of the masks' bit counts over pre-order (k_node_scan), a child's
 //     place under its parent the bits below its own (k_nodes_out).
 //  7. Upsweep in FP64, children always combined in index order: one launch for the leaves (one
-//     thread per leaf, leaves bucketed by body count), then the depths from the deepest (four lanes
-//     per node, each sequential sum folded by one lane), the narrow depths at the top together in
-//     one launch. The group boxes are computed on a side stream meanwhile. (A single-launch form in
-//     which the last-arriving child of each node combines it was measured slower: its combines run
-//     one node per thread in sparse warps, and an FP64 warp instruction costs the same however few
-//     lanes are active.)
+//     thread per leaf, leaves bucketed by body count; eight lanes per leaf in small trees), then the
+//     depths from the deepest (eight lanes per node, each sequential sum folded by one lane), the
+//     narrow depths at the top, or all of a small tree's, together in one launch. The group boxes are
+//     computed on a side stream meanwhile. (A single-launch form in which the last-arriving child of
+//     each node combines it was measured slower: its combines run one node per thread in sparse
+//     warps, and an FP64 warp instruction costs the same however few lanes are active.)
 // Steps 4 to 6 are four launches (they were 22 with their scans, and 13 clears; build phase 238 ->
 // 146 us at 8191 bodies, 289 -> 200 at 1e5, 514 -> 385 on the 1e6 disk, 4.16 -> 3.26 ms at 1.6e7).
 #include <cuda_runtime.h>
