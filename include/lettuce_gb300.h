@@ -318,6 +318,9 @@ lg_status lg_ensemble_tune(lg_ensemble* en);
 lg_status lg_ensemble_get_tuning(lg_ensemble* en, lg_ensemble_tuning* out);
 lg_status lg_ensemble_set_tuning(lg_ensemble* en, const lg_ensemble_tuning* t);
 lg_status lg_ensemble_get_stats(lg_ensemble* en, lg_ensemble_stats* out);
+/* Self-test of failure detection: as lg_probe_wait_timeout, but the waits that gave up are left to be
+ * reported by the ensemble's next call that computes forces, as those of one of its steps would be. */
+lg_status lg_ensemble_probe_wait_timeout(lg_ensemble* en, unsigned polls);
 
 /* Direct-summation forces with no device allocation. No counterpart in the reference: it is for
  * callers that cannot allocate device memory when they need forces, such as a code that owns all

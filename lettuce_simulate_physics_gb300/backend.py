@@ -230,6 +230,7 @@ def _lib() -> C.CDLL:
         "lg_ensemble_get_tuning": (st, [vp, C.POINTER(_CEnsTuning)]),
         "lg_ensemble_set_tuning": (st, [vp, C.POINTER(_CEnsTuning)]),
         "lg_ensemble_get_stats": (st, [vp, C.POINTER(_CEnsStats)]),
+        "lg_ensemble_probe_wait_timeout": (st, [vp, C.c_uint]),
     }
     for name, (res, args) in sigs.items():
         fn = getattr(lib, name)

@@ -381,6 +381,14 @@ public:
 
     lg_ensemble_tuning tuning() const { return tuning_; }
 
+    void probe_wait_timeout(unsigned polls) {
+        Engine& e = *e_;
+        if (polls < 1 || polls > (1u << 20)) fail(kArg, "ensemble probe_wait_timeout: polls must be in [1, 2^20]");
+        LG_CK(cudaSetDevice(e.dev));
+        probe_waits(e.stream, polls, e.ticket(), e.err_word());  // (the ticket is zero between launches)
+        ++e.launches;
+    }
+
     lg_ensemble_stats stats() const {
         lg_ensemble_stats s = stats_;
         s.nsys = nsys_;
@@ -811,6 +819,10 @@ lg_status lg_ensemble_set_tuning(lg_ensemble* en, const lg_ensemble_tuning* t) {
         if (!t) lg::fail(lg::kArg, "null pointer: tuning");
         ens(en).set_tuning(*t);
     });
+}
+
+lg_status lg_ensemble_probe_wait_timeout(lg_ensemble* en, unsigned polls) {
+    return eguard([&] { ens(en).probe_wait_timeout(polls); });
 }
 
 lg_status lg_ensemble_get_stats(lg_ensemble* en, lg_ensemble_stats* out) {

@@ -1940,7 +1940,8 @@ void tree_sort(Engine& e) {
         z.span[1] = {t.hist.as<uint4>(), hist_words()};
         z.span[2] = {t.lookback.as<uint4>(), lookback_words(n, passes)};
         z.span[3] = {t.leaf_state.as<uint4>(), leaf_state_words(n)};
-        z.span[4] = {reinterpret_cast<uint4*>(e.err_word()), 1};  // (the frame kernel's ticket lies behind it)
+        // A forest's runs read the error word once, after all their steps: it is theirs to clear.
+        if (!sys) z.span[4] = {reinterpret_cast<uint4*>(e.err_word()), 1};  // (the frame kernel's ticket lies behind it)
         if (sys) {
             launch_pdl(overlap(n), k_frame_sys, t.nsys, BS, s, e.bodies(e.cur), t.sys_off,
                        t.frame.as<double>(), z);

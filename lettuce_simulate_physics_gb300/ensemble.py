@@ -131,6 +131,11 @@ class Ensemble:
         t.tuned = 1
         _check(self._lib.lg_ensemble_set_tuning(self._h, C.byref(t)))
 
+    def probe_wait_timeout(self, polls: int = 4096) -> None:
+        """Self-test of failure detection: device waits that are never satisfied give up after `polls`
+        polls; the next call that computes forces reports them (RuntimeError)."""
+        _check(self._lib.lg_ensemble_probe_wait_timeout(self._h, int(polls)))
+
     def stats(self) -> EnsembleStats:
         s = _CEnsStats()
         _check(self._lib.lg_ensemble_get_stats(self._h, C.byref(s)))
