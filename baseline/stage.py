@@ -22,12 +22,14 @@ STAGE = os.path.join(HERE, "_ref", "lettuce")
 PARTS = ("src", "tests", "vendor", "configs")
 
 
+def is_checkout(path: str) -> bool:
+    return os.path.isfile(os.path.join(path, "src", "backend.hpp"))
+
+
 def staged_root() -> str | None:
     """The reference checkout to build from: LETTUCE_REF if set, else the staged copy if present."""
-    env = os.environ.get("LETTUCE_REF")
-    if env:
-        return env if os.path.isfile(os.path.join(env, "src", "backend.hpp")) else None
-    return STAGE if os.path.isfile(os.path.join(STAGE, "src", "backend.hpp")) else None
+    path = os.environ.get("LETTUCE_REF") or STAGE
+    return path if is_checkout(path) else None
 
 
 def _same_tree(a: str, b: str) -> bool:
@@ -42,7 +44,7 @@ def _same_tree(a: str, b: str) -> bool:
 def stage(checkout: str) -> str:
     """Copies the parts of `checkout` into the stage (unchanged files keep their times, so the
     recipes above do not rebuild). Returns the stage path."""
-    if not os.path.isfile(os.path.join(checkout, "src", "backend.hpp")):
+    if not is_checkout(checkout):
         raise FileNotFoundError(f"{checkout} is not a lettuce checkout (no src/backend.hpp)")
     os.makedirs(STAGE, exist_ok=True)
     for part in PARTS:
