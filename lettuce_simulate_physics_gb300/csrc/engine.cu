@@ -263,6 +263,7 @@ void Engine::download(float* x, float* y, float* z, float* vx, float* vy, float*
 }
 
 unsigned* Engine::err_word() const { return small.as<unsigned>(); }
+unsigned* Engine::side_err_word() const { return err_word() + 1; }
 unsigned* Engine::ticket() const { return small.as<unsigned>() + 4; }
 unsigned long long* Engine::inter_counter() const { return reinterpret_cast<unsigned long long*>(small.as<char>() + 64); }
 double* Engine::dscratch() const { return reinterpret_cast<double*>(small.as<char>() + 128); }

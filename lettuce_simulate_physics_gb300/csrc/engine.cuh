@@ -117,6 +117,7 @@ struct Engine {
     BodyArrays bodies(int which) const;
     void reserve_bodies(size_t count);
     unsigned* err_word() const;
+    unsigned* side_err_word() const;  // of kernels that run beside a tree's (an ensemble's direct systems)
     unsigned* ticket() const;
     unsigned long long* inter_counter() const;
     double* dscratch() const;

@@ -320,11 +320,11 @@ public:
                 const int nw = static_cast<int>(items.size());
                 for (int tile : kTileCandidates) {
                     launch_direct_batch(b, tune_work_.as<DirectWork>(), nw, ipt, tile, static_cast<float>(G_), false,
-                                        false, e.acc.as<float4>(), e.err_word(), s);
+                                        false, e.acc.as<float4>(), e.side_err_word(), s);
                     LG_CK(cudaEventRecord(t0_, s));
                     for (int r = 0; r < 5; ++r)
                         launch_direct_batch(b, tune_work_.as<DirectWork>(), nw, ipt, tile, static_cast<float>(G_),
-                                            false, false, e.acc.as<float4>(), e.err_word(), s);
+                                            false, false, e.acc.as<float4>(), e.side_err_word(), s);
                     LG_CK(cudaEventRecord(t1_, s));
                     LG_CK(cudaStreamSynchronize(s));
                     float ms = 0;
@@ -418,7 +418,7 @@ private:
             // copies those bodies unchanged into the other set, and writes acc only below n_tree.
             for (const Segment& g : segs_) {
                 launch_direct_batch(b, d_work_.as<DirectWork>() + g.first, g.count, g.ipt, g.tile,
-                                    static_cast<float>(G_), pot, false, e.acc.as<float4>(), e.err_word(), ds);
+                                    static_cast<float>(G_), pot, false, e.acc.as<float4>(), e.side_err_word(), ds);
                 ++e.launches;
             }
             if (split) LG_CK(cudaEventRecord(join_, side_));
@@ -454,7 +454,7 @@ private:
             LG_CK(cudaStreamSynchronize(s));
             if (n_tree_ > 0 && !tree_verify(e, e.pinned_small + 64)) {
                 if (attempt >= 2) fail(kRuntime, "ensemble: tree sizes still wrong after an exact rebuild");
-                LG_CK(cudaMemsetAsync(e.err_word(), 0, 4, s));
+                LG_CK(cudaMemsetAsync(e.err_word(), 0, 8, s));
                 continue;
             }
             check_err("ensemble forces");
@@ -472,9 +472,9 @@ private:
 
     void check_err(const char* where) {
         Engine& e = *e_;
-        const unsigned w = e.pinned_small[0];
+        const unsigned w = e.pinned_small[0] | e.pinned_small[1];
         if (!w) return;
-        LG_CK(cudaMemsetAsync(e.err_word(), 0, 4, e.stream));
+        LG_CK(cudaMemsetAsync(e.err_word(), 0, 8, e.stream));
         LG_CK(cudaStreamSynchronize(e.stream));
         std::string why;
         if (w & kErrWaitTimeout) why += " wait-timeout";

@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(SORT_BS) k_sort_pass(const uint64_t* __restric
         const uint64_t k = stage_k[p];
         const int d = static_cast<int>((k >> shift) & 255);
         const unsigned gpos = gbase[d] + (p - tstart[d]);
-        if (gpos < static_cast<unsigned>(n)) {  // false only after a wait that timed out
+        if (gpos < static_cast<unsigned>(n)) {  // false only after a wait that ran out
             dst_k[gpos] = k;
             dst_v[gpos] = stage_v[p];
         }
@@ -544,18 +544,20 @@ __global__ void __launch_bounds__(SORT_BS) k_sort_pass(const uint64_t* __restric
 // that of a stable sort by the whole keys. A run of more than LEAF_MAX is left as it is and
 // flagged: the tree is then deeper than the sorted digits, and the sort is redone with all of them.
 // key1_in (optional): a second key carried through the permutation (no partial runs then).
+// After a wait of the passes that ran out (*err) the permutation is not one: every body keeps its
+// place, and the kernels that follow do nothing (build_ok).
 __global__ void k_permute(const BodyArrays src, BodyArrays dst, const uint64_t* __restrict__ keys,
                           const uint32_t* __restrict__ vals, const uint64_t* __restrict__ mkeys,
                           uint64_t* __restrict__ skey, const uint64_t* __restrict__ key1_in,
-                          uint64_t* __restrict__ key1_out, int n, int n_total, int partial, unsigned* long_run) {
+                          uint64_t* __restrict__ key1_out, int n, int n_total, int partial, unsigned* long_run,
+                          const unsigned* err) {
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_total) return;
     int to = i;
     uint32_t j = static_cast<uint32_t>(i);  // bodies past the tree's range (the forest's direct systems) stay
-    if (i < n) {
+    if (i < n && !(*err & kErrWaitTimeout)) {
         j = vals[i];
-        if (j >= static_cast<uint32_t>(n)) return;  // only after a wait that timed out
         if (skey) {
             const uint64_t m = mkeys[j];
             if (partial) {
@@ -576,6 +578,9 @@ __global__ void k_permute(const BodyArrays src, BodyArrays dst, const uint64_t* 
             skey[to] = m;
         }
         if (key1_in) key1_out[to] = key1_in[j];
+    } else if (i < n) {
+        if (skey) skey[i] = mkeys[i];
+        if (key1_in) key1_out[i] = key1_in[i];
     }
     dst.x[to] = src.x[j];
     dst.y[to] = src.y[j];
@@ -993,8 +998,12 @@ struct NodeCtx {
     unsigned nroots;       // systems in the forest (1 for one system); roots take node indices 0..nroots-1
 };
 
-// Whether the leaves are there and fit what the build was launched for, and their number and the nodes'.
-__device__ __forceinline__ bool build_ok(const unsigned* counts) { return counts[8] != 0; }
+// Whether the leaves are there and fit what the build was launched for, and no wait before this kernel
+// ran out: what a kernel left after one is not to be used as an index. (In a forest only the tree's own
+// kernels, one after another, set that bit; the direct systems' have a word of their own.)
+__device__ __forceinline__ bool build_ok(const unsigned* counts, const unsigned* err) {
+    return counts[8] != 0 && !(*err & kErrWaitTimeout);
+}
 
 // Pre-order nodes as k_nodes leaves them. meta: depth | leaf << 8 | group << 9 | octal digit under
 // the parent << 10; mask (zero before): which of a node's eight octants have a child; first: its
@@ -1052,10 +1061,10 @@ __device__ __forceinline__ int last_sharing(int a, int end, F&& share) {
 // node that is not its leaf's first is the node before it, that of a first node the node at depth
 // c[l] that also holds the body before the leaf.
 constexpr int NODE_BS = 256;
-__global__ void __launch_bounds__(NODE_BS) k_nodes(NodeCtx x, PreNodes pn) {
+__global__ void __launch_bounds__(NODE_BS) k_nodes(NodeCtx x, PreNodes pn, const unsigned* err) {
     pdl_wait();
     __shared__ int l_first;
-    if (!build_ok(x.counts)) return;
+    if (!build_ok(x.counts, err)) return;
     const uint32_t T = x.counts[2];
     const int K = static_cast<int>(x.counts[1]);
     const uint32_t v0 = blockIdx.x * NODE_BS;
@@ -1130,7 +1139,7 @@ __global__ void __launch_bounds__(NSCAN_BS) k_node_scan(NodeCtx x, PreNodes pn, 
     pdl_wait();
     __shared__ unsigned long long warp_sum[NSCAN_BS / 32], prefix_s;
     __shared__ unsigned tile_s, bucket[NBUCKET];
-    if (!build_ok(x.counts)) return;
+    if (!build_ok(x.counts, err)) return;
     const uint32_t T = x.counts[2];
     const int tid = threadIdx.x;
     if (tid == 0) tile_s = atomicAdd(tile_ctr, 1u);
@@ -1215,7 +1224,7 @@ __global__ void __launch_bounds__(NODE_BS) k_nodes_out(NodeCtx x, PreNodes pn, c
                                                        unsigned* err) {
     pdl_wait();
     __shared__ unsigned start[NBUCKET], count[NBUCKET];
-    if (!build_ok(x.counts)) return;
+    if (!build_ok(x.counts, err)) return;
     const uint32_t T = x.counts[2], K = x.counts[1];
     const int tid = threadIdx.x;
     if (blockIdx.x * NODE_BS >= T) return;
@@ -1473,7 +1482,7 @@ __global__ void k_leaf_moments(const uint32_t* __restrict__ leaf_order, const un
                                const float* __restrict__ inv_theta_sys, const uint32_t* __restrict__ sys, unsigned* err) {
     pdl_wait();
     const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (!build_ok(counts)) return;
+    if (!build_ok(counts, err)) return;
     const uint32_t T = counts[2];
     if (l >= counts[1]) return;
     const uint32_t node = leaf_order[l];
@@ -1565,7 +1574,7 @@ __global__ void __launch_bounds__(LEAFW_BS) k_leaf_moments_wide(const uint32_t* 
                                                                 const uint32_t* __restrict__ sys, unsigned* err) {
     __shared__ __align__(16) double rows[LEAFW_BS / WIDE][8][ROW];
     pdl_wait();
-    if (!build_ok(counts)) return;
+    if (!build_ok(counts, err)) return;
     const uint32_t T = counts[2], K = counts[1];
     const int lane = threadIdx.x & 31, j = lane & 7, base = lane & ~7;
     double(*row)[ROW] = rows[threadIdx.x / WIDE];
@@ -1754,7 +1763,7 @@ __global__ void __launch_bounds__(COMBINE_BS) k_combine_level(const uint32_t* __
                                                               const uint32_t* __restrict__ sys, unsigned* err) {
     __shared__ __align__(16) double rows[COMBINE_NODES][ROW][ROW];
     pdl_wait();
-    if (!build_ok(counts)) return;
+    if (!build_ok(counts, err)) return;
     const uint32_t T = counts[2];
     const unsigned lo = dep_begin(ix, depth), hi = dep_begin(ix, depth + 1), end = dep_begin(ix, depth + 2);
     const unsigned sub = threadIdx.x / WIDE, of = gridDim.x * COMBINE_NODES;
@@ -1777,7 +1786,7 @@ __global__ void __launch_bounds__(TOP_BS) k_combine_top(const uint32_t* __restri
                                                         const uint32_t* __restrict__ sys, unsigned* err) {
     __shared__ __align__(16) double rows[TOP_BS / WIDE][ROW][ROW];
     pdl_wait();
-    if (!build_ok(counts)) return;  // the same word for all blocks
+    if (!build_ok(counts, err)) return;  // the same words for all blocks
     const uint32_t T = counts[2];
     const unsigned sub = threadIdx.x / WIDE;
     // Nodes in order go to the blocks' first warps, then to their second: a narrow depth is spread
@@ -1969,7 +1978,7 @@ void tree_sort(Engine& e) {
         launch_pdl(overlap(n), k_permute, grid_for(n_total, BS), BS, s, e.bodies(e.cur), e.bodies(other),
                    at ? t.keysB.as<uint64_t>() : t.keysA.as<uint64_t>(),
                    at ? t.valsB.as<uint32_t>() : t.valsA.as<uint32_t>(), t.mkeys.as<uint64_t>(),
-                   t.skey.as<uint64_t>(), nullptr, nullptr, n, n_total, full ? 0 : 1, counts + 7);
+                   t.skey.as<uint64_t>(), nullptr, nullptr, n, n_total, full ? 0 : 1, counts + 7, e.err_word());
         ++e.launches;
         e.cur = other;
         if (full) {
@@ -2032,7 +2041,7 @@ void tree_sort(Engine& e) {
         const int other = e.cur ^ 1;
         launch_pdl(overlap(n), k_permute, grid_for(n_total, BS), BS, s, e.bodies(e.cur), e.bodies(other),
                    t.keysA.as<uint64_t>(), t.valsA.as<uint32_t>(), nullptr, nullptr, key1,
-                   t.fkey[f].as<uint64_t>(), n, n_total, 0, nullptr);
+                   t.fkey[f].as<uint64_t>(), n, n_total, 0, nullptr, e.err_word());
         e.cur = other;
         ft.key[f] = t.fkey[f].as<uint64_t>();
         ft.runid[f] = runid;
@@ -2094,7 +2103,7 @@ void tree_build(Engine& e, double theta) {
         LG_CK(cudaStreamSynchronize(s));
         const size_t Kx = e.pinned_small[1], Tx = e.pinned_small[2];
         const int dx = static_cast<int>(e.pinned_small[4]);
-        if (Kx < 1 || Kx > static_cast<size_t>(n) || Tx < Kx)
+        if (Kx < 1 || Kx > static_cast<size_t>(n) || Tx < Kx || Tx > Kx * (MAX_DEPTH + 1))
             fail(kRuntime, "cuda tree build: bad leaf/node count " + std::to_string(Kx) + "/" + std::to_string(Tx));
         // Headroom for the sync-free builds that follow (LETTUCE_GB300_TREE_HEADROOM percent, default
         // 25, plus a fixed slack unless it is 0): more memory against fewer exact rebuilds.
@@ -2148,7 +2157,7 @@ void tree_build(Engine& e, double theta) {
     const NodeCtx x{sys, k0, ft, leaf, n, counts, static_cast<unsigned>(sys ? t.nsys : 1)};
     const uint32_t Tc = static_cast<uint32_t>(T);
     const int tb = grid_for(static_cast<long long>(T), NODE_BS);
-    launch_pdl(overlap(n), k_nodes, tb, NODE_BS, s, x, pn);
+    launch_pdl(overlap(n), k_nodes, tb, NODE_BS, s, x, pn, e.err_word());
     launch_pdl(overlap(n), k_node_scan, scan_tiles, NSCAN_BS, s, x, pn, scan_state,
                reinterpret_cast<unsigned*>(scan_state + scan_tiles), counts, ix, t.grp_node.as<uint32_t>(),
                e.err_word());

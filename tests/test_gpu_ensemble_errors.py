@@ -45,3 +45,23 @@ def test_first_forces_report_an_error(call):
     with ensemble([1, 0]) as en:
         with pytest.raises(ValueError):
             en.probe_wait_timeout(0)
+
+
+# After a wait that ran out the permutation and the tree may be anything: the gather leaves every body
+# where it is, and nothing else of the build or the walk runs.
+def test_bodies_stay_in_place_after_a_wait_that_ran_out():
+    n = 5000
+    b = S.plummer(n, 3, cut=10)
+    b.vx[:] = b.vy[:] = b.vz[:] = 0
+    b.id[:] = np.arange(n)
+    with ensemble([0]) as en:
+        for _ in range(2):
+            en.upload(b, [n], [0.02], [0.6], [1])
+            en.probe_wait_timeout(2048)
+            with pytest.raises(RuntimeError, match="wait-timeout"):
+                en.energy()
+            out = en.download()
+            for f in FIELDS:
+                assert np.array_equal(getattr(out, f), getattr(b, f)), f
+            en.energy()
+            assert not np.array_equal(en.download().id, b.id)  # sorted
