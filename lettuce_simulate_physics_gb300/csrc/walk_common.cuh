@@ -118,6 +118,7 @@ __device__ __forceinline__ void build_lists(const ListArgs& w, S& s) {
     if (lane < BWORDS) s.pk[0].starts[lane] = s.pk[1].starts[lane] = 0u;
     __syncwarp();
     auto send = [&](unsigned flags) {
+        __syncwarp();  // the lanes' entries and start bits are there
         list_len += static_cast<uint32_t>(nc + nb);
         cells_len += static_cast<uint32_t>(nc);
         Packet& k = s.pk[sent & 1];
