@@ -237,6 +237,9 @@ lg_status lg_probe_fp32_peak(lg_engine* e, double* tflops);
  * primitives the kernels use. Both waits give up; the call returns LG_ERR_RUNTIME with "device wait
  * timed out" in lg_last_error(), the error word is cleared and the engine stays usable. */
 lg_status lg_probe_wait_timeout(lg_engine* e, unsigned polls);
+/* The same waits, left in the error word for the call after this one that reads it (an adjoint pass) or
+ * replaces what it speaks of (a tree build), as those of a kernel of that call would be. */
+lg_status lg_probe_wait_pending(lg_engine* e, unsigned polls);
 /* Page-locked host memory for transfers that overlap (cudaMallocHost / cudaFreeHost). */
 lg_status lg_host_alloc(size_t bytes, void** out);
 lg_status lg_host_free(void* p);

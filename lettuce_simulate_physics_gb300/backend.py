@@ -213,6 +213,7 @@ def _lib() -> C.CDLL:
         "lg_interaction_split": (st, [vp, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]),
         "lg_probe_fp32_peak": (st, [vp, C.POINTER(C.c_double)]),
         "lg_probe_wait_timeout": (st, [vp, C.c_uint]),
+        "lg_probe_wait_pending": (st, [vp, C.c_uint]),
         "lg_host_alloc": (st, [C.c_size_t, C.POINTER(vp)]),
         "lg_adjoint_forward": (st, [vp, C.POINTER(_CForceParams), C.c_double, C.c_int, C.c_int]),
         "lg_adjoint_backward": (st, [vp, _d, _d, _d, _d, _d, _d, _d, _d, _d, _d, _d]),
@@ -532,6 +533,10 @@ class CudaBackend:
         `polls` polls and the call raises RuntimeError("... device wait timed out ..."); the engine
         stays usable."""
         _check(self._lib.lg_probe_wait_timeout(self._h, int(polls)))
+
+    def probe_wait_pending(self, polls: int = 4096) -> None:
+        """The waits of probe_wait_timeout, left for an adjoint pass to report."""
+        _check(self._lib.lg_probe_wait_pending(self._h, int(polls)))
 
     def adjoint_forward(self, p: ForceParams, dt: float, steps: int, checkpoint_every: int) -> None:
         """Runs `steps` KDK steps from the resident state, keeping adjoint checkpoints."""

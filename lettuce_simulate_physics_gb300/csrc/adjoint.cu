@@ -727,6 +727,7 @@ void adjoint_forward(Engine& e, AdjointState& a, const lg_force_params& p, doubl
     e.tree_ok = tree;
     e.costs_ok = tree;
     a.have_forward = true;
+    LG_CK(cudaMemcpyAsync(e.pinned_small, e.err_word(), 4, cudaMemcpyDeviceToHost, e.stream));
     LG_CK(cudaStreamSynchronize(e.stream));
     e.check_device_errors("adjoint forward");
 }
@@ -994,6 +995,7 @@ double adjoint_backward(Engine& e, AdjointState& a, const double* tx, const doub
     std::vector<uint32_t> ids(tree ? 0 : static_cast<size_t>(n));
     if (!tree)
         LG_CK(cudaMemcpyAsync(ids.data(), e.bodies(e.cur).id, static_cast<size_t>(n) * 4, cudaMemcpyDeviceToHost, s));
+    LG_CK(cudaMemcpyAsync(e.pinned_small, e.err_word(), 4, cudaMemcpyDeviceToHost, s));
     LG_CK(cudaStreamSynchronize(s));
     e.check_device_errors("adjoint backward");
     double L = 0;

@@ -952,6 +952,16 @@ lg_status lg_probe_wait_timeout(lg_engine* e, unsigned polls) {
     });
 }
 
+lg_status lg_probe_wait_pending(lg_engine* e, unsigned polls) {
+    return guard([&] {
+        Engine& E = eng(e);
+        if (polls < 1 || polls > (1u << 20)) lg::fail(lg::kArg, "probe_wait_pending: polls must be in [1, 2^20]");
+        LG_CK(cudaSetDevice(E.dev));
+        lg::probe_waits(E.stream, polls, E.ticket(), E.err_word());  // (the ticket is zero between launches)
+        ++E.launches;
+    });
+}
+
 lg_status lg_adjoint_forward(lg_engine* e, const lg_force_params* p, double dt, int steps, int checkpoint_every) {
     return guard([&] {
         need(p, "params");
