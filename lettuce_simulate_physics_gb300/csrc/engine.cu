@@ -110,9 +110,25 @@ Engine::~Engine() {
     if (stream) cudaStreamDestroy(stream);
 }
 
+namespace {
+// Memory that CUDA knows: page-locked, managed or its own (0.4 us).
+bool known_to_cuda(const void* p) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type != cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return false;
+}
+}  // namespace
+
+// A copy may not reach over the end of a page-locked range, and addresses alone do not tell whether two
+// such columns are one: only pageable ones are joined.
 int adjacent_columns(void* const* dst, int c, int columns, size_t bytes) {
+    auto next = [&](int k) {
+        return c + k < columns && dst[c] && dst[c + k] == static_cast<char*>(dst[c]) + bytes * static_cast<size_t>(k);
+    };
+    if (!next(1) || known_to_cuda(dst[c])) return 1;
     int k = 1;
-    while (c + k < columns && dst[c] && dst[c + k] == static_cast<char*>(dst[c]) + bytes * static_cast<size_t>(k)) ++k;
+    while (next(k) && !known_to_cuda(dst[c + k])) ++k;
     return k;
 }
 
@@ -125,12 +141,7 @@ void map_host_pages(void* const* dst, int columns, size_t bytes) {
         k = adjacent_columns(dst, c, columns, bytes);
         char *p = static_cast<char*>(dst[c]), *end = p + bytes * static_cast<size_t>(k);
         if (!p) continue;
-        // To ask whether it is page-locked takes 10 us, as long as to write to 2 MB of pages that are.
-        if (end - p > (2 << 20)) {
-            cudaPointerAttributes at{};
-            if (cudaPointerGetAttributes(&at, p) != cudaSuccess) cudaGetLastError();
-            else if (at.type != cudaMemoryTypeUnregistered) continue;
-        }
+        if (known_to_cuda(p)) continue;
         total += static_cast<size_t>(end - p);
         for (char* q = p; q < end; q += kShare) parts.emplace_back(q, std::min(q + kShare, end));
     }

@@ -81,7 +81,7 @@ struct BodySet {
 // (83 MB took 70 ms that way; one thread maps them in 2.7 ms, several, where there are many, in 1, and
 // the copy then takes 0.6). `columns` arrays of `bytes` each; those that follow one another count as one.
 void map_host_pages(void* const* dst, int columns, size_t bytes);
-// Columns c .. of dst that follow column c in memory, itself included.
+// Columns c .. of dst that follow column c in memory and may be written as one, itself included.
 int adjacent_columns(void* const* dst, int c, int columns, size_t bytes);
 
 struct Engine {
