@@ -78,8 +78,9 @@ struct BodySet {
 
 // Has the CPU give memory to those pages of host arrays (null ones are left out) that have none yet,
 // before a copy fills them: a caller's new arrays, whose pages the copy would fault in from the device
-// (83 MB took 70 ms that way; one thread maps them in 2.7 ms, several, where there are many, in 1, and
-// the copy then takes 0.6). `columns` arrays of `bytes` each; those that follow one another count as one.
+// (83 MB took 70 ms that way; one thread maps them in 2 ms, several, where there are many, in 1.2, and
+// the copy then takes 0.6). The arrays' contents stay as they are, so it may run beside work that can
+// still fail. `columns` arrays of `bytes` each; those that follow one another count as one.
 void map_host_pages(void* const* dst, int columns, size_t bytes);
 // Columns c .. of dst that follow column c in memory and may be written as one, itself included.
 int adjacent_columns(void* const* dst, int c, int columns, size_t bytes);

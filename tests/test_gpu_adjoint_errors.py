@@ -53,3 +53,20 @@ def test_direct_passes_report_waits_that_ran_out(be, n):
     assert np.isfinite(be.adjoint_backward(target)[0])
     with pytest.raises(ValueError):
         be.probe_wait_pending(0)
+
+
+# The gradients' arrays are the caller's until the pass has succeeded, new ones without pages among them
+# (131 072 bodies: 8 MB and more).
+@pytest.mark.parametrize("n", [3000, 131072])
+def test_a_pass_that_fails_leaves_the_arrays_alone(be, n):
+    b, p, target = problem(n, L.ForceMethod.direct)
+    t = np.ascontiguousarray(target.T)
+    seven = np.full((7, n), 7.0)
+    d = lambda a: a.ctypes.data_as(L.backend._d)
+    be.upload(b)
+    be.adjoint_forward(p, 1e-3, 1, 1)
+    be.probe_wait_pending(2048)
+    with pytest.raises(RuntimeError, match="device wait timed out"):
+        L.backend._check(be._lib.lg_adjoint_backward(be._h, *(d(t[k]) for k in range(3)), None,
+                                                     *(d(seven[k]) for k in range(7))))
+    assert (seven == 7.0).all()
