@@ -1752,10 +1752,10 @@ __device__ __forceinline__ void rcrit_range(const uint32_t* __restrict__ dep_nod
 }
 
 __device__ __forceinline__ unsigned dep_begin(const UpsweepIndex* ix, int depth) {  // of a depth's list
-    return ix->off[min(depth, NDEP - 1)];
+    return ix->off[min(max(depth, 0), NDEP - 1)];
 }
 
-// One depth, and the opening radii of the depth below it.
+// One depth, and the opening radii of the depth below it (depth -1: those of the roots alone).
 __global__ void __launch_bounds__(COMBINE_BS) k_combine_level(const uint32_t* __restrict__ dep_nodes,
                                                               const UpsweepIndex* ix, int depth, const unsigned* counts,
                                                               const float4* __restrict__ nd_geo, Moments mo,
@@ -2224,7 +2224,10 @@ void tree_build(Engine& e, double theta) {
     else
         for (size_t width = x.nroots; width <= TOP_NODES && top < depth - 1; width *= 8) ++top;
     const int cb = std::max(1, std::min(4 * e.sms, grid_for(static_cast<long long>(T), COMBINE_NODES)));
-    for (int d = depth - 1; d > top; --d) {
+    // With more roots than one round of the cluster takes (a wide forest), every depth has its launch, and
+    // the roots' radii a last one.
+    const int last = top < 0 && depth > 0 ? -1 : top + 1;
+    for (int d = depth - 1; d >= last; --d) {
         launch_pdl(overlap(n), k_combine_level, cb, COMBINE_BS, s, t.dep_nodes.as<uint32_t>(), ix, d,
                    counts, t.nd_geo.as<float4>(), mo, inv_theta, t.inv_theta_sys, sys, e.err_word());
         ++e.launches;
