@@ -216,17 +216,21 @@ __global__ void k_vjp_apply(const float4* __restrict__ partial, int n, int slice
 // which is 34 FP32 operations for two ordered pairs instead of 52. Work units are pairs of
 // STILE-body tiles (I, J), J >= I; a block takes a strip of SSTRIP J tiles (or fewer) for one I tile,
 // its threads holding SIPT i-bodies each. The i side sums in registers over the strip. The j side of
-// a warp: its lanes hold different pairs of j-bodies, 32 pairs at a time, and the pairs' sums move on
-// by one lane after each step, so that after 32 steps every pair has met every lane's i-bodies. Only
-// what the body's gradient needs travels, four sums per body: with m_j and w_j at hand the lane adds
-//   o = m_j S1 - w_j S2 - 3 S3  (its i-bodies' share of S1, S2, S3)  and h.
-// The block's warps are added in shared memory (warp order), and stored per unit. A diagonal unit
-// (J == I) masks the pairs j <= k. All sums run in a fixed order, so results do not depend on
-// scheduling; k_vjp_sym_apply adds the strips' and units' partial sums per body in FP64.
-// Bound by the FMA pipe: 146 packed instructions per step of a warp. With all lanes on one pair of
-// j-bodies and a butterfly of 16 values after it (62 instructions) 65 536 bodies took 2.99 ms and the
-// partial sums, twice as many, 0.27 ms; now 2.55 and 0.11 (two resident blocks instead of three: 2.52, two
-// i-bodies per thread: 3.0).
+// a warp: its lanes hold different pairs of j-bodies, 32 pairs at a time, and the pairs' eight sums move
+// on by one lane after each step, so that after 32 steps every pair has met every lane's i-bodies.
+// After STURN steps they are laid down in shared memory, and what the block's warps laid down for a
+// body is added with the roundings carried along and stored per unit. A diagonal unit (J == I) masks
+// the pairs j <= k. All sums run in a fixed order, so results do not depend on scheduling.
+// k_vjp_sym_apply adds the strips' and units' partial sums per body and combines them, both in FP64:
+// m S1 - w S2 - 3 S3 cancels between near neighbours, and in FP32 it would keep the roundings of its
+// terms.
+// Bound by the FMA pipe, with the shuffles beside it: 142 packed instructions and 16 shuffles per step
+// of a warp. With all lanes on one pair of j-bodies and a butterfly of 16 values after it (62
+// instructions more, 46 of them selects and scalar additions), and one thread per body to add the
+// partial sums, a backward pass of eight steps over 65 536 bodies took 28.3 ms; now 25.7 (two resident
+// blocks instead of three: 25.6). The error against FP64, over three scenarios, sizes and kinds of
+// weights, is that form's (ratio of the means 1.00 on the i side, 0.95 on the j side). Travelling with
+// the four combined sums only, 23.0 ms, is not: the combination is then rounded at every step.
 #ifndef LG_VJPS_BS
 #define LG_VJPS_BS 128
 #endif
@@ -250,9 +254,13 @@ constexpr int SSTRIP = LG_VJPS_STRIP;  // J tiles per block
 constexpr int SWARPS = SBS / 32;
 static_assert(STILE % SSUB == 0 && SSUB % 64 == 0, "sub-tiles hold whole turns of 32 j pairs");
 
+constexpr int STURN = 8;               // steps the travelling sums take before they are laid down
+constexpr int SROWS = 2;               // rows a warp lays them down in, in turn
+static_assert(32 % (STURN * SROWS) == 0, "every row takes as many turns");
+
 struct __align__(16) SymSmem {
     float jx[STILE], jy[STILE], jz[STILE], jnm[STILE], jwx[STILE], jwy[STILE], jwz[STILE];
-    float4 red[SWARPS][SSUB];
+    float4 red[SWARPS][SROWS][2][SSUB];  // (S1, -S2) and (S3, h) of a body
 };
 
 constexpr float kFarV = 1e18f;  // a far, massless, zero-weight body: adds nothing to either side
@@ -264,12 +272,13 @@ __device__ __forceinline__ size_t jrow(int I, int npad) {
 
 // units[b] = (I, J0, J1, strip): block b evaluates tile I against tiles [J0, J1) and writes its i
 // sums to row `strip` of ipart (the tile's STILE bodies); the j sums of unit (I, J) go to row I of
-// jpart. Entries are o and h of the body, both with the opposite sign.
+// jpart. Entries are 8 floats: S1 (3), -S2, S3 (3), h, where jpart holds the j side's -S2, S3 and
+// h with the opposite sign.
 template <bool EPS0>
 __global__ void __launch_bounds__(SBS, LG_VJPS_MINB) k_vjp_sym(const float4* __restrict__ hm, const float4* __restrict__ lo,
                                                    const float4* __restrict__ wv, int n, int npad, float e2,
-                                                   const int4* __restrict__ units, float4* __restrict__ ipart,
-                                                   float4* __restrict__ jpart) {
+                                                   const int4* __restrict__ units, float* __restrict__ ipart,
+                                                   float* __restrict__ jpart) {
     __shared__ SymSmem sm;
     const int4 un = units[blockIdx.x];
     const int I = un.x, J0 = un.y, J1 = un.z, strip = un.w;
@@ -300,7 +309,6 @@ __global__ void __launch_bounds__(SBS, LG_VJPS_MINB) k_vjp_sym(const float4* __r
         for (int q = 0; q < 8; ++q) a[u][q] = 0ull;
     }
     const f2x E2 = f2_bcast(e2);
-    const f2x CN3 = f2_bcast(-3.f);
     for (int J = J0; J < J1; ++J) {
         const int jb = J * STILE;
         __syncthreads();  // the previous tile's readers are done
@@ -325,9 +333,13 @@ __global__ void __launch_bounds__(SBS, LG_VJPS_MINB) k_vjp_sym(const float4* __r
         constexpr bool DIAG = decltype(diag_tag)::value;
         for (int s0 = 0; s0 < STILE; s0 += SSUB) {
           for (int c0 = s0; c0 < s0 + SSUB; c0 += 64) {
-            f2x ox = 0ull, oy = 0ull, oz = 0ull, oh = 0ull;  // the pair's sums, of opposite sign
 #pragma unroll 1
-            for (int st = 0; st < 32; ++st) {
+            for (int t = 0; t < 32; t += STURN) {
+            f2x o[8];  // the travelling sums of a pair
+#pragma unroll
+            for (int q = 0; q < 8; ++q) o[q] = 0ull;
+#pragma unroll 1
+            for (int st = t; st < t + STURN; ++st) {
                 const int jp = c0 + 2 * ((lane + st) & 31);
                 const f2x X = ld2(sm.jx + jp), Y = ld2(sm.jy + jp), Z = ld2(sm.jz + jp), NM = ld2(sm.jnm + jp);
                 const f2x WX = ld2(sm.jwx + jp), WY = ld2(sm.jwy + jp), WZ = ld2(sm.jwz + jp);
@@ -372,32 +384,45 @@ __global__ void __launch_bounds__(SBS, LG_VJPS_MINB) k_vjp_sym(const float4* __r
                     b[6] = f2_fma(cc, dz, b[6]);
                     b[7] = f2_fma(dwk, inv3, b[7]);
                 }
-                // Every sum goes to the lane that meets the pair next: after 32 steps to lane l pair l.
-                const int from = (lane + 1) & 31;
-                ox = __shfl_sync(0xffffffffu, f2_fma(NM, b[0], f2_fma(WX, b[3], f2_fma(CN3, b[4], ox))), from);
-                oy = __shfl_sync(0xffffffffu, f2_fma(NM, b[1], f2_fma(WY, b[3], f2_fma(CN3, b[5], oy))), from);
-                oz = __shfl_sync(0xffffffffu, f2_fma(NM, b[2], f2_fma(WZ, b[3], f2_fma(CN3, b[6], oz))), from);
-                oh = __shfl_sync(0xffffffffu, f2_add(oh, b[7]), from);
+                // To the lane that meets the pair next.
+#pragma unroll
+                for (int q = 0; q < 8; ++q) o[q] = __shfl_sync(0xffffffffu, f2_add(o[q], b[q]), (lane + 1) & 31);
             }
-            float4 r0, r1;
-            f2_unpack(ox, r0.x, r1.x);
-            f2_unpack(oy, r0.y, r1.y);
-            f2_unpack(oz, r0.z, r1.z);
-            f2_unpack(oh, r0.w, r1.w);
-            sm.red[warp][c0 - s0 + 2 * lane] = r0;
-            sm.red[warp][c0 - s0 + 2 * lane + 1] = r1;
+            const int at = c0 - s0 + 2 * ((lane + t + STURN) & 31), row = t / STURN % SROWS;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float4 r0, r1;
+                f2_unpack(o[4 * h], r0.x, r1.x);
+                f2_unpack(o[4 * h + 1], r0.y, r1.y);
+                f2_unpack(o[4 * h + 2], r0.z, r1.z);
+                f2_unpack(o[4 * h + 3], r0.w, r1.w);
+                float4* red = sm.red[warp][row][h] + at;
+                if (t >= STURN * SROWS) {
+                    r0 = add4(red[0], r0);
+                    r1 = add4(red[1], r1);
+                }
+                red[0] = r0;
+                red[1] = r1;
+            }
+            __syncwarp();  // other lanes of the warp add to them
+            }
           }
             __syncthreads();
-            // The sub-tile's j sums over the block's warps, in warp order.
-            for (int jj = tid; jj < SSUB; jj += SBS) {
-                float4 sum = sm.red[0][jj];
+            // The sub-tile's j sums over the warps' rows.
+            for (int q = tid; q < 2 * SSUB; q += SBS) {
+                const int jj = q >> 1, h = q & 1;
+                float4 sum = sm.red[0][0][h][jj], err = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int w = 1; w < SWARPS; ++w) {
-                    const float4 r = sm.red[w][jj];
-                    sum = make_float4(sum.x + r.x, sum.y + r.y, sum.z + r.z, sum.w + r.w);
+                for (int w = 1; w < SWARPS * SROWS; ++w) {
+                    const float4 r = sm.red[w / SROWS][w % SROWS][h][jj];
+                    two_sum(sum.x, err.x, r.x);
+                    two_sum(sum.y, err.y, r.y);
+                    two_sum(sum.z, err.z, r.z);
+                    two_sum(sum.w, err.w, r.w);
                 }
                 const int j = jb + s0 + jj;
-                if (j < n) jpart[jrow(I, npad) + (j - ib)] = sum;
+                if (j < n) reinterpret_cast<float4*>(jpart)[(jrow(I, npad) + (j - ib)) * 2 + h] =
+                    make_float4(carried(sum.x, err.x), carried(sum.y, err.y), carried(sum.z, err.z), carried(sum.w, err.w));
             }
             __syncthreads();  // red is rewritten by the next sub-tile
         }
@@ -408,56 +433,60 @@ __global__ void __launch_bounds__(SBS, LG_VJPS_MINB) k_vjp_sym(const float4* __r
 #pragma unroll
     for (int u = 0; u < SIPT; ++u) {
         if (iidx[u] >= n) continue;
-        // -(m S1 - w S2 - 3 S3), -h; a[u][3] holds -S2
-        const float m = hm[iidx[u]].w, s2 = f2_sum(a[u][3]);
-        const float4 w = wv[iidx[u]];
-        ipart[static_cast<size_t>(strip) * STILE + (iidx[u] - ib)] =
-            make_float4(fmaf(-m, f2_sum(a[u][0]), fmaf(-w.x, s2, 3.f * f2_sum(a[u][4]))),
-                        fmaf(-m, f2_sum(a[u][1]), fmaf(-w.y, s2, 3.f * f2_sum(a[u][5]))),
-                        fmaf(-m, f2_sum(a[u][2]), fmaf(-w.z, s2, 3.f * f2_sum(a[u][6]))), -f2_sum(a[u][7]));
+        float4* o = reinterpret_cast<float4*>(ipart) + (static_cast<size_t>(strip) * STILE + (iidx[u] - ib)) * 2;
+        o[0] = make_float4(f2_sum(a[u][0]), f2_sum(a[u][1]), f2_sum(a[u][2]), f2_sum(a[u][3]));
+        o[1] = make_float4(f2_sum(a[u][4]), f2_sum(a[u][5]), f2_sum(a[u][6]), f2_sum(a[u][7]));
     }
 }
 
 // Per body k of tile K: the i sums of K's strips and the j sums of units (I, K), I <= K, in FP64; then
-// lx += G o, lm -= G h. APARTS threads per body take every APARTS-th row (a thread per body had up to
-// 192 dependent reads), and their sums are added in order.
-constexpr int ABODIES = 32, APARTS = 8;  // 65 536 bodies: 0.27 -> 0.11 ms, FP64 additions
-__global__ void __launch_bounds__(ABODIES * APARTS) k_vjp_sym_apply(const float4* __restrict__ ipart,
-                                                                    const float4* __restrict__ jpart,
-                                                                    const int* __restrict__ strip_base, int n,
-                                                                    int npad, double G, double* lx, double* ly,
-                                                                    double* lz, double* lm) {
-    __shared__ double sums[APARTS][4][ABODIES];
+// lx += G (m_k S1 - w_k S2 - 3 S3), lm -= G h. APARTS threads per body take every APARTS-th row (a
+// thread per body had up to 192 dependent reads), and their sums are added in order.
+constexpr int ABODIES = 32, APARTS = 8;
+__global__ void __launch_bounds__(ABODIES * APARTS) k_vjp_sym_apply(const float* __restrict__ ipart,
+                                                                    const float* __restrict__ jpart,
+                                                                    const int* __restrict__ strip_base,
+                                                                    const float4* __restrict__ hm,
+                                                                    const float4* __restrict__ wv, int n, int npad,
+                                                                    double G, double* lx, double* ly, double* lz,
+                                                                    double* lm) {
+    __shared__ double sums[APARTS][8][ABODIES];
     const int lane = threadIdx.x % ABODIES, part = threadIdx.x / ABODIES;
     const int k = blockIdx.x * ABODIES + lane;
-    double S[4] = {0, 0, 0, 0};
+    double S[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (k < n) {
         const int K = k / STILE;
-        auto add = [&](const float4 p) {
-            S[0] += p.x;
-            S[1] += p.y;
-            S[2] += p.z;
-            S[3] += p.w;
-        };
         const int st1 = strip_base[K + 1];
 #pragma unroll 4
-        for (int st = strip_base[K] + part; st < st1; st += APARTS)
-            add(ipart[static_cast<size_t>(st) * STILE + (k - K * STILE)]);
+        for (int st = strip_base[K] + part; st < st1; st += APARTS) {
+            const float4* p = reinterpret_cast<const float4*>(ipart) + (static_cast<size_t>(st) * STILE + (k - K * STILE)) * 2;
+            const float4 p0 = p[0], p1 = p[1];
+            S[0] += p0.x; S[1] += p0.y; S[2] += p0.z; S[3] += p0.w;
+            S[4] += p1.x; S[5] += p1.y; S[6] += p1.z; S[7] += p1.w;
+        }
 #pragma unroll 4
-        for (int I = part; I <= K; I += APARTS) add(jpart[jrow(I, npad) + (k - I * STILE)]);
+        for (int I = part; I <= K; I += APARTS) {
+            const float4* p = reinterpret_cast<const float4*>(jpart) + (jrow(I, npad) + (k - I * STILE)) * 2;
+            const float4 p0 = p[0], p1 = p[1];
+            S[0] += p0.x; S[1] += p0.y; S[2] += p0.z; S[3] -= p0.w;
+            S[4] -= p1.x; S[5] -= p1.y; S[6] -= p1.z; S[7] -= p1.w;
+        }
     }
 #pragma unroll
-    for (int c = 0; c < 4; ++c) sums[part][c][lane] = S[c];
+    for (int c = 0; c < 8; ++c) sums[part][c][lane] = S[c];
     __syncthreads();
     if (part != 0 || k >= n) return;
 #pragma unroll
     for (int p = 1; p < APARTS; ++p)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) S[c] += sums[p][c][lane];
-    lx[k] -= G * S[0];
-    ly[k] -= G * S[1];
-    lz[k] -= G * S[2];
-    lm[k] += G * S[3];
+        for (int c = 0; c < 8; ++c) S[c] += sums[p][c][lane];
+    const double m = hm[k].w;
+    const float4 w = wv[k];
+    // S[3] holds -S2
+    lx[k] += G * (m * S[0] + w.x * S[3] - 3.0 * S[4]);
+    ly[k] += G * (m * S[1] + w.y * S[3] - 3.0 * S[5]);
+    lz[k] += G * (m * S[2] + w.z * S[3] - 3.0 * S[6]);
+    lm[k] -= G * S[7];
 }
 
 // lv += dt lx; w = c lv (FP32 for the VJP), with the body's mass alongside.
@@ -802,14 +831,14 @@ double adjoint_backward(Engine& e, AdjointState& a, const double* tx, const doub
     slices = (n + jslice - 1) / jslice;
     // Symmetric VJP (each unordered pair once) when there are enough tile units to fill the GPU
     // (at least four per SM: about 26k bodies and up; below that the one-sided kernel's split-j
-    // grid fills it better) and its partial sums stay within 2 GB (about 250k bodies).
+    // grid fills it better) and its partial sums stay within 4 GB (about 250k bodies).
     // LETTUCE_GB300_VJP=pairs or =symmetric overrides the size rule (not the memory bound).
     const int T = (n + STILE - 1) / STILE;
     const int npad = T * STILE;
-    const size_t jbytes = static_cast<size_t>(STILE) * T * (T + 1) / 2 * 16;
+    const size_t jbytes = static_cast<size_t>(STILE) * T * (T + 1) / 2 * 32;
     long long units_needed = 0;  // one block per strip of up to SSTRIP tiles: sum over I of ceil((T - I) / SSTRIP)
     for (int I = 0; I < T; ++I) units_needed += (T - I + SSTRIP - 1) / SSTRIP;
-    const bool fits = jbytes + static_cast<size_t>(units_needed) * STILE * 16 <= (size_t(2) << 30);
+    const bool fits = jbytes + static_cast<size_t>(units_needed) * STILE * 32 <= (size_t(4) << 30);
     bool sym = !tree && fits && units_needed >= 4LL * e.sms;
     if (const char* v = std::getenv("LETTUCE_GB300_VJP")) {
         const std::string m = v;
@@ -836,7 +865,7 @@ double adjoint_backward(Engine& e, AdjointState& a, const double* tx, const doub
                               cudaMemcpyHostToDevice, s));
         LG_CK(cudaMemcpyAsync(a.sym_sbase.as<int>(), a.sym_sbase_h.data(), a.sym_sbase_h.size() * sizeof(int),
                               cudaMemcpyHostToDevice, s));
-        a.ipart.reserve(static_cast<size_t>(strip) * STILE * 16);
+        a.ipart.reserve(static_cast<size_t>(strip) * STILE * 32);
         a.jpart.reserve(jbytes);
     } else if (!tree) {
         a.partial.reserve(static_cast<size_t>(slices) * n * 16);
@@ -922,16 +951,16 @@ double adjoint_backward(Engine& e, AdjointState& a, const double* tx, const doub
                 if (sym) {
                     if (eps0)
                         k_vjp_sym<true><<<nunits, SBS, 0, vs>>>(hm, lo, a.w.as<float4>(), n, npad, e2,
-                                                                a.sym_units.as<int4>(), a.ipart.as<float4>(),
-                                                                a.jpart.as<float4>());
+                                                                a.sym_units.as<int4>(), a.ipart.as<float>(),
+                                                                a.jpart.as<float>());
                     else
                         k_vjp_sym<false><<<nunits, SBS, 0, vs>>>(hm, lo, a.w.as<float4>(), n, npad, e2,
-                                                                 a.sym_units.as<int4>(), a.ipart.as<float4>(),
-                                                                 a.jpart.as<float4>());
+                                                                 a.sym_units.as<int4>(), a.ipart.as<float>(),
+                                                                 a.jpart.as<float>());
                     LG_LAUNCHED();
                     k_vjp_sym_apply<<<grid_for(n, ABODIES), ABODIES * APARTS, 0, vs>>>(
-                        a.ipart.as<float4>(), a.jpart.as<float4>(), a.sym_sbase.as<int>(), n, npad, a.p.G,
-                        a.lx.as<double>(), a.ly.as<double>(), a.lz.as<double>(), a.lm.as<double>());
+                        a.ipart.as<float>(), a.jpart.as<float>(), a.sym_sbase.as<int>(), hm, a.w.as<float4>(), n, npad,
+                        a.p.G, a.lx.as<double>(), a.ly.as<double>(), a.lz.as<double>(), a.lm.as<double>());
                     LG_LAUNCHED();
                     e.launches += 3;
                     continue;

@@ -210,6 +210,20 @@ __device__ __forceinline__ float f2_sum(f2x v) {
 }
 
 // ---- compensated summation ---------------------------------------------------------------
+// Adds x to s, and what s cannot hold of the sum, exactly, to err (Knuth's two-sum): s + err at the end
+// carries every term, also where large ones cancel.
+__device__ __forceinline__ void two_sum(float& s, float& err, float x) {
+    const float t = __fadd_rn(s, x), b = __fsub_rn(t, s);
+    err = __fadd_rn(err, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b)));
+    s = t;
+}
+// The sum; past the type's range as without the compensation.
+__device__ __forceinline__ float carried(float s, float err) {
+    return fabsf(s) <= 3.402823466e38f ? __fadd_rn(s, err) : s;
+}
+__device__ __forceinline__ float4 add4(float4 a, float4 b) {
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
 // Kahan step: adds x to (s, c), c carrying the low-order bits lost by s.
 __device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
     float y = x - c;
