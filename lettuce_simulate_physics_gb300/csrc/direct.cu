@@ -234,36 +234,46 @@ __global__ void __launch_bounds__(DBS, LG_DIRECT_MINB) k_direct_batch(const floa
     direct_block<IPT, TL, POT, EPS0>(sm, hm, lo, w.base, w.iend, w.j0, w.j1, G, w.e2, acc, true, err);
 }
 
-// Sums the split-j partials (Kahan) and scales by G: `parts` threads per body take every parts-th slice
-// in order, and their sums are added in order. One thread per body read up to 40 slices one after
-// another on a few SMs; see launch_direct for what it measured.
+// Sums the split-j partials and scales by G: `parts` threads per body take every parts-th slice in order,
+// and their sums are added in order. What the sums cannot hold is carried along and handed over with
+// them, so that a slice's part is kept although another thread holds what cancels the larger ones. One
+// thread per body read up to 40 slices one after another on a few SMs; see launch_direct for what it
+// measured.
 constexpr int RBS = 256;
 __global__ void __launch_bounds__(RBS) k_direct_reduce(const float4* __restrict__ partial, int n, int slices, int parts,
                                                        float G, float4* __restrict__ acc, float* __restrict__ cost) {
-    __shared__ float4 sums[RBS];
+    __shared__ float4 sums[RBS], errs[RBS];
     pdl_wait();
     const int bodies = RBS / parts, part = threadIdx.x / bodies, lane = threadIdx.x - part * bodies;
     const int i = blockIdx.x * bodies + lane;
     float s[4] = {0, 0, 0, 0}, c[4] = {0, 0, 0, 0};
     auto add = [&](const float4 p) {
-        kahan_add(s[0], c[0], p.x);
-        kahan_add(s[1], c[1], p.y);
-        kahan_add(s[2], c[2], p.z);
-        kahan_add(s[3], c[3], p.w);
+        two_sum(s[0], c[0], p.x);
+        two_sum(s[1], c[1], p.y);
+        two_sum(s[2], c[2], p.z);
+        two_sum(s[3], c[3], p.w);
     };
     if (i < n) {
 #pragma unroll 4
         for (int k = part; k < slices; k += parts) add(partial[static_cast<size_t>(k) * n + i]);
     }
     if (parts > 1) {
-        sums[threadIdx.x] = make_float4(s[0] - c[0], s[1] - c[1], s[2] - c[2], s[3] - c[3]);
+        sums[threadIdx.x] = make_float4(s[0], s[1], s[2], s[3]);
+        errs[threadIdx.x] = make_float4(c[0], c[1], c[2], c[3]);
         __syncthreads();
         if (part) return;
-        for (int p = 1; p < parts; ++p) add(sums[p * bodies + lane]);
+        for (int p = 1; p < parts; ++p) {
+            add(sums[p * bodies + lane]);
+            const float4 e = errs[p * bodies + lane];
+            c[0] += e.x;
+            c[1] += e.y;
+            c[2] += e.z;
+            c[3] += e.w;
+        }
     }
     if (i >= n) return;
     if (cost) cost[i] = static_cast<float>(n - 1);
-    acc[i] = make_float4(G * (s[0] - c[0]), G * (s[1] - c[1]), G * (s[2] - c[2]), -G * (s[3] - c[3]));
+    acc[i] = make_float4(G * (s[0] + c[0]), G * (s[1] + c[1]), G * (s[2] + c[2]), -G * (s[3] + c[3]));
 }
 
 template <int IPT, int TL>
