@@ -112,7 +112,7 @@ struct TreeState {
     // sort
     DevBuf keysA, keysB, valsA, valsB, hist, lookback;
     bool clusters_of_16 = false;  // k_combine_top may be launched as one
-    bool sort_full = false;  // a partial sort met a run too long to order locally: all key bits from now on
+    int known_depth = 0;  // the tree's depth at its last exact build, with headroom (0: unknown): digits to sort
     // sorted frame-0 keys, per-body tree data
     DevBuf skey, leafid;
     // frame, key-restart runs and frames (index 0 of the per-frame buffers unused)
@@ -1886,15 +1886,6 @@ void reserve_sort(TreeState& t, int n) {
     t.leaf_state.reserve(leaf_state_words(n) * 16);
 }
 
-// Octal digits to sort by when no earlier build says how deep the tree is: one and a half times
-// log8 n and two more (cells of that depth hold a few bodies at most in the scenarios' density
-// ranges: the trees of 8e3, 1e5, 1e6 and 1.6e7 bodies are 7, 9, 11 and 13 deep).
-int default_levels(int n) {
-    int l = 0;
-    while ((1ll << (3 * l)) < n) ++l;
-    return std::min(MAX_LEVEL, l + (l + 1) / 2 + 2);
-}
-
 int bits_for(int count) {
     int b = 0;
     while ((1 << b) < count) ++b;
@@ -1925,18 +1916,20 @@ void tree_sort(Engine& e) {
     const int run_cap = std::max(1, n / (LEAF_MAX + 1) + 1);  // runs hold more than LEAF_MAX bodies each
     unsigned R = 0;
     // The leading digits decide the order of all bodies but those of one cell that deep: as many
-    // digits are sorted as the tree was deep last time (with its headroom), in whole 8-bit passes
-    // (8e3 bodies: 4 passes, 1e5: 5, 1e6: 5, 1.6e7: 6, of 8 for all 63 bits), and bodies that tie
-    // are ordered where they are gathered (k_permute). A tree that turns out deeper is found there,
-    // and the sort redone with every digit; so it is from then on. With the clearing, the
-    // histograms and the digits' scans folded into the kernels around the passes: sort phase 142 ->
-    // 54 us (8191 bodies), 160 -> 75 (1e5), 302 -> 184 (1e6 disk), 2.76 -> 2.12 ms (1.6e7); below
-    // 1e6 it is the latency of 7 or 8 dependent launches, above, the passes' traffic.
-    for (bool full = t.sort_full || t.restart_mode;; full = true) {
+    // digits are sorted as the tree was deep at its last exact build (with its headroom), in whole
+    // 8-bit passes (8e3 bodies: 4 passes, 1e5: 5, 1e6: 5, 1.6e7: 6, of 8 for all 63 bits), and bodies
+    // that tie are ordered where they are gathered (k_permute). A tree that turns out deeper is found
+    // there; the sort is redone with every digit and the depth measured anew. Nothing is assumed of new
+    // bodies: a first sort takes every digit (a guess from n took three passes less on smooth scenes, 131 072
+    // bodies 95 us against 131, and a second whole sort where more than 16 bodies tied: with a tenth of
+    // the bodies in a core 220 against 132). With the clearing, the histograms and the digits' scans folded into the kernels
+    // around the passes: sort phase 142 -> 54 us (8191 bodies), 160 -> 75 (1e5), 302 -> 184 (1e6 disk),
+    // 2.76 -> 2.12 ms (1.6e7); below 1e6 it is the latency of 7 or 8 dependent launches, above, the
+    // passes' traffic.
+    for (bool full = t.known_depth <= 0 || t.restart_mode;; full = true) {
         int levels = MAX_LEVEL, passes = PASSES;
         if (!full) {
-            const int want = t.have_guess ? std::min(t.max_depth, MAX_LEVEL) : default_levels(n);
-            passes = std::max(1, (3 * want + sysbits + 7) / 8);
+            passes = std::max(1, (3 * std::min(t.known_depth, MAX_LEVEL) + sysbits + 7) / 8);
             levels = std::min(MAX_LEVEL, (8 * passes - sysbits) / 3);
             full = passes >= PASSES;
         }
@@ -1998,7 +1991,7 @@ void tree_sort(Engine& e) {
         LG_CK(cudaStreamSynchronize(s));
         R = e.pinned_small[0];
         if (full || !e.pinned_small[7]) break;
-        t.sort_full = true;
+        t.known_depth = 0;
     }
     // Runs are disjoint and longer than LEAF_MAX, so there are fewer than run_cap.
     R = std::min(R, static_cast<unsigned>(run_cap));
@@ -2113,6 +2106,7 @@ void tree_build(Engine& e, double theta) {
         t.K = std::min(static_cast<size_t>(n), Kx + Kx * pct / 100 + slack);
         t.T = Tx + Tx * pct / 100 + slack;
         t.max_depth = std::min(dx + (pct ? 2 : 0), MAX_DEPTH + 1);
+        t.known_depth = std::max(1, t.max_depth);
         t.have_guess = true;
         ++t.generation;
     }
@@ -2271,7 +2265,7 @@ bool tree_verify(Engine& e, const unsigned* counts_host) {
     const bool ok = (t.restarted || R == 0) && K <= t.K && T <= t.T && depth <= t.max_depth && !long_run;
     if (!ok) {
         if (!t.restarted && R > 0) t.restart_mode = true;
-        if (long_run) t.sort_full = true;
+        if (long_run) t.known_depth = 0;
         t.have_guess = false;  // next build reads exact sizes
     }
     return ok;
@@ -2300,7 +2294,7 @@ void tree_set_forest(Engine& e, int n_tree, int nsys, const uint32_t* sys, const
     t.inv_theta_sys = inv_theta_sys;
     t.have_guess = false;
     t.restart_mode = false;
-    t.sort_full = false;
+    t.known_depth = 0;
 }
 
 bool tree_sync_free_ready(const Engine& e) { return e.tree->have_guess && !e.tree->restart_mode; }
@@ -2320,7 +2314,7 @@ void tree_reset_guess(Engine& e) {
 }
 void tree_reset(Engine& e) {
     tree_reset_guess(e);
-    e.tree->sort_full = false;
+    e.tree->known_depth = 0;
 }
 double tree_theta(const Engine& e) { return e.tree->theta; }
 
