@@ -32,9 +32,10 @@ namespace {
 #define LG_DIRECT_MINB 1    // resident blocks per SM the register budget is sized for
 #endif
 // j-pair iterations unrolled in the inner loop: as many as give eight packed pairs in flight per
-// thread (two i-bodies with four: N = 65537 1.52 ms against 1.66 with two; four i-bodies with two:
-// 1.53 against 1.61 with four).
-constexpr int direct_unroll(int ipt) { return ipt <= 2 ? 4 : 2; }
+// thread, two at least. One i-body with two, four, eight: 48 systems of 3000 203, 198, 193 us, one of
+// 2047 with the potential 13.7, 13.2, 11.8 us. Two i-bodies with two and four: N = 65537 1.66 and 1.52
+// ms. Four with four and two: 1.61 and 1.53. Eight with one and two: N = 4e5 103.9 and 98.6 ms.
+constexpr int direct_unroll(int ipt) { return ipt <= 4 ? 8 / ipt : 2; }
 constexpr int DBS = 256;   // threads per block
 constexpr int TILE = 256;  // j-bodies per stage (default; 128 is the other compiled shape)
 
