@@ -132,6 +132,7 @@ struct TreeState {
     // scan state (merged walk groups)
     DevBuf scan_state, scan_ctr;
     size_t K = 0, T = 0, ngroups = 0;  // sizes the last build was launched with
+    size_t leaves = 0, nodes = 0;      // what the last exact build counted (K and T: with headroom)
     int max_depth = 0;
     bool restarted = false;
     int group_max = 128;
@@ -1562,10 +1563,10 @@ __device__ __forceinline__ void store_rcrit(const Moments& mo, uint32_t node, fl
 // k_leaf_moments for the trees whose leaves are too few to fill the FP64 units one to a thread, where
 // a leaf's chain of about 40 FP64 instructions per body is the time (8191 bodies: 27 -> 10 us). Bodies
 // in rounds of eight. The two folds of a body leave lanes idle, so more FP64 work is issued in all,
-// hence the line (build phase with a thread -> eight lanes per leaf: 8191 bodies 108 -> 90 us, 25000, of 4e3
-// leaves, 129 -> 123, 40000, of 6.4e3, 141 -> 147).
+// hence the line (build phase with a thread -> eight lanes per leaf, Plummer: 8191 bodies, 1748 leaves,
+// 106 -> 90 us, 16 000, 3348, 115 -> 100, 25 000, 5180, 117 -> 115, 30 000, 6173, 121 -> 129).
 constexpr int LEAFW_BS = 128;
-constexpr size_t LEAFW_MAX = 4096;
+constexpr size_t LEAFW_MAX = 5120;  // leaves at the last exact build
 __global__ void __launch_bounds__(LEAFW_BS) k_leaf_moments_wide(const uint32_t* __restrict__ leaf_order,
                                                                 const unsigned* counts,
                                                                 const float4* __restrict__ nd_geo,
@@ -2105,6 +2106,8 @@ void tree_build(Engine& e, double theta) {
         const size_t slack = pct ? 1024 : 0;
         t.K = std::min(static_cast<size_t>(n), Kx + Kx * pct / 100 + slack);
         t.T = Tx + Tx * pct / 100 + slack;
+        t.leaves = Kx;
+        t.nodes = Tx;
         t.max_depth = std::min(dx + (pct ? 2 : 0), MAX_DEPTH + 1);
         t.known_depth = std::max(1, t.max_depth);
         t.have_guess = true;
@@ -2203,18 +2206,19 @@ void tree_build(Engine& e, double theta) {
     // most TOP_NODES nodes (by the eight-way branching, or because the whole tree is small) together.
     const float inv_theta = theta > 0 ? static_cast<float>(1.0 / theta) : FLT_MAX;
     Moments mo{t.nd_test.as<NodeTest>(), t.nd_cell.as<NodeCell>()};
-    const bool wide = K <= LEAFW_MAX;
+    const bool wide = t.leaves <= LEAFW_MAX;
     launch_pdl(overlap(n), wide ? k_leaf_moments_wide : k_leaf_moments,
                grid_for(static_cast<long long>(K), wide ? LEAFW_BS / WIDE : 128), wide ? LEAFW_BS : 128, s,
                t.leaf_order.as<uint32_t>(), counts, t.nd_geo.as<float4>(), e.bodies(e.cur), mo, inv_theta,
                t.inv_theta_sys, sys, e.err_word());
     ++e.launches;
     int top = -1;
-    // The whole tree where that is no slower than a launch per depth on all SMs: up to 32 768 nodes (build
-    // phase, from 4096 nodes on by depths -> all in one: 25 000 bodies 136 -> 117 us, 65 536 163 -> 140,
-    // 100 003 176 -> 152; at 40 000 nodes, 131 072 bodies, 182 -> 172 and 155 -> 164 for a disk and a
-    // Plummer sphere, at 200 000 bodies 186 -> 215).
-    if (T <= 64 * TOP_NODES) top = depth - 1;
+    // The whole tree where that is faster than a launch per depth on all SMs: up to about 25 000 nodes at
+    // the last exact build (build phase by depths -> all in one: Plummer 60 000 bodies, 14 460 nodes, 166
+    // -> 133 us, 110 000, 25 423, 176 -> 165, 180 000, 41 051, 178 -> 193; a uniform cube, which has fewer
+    // and wider depths, 60 000, 13 966, 133 -> 123, 80 000, 27 379, 137 -> 145).
+    constexpr size_t WHOLE_MAX = 50 * TOP_NODES;
+    if (t.nodes <= WHOLE_MAX) top = depth - 1;
     else
         for (size_t width = x.nroots; width <= TOP_NODES && top < depth - 1; width *= 8) ++top;
     const int cb = std::max(1, std::min(4 * e.sms, grid_for(static_cast<long long>(T), COMBINE_NODES)));

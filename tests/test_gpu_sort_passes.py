@@ -60,3 +60,17 @@ def test_deeper_trees_take_the_digits_they_need(be, spread):
     deep, more = launches(be), passes(be)
     assert few < more < 8
     assert deep - shallow == more - few
+
+
+# The lines of the upsweep's dispatch are drawn by what the tree has, not by what is allocated for it.
+@pytest.mark.parametrize("n", [14000, 80000])
+def test_headroom_changes_no_launches(n, monkeypatch):
+    b = S.plummer(n, 3, cut=10)
+    got = []
+    for percent in (0, 25, 100):
+        monkeypatch.setenv("LETTUCE_GB300_TREE_HEADROOM", str(percent))
+        with L.CudaBackend(0) as be:
+            be.upload(b)
+            launches(be)
+            got.append(launches(be) - min(8, -(-3 * (be.tree_counts()["max_depth"] + (2 if percent else 0)) // 8)))
+    assert got[0] == got[1] == got[2]
