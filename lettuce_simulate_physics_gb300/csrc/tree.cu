@@ -557,8 +557,9 @@ __global__ void k_permute(const BodyArrays src, BodyArrays dst, const uint64_t* 
     if (i >= n_total) return;
     int to = i;
     uint32_t j = static_cast<uint32_t>(i);  // bodies past the tree's range (the forest's direct systems) stay
-    if (i < n && !(*err & kErrWaitTimeout)) {
-        j = vals[i];
+    const uint32_t from = vals[min(i, n - 1)], ran_out = *err & kErrWaitTimeout;  // one round trip for both
+    if (i < n && !ran_out) {
+        j = from;
         if (skey) {
             const uint64_t m = mkeys[j];
             if (partial) {
@@ -1003,7 +1004,8 @@ struct NodeCtx {
 // ran out: what a kernel left after one is not to be used as an index. (In a forest only the tree's own
 // kernels, one after another, set that bit; the direct systems' have a word of their own.)
 __device__ __forceinline__ bool build_ok(const unsigned* counts, const unsigned* err) {
-    return counts[8] != 0 && !(*err & kErrWaitTimeout);
+    const unsigned fit = counts[8], ran_out = *err & kErrWaitTimeout;  // one round trip for both
+    return (fit != 0) & (ran_out == 0);
 }
 
 // Pre-order nodes as k_nodes leaves them. meta: depth | leaf << 8 | group << 9 | octal digit under

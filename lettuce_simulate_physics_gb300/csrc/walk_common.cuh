@@ -99,7 +99,8 @@ __device__ __forceinline__ void build_lists(const ListArgs& w, S& s) {
     const uint32_t sub = lane & 7;
     uint2* gstk = w.stack + static_cast<size_t>(blockIdx.x) * SCAP;
     // No groups after a build in which a wait ran out: its nodes are not all there.
-    const unsigned ngroups = *w.err & kErrWaitTimeout ? 0u : *w.tv.ngroups;
+    const unsigned ran_out = *w.err & kErrWaitTimeout, groups = *w.tv.ngroups;
+    const unsigned ngroups = ran_out ? 0u : groups;
     const uint32_t T = static_cast<uint32_t>(w.tv.T);
     // With the local tree the own body is in the list (its leaf is inside the group, so it is
     // opened): it is not an interaction, adds nothing to a (d = 0) and is excluded from the
