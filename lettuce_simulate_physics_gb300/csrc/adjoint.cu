@@ -224,8 +224,8 @@ __global__ void k_vjp_apply(const float4* __restrict__ partial, int n, int slice
 // k_vjp_sym_apply adds the strips' and units' partial sums per body and combines them, both in FP64:
 // m S1 - w S2 - 3 S3 cancels between near neighbours, and in FP32 it would keep the roundings of its
 // terms.
-// Bound by the FMA pipe, with the shuffles beside it: 142 packed instructions and 16 shuffles per step
-// of a warp. With all lanes on one pair of j-bodies and a butterfly of 16 values after it (62
+// Bound by the FMA pipe, with the shuffles beside it: 144 packed instructions and 16 shuffles per step
+// of a warp, 2.79 ms at 65 536 bodies. With all lanes on one pair of j-bodies and a butterfly of 16 values after it (62
 // instructions more, 46 of them selects and scalar additions), and one thread per body to add the
 // partial sums, a backward pass of eight steps over 65 536 bodies took 28.3 ms; now 25.7 (two resident
 // blocks instead of three: 25.6). The error against FP64, over three scenarios, sizes and kinds of
@@ -441,7 +441,8 @@ __global__ void __launch_bounds__(SBS, LG_VJPS_MINB) k_vjp_sym(const float4* __r
 
 // Per body k of tile K: the i sums of K's strips and the j sums of units (I, K), I <= K, in FP64; then
 // lx += G (m_k S1 - w_k S2 - 3 S3), lm -= G h. APARTS threads per body take every APARTS-th row (a
-// thread per body had up to 192 dependent reads), and their sums are added in order.
+// thread per body had up to 192 dependent reads), and their sums are added in order. Bound by the FP64
+// pipe (85%): 65 536 bodies 0.27 -> 0.21 ms.
 constexpr int ABODIES = 32, APARTS = 8;
 __global__ void __launch_bounds__(ABODIES * APARTS) k_vjp_sym_apply(const float* __restrict__ ipart,
                                                                     const float* __restrict__ jpart,

@@ -232,11 +232,6 @@ void let_export_read(Engine& e, lg_let_node* nodes, float* bx, float* by, float*
 // differentiated through the bodies: g (4 arrays of n doubles: x, y, z, m; current body order)
 // accumulates d(sum_i w_i . a_i / G)/d(x, m). w: float4 weights per body (current order).
 void tree_walk_vjp(Engine& e, const float4* w, float e2, bool eps0, double* g);
-// walk_vjp.cu: vector-Jacobian product of the tree forces over the current tree's interaction
-// lists (the lists are those of the force walk on the same tree), with the cell moments
-// differentiated through the bodies: g (4 arrays of n doubles: x, y, z, m; current body order)
-// accumulates d(sum_i w_i . a_i / G)/d(x, m). w: float4 weights per body (current order).
-void tree_walk_vjp(Engine& e, const float4* w, float e2, bool eps0, double* g);
 // adjoint.cu
 std::unique_ptr<AdjointState, void (*)(AdjointState*)> make_adjoint_state();
 void adjoint_forward(Engine& e, AdjointState& a, const lg_force_params& p, double dt, int steps, int every);

@@ -1,5 +1,5 @@
 // Locally-essential trees (LETs): the reference's multi-rank support (src/backend.hpp:50-86).
-//  - let_upload: remote trees to the device for the walk (walk.cu), indices
+//  - let_upload: remote trees to the device for the walk (build_lists in walk_common.cuh), indices
 //    made global over the concatenated trees, every link checked on the host first.
 //  - let_body_blocks: blocks of 128 consecutive bodies with their FP32 bounding boxes, the direct
 //    method's receiver groups (src/cpu_backend.cpp:695-728).

@@ -1925,10 +1925,10 @@ void tree_sort(Engine& e) {
     // there; the sort is redone with every digit and the depth measured anew. Nothing is assumed of new
     // bodies: a first sort takes every digit (a guess from n took three passes less on smooth scenes, 131 072
     // bodies 95 us against 131, and a second whole sort where more than 16 bodies tied: with a tenth of
-    // the bodies in a core 220 against 132). With the clearing, the histograms and the digits' scans folded into the kernels
-    // around the passes: sort phase 142 -> 54 us (8191 bodies), 160 -> 75 (1e5), 302 -> 184 (1e6 disk),
-    // 2.76 -> 2.12 ms (1.6e7); below 1e6 it is the latency of 7 or 8 dependent launches, above, the
-    // passes' traffic.
+    // the bodies in a core 220 against 132). With the clearing, the histograms and the digits' scans
+    // folded into the kernels around the passes: sort phase 142 -> 54 us (8191 bodies), 160 -> 75 (1e5),
+    // 302 -> 184 (1e6 disk), 2.76 -> 2.12 ms (1.6e7); below 1e6 it is the latency of 7 or 8 dependent
+    // launches, above, the passes' traffic.
     for (bool full = t.known_depth <= 0 || t.restart_mode;; full = true) {
         int levels = MAX_LEVEL, passes = PASSES;
         if (!full) {
