@@ -873,6 +873,11 @@ double adjoint_backward(Engine& e, AdjointState& a, const double* tx, const doub
     }
     const float e2 = static_cast<float>(a.p.eps * a.p.eps);
     const bool eps0 = !(e2 >= 1.17549435e-38f);
+    // From here on the segments are replayed: the forward pass's final state is no longer resident, also
+    // after a pass that fails.
+    a.have_forward = false;
+    e.acc_ok = false;
+    e.tree_ok = false;
     const double h = 0.5 * a.dt;
     void* const dst[7] = {gx, gy, gz, gvx, gvy, gvz, gm};
     // Recomputes segment seg (checkpoint restore, then the segment's positions; the forces at the
@@ -1044,9 +1049,7 @@ double adjoint_backward(Engine& e, AdjointState& a, const double* tx, const doub
         for (int i = 0; i < n; ++i) static_cast<double*>(dst[k])[ids[i]] = buf[i];
     }
     LG_CK(cudaStreamSynchronize(s));
-    // The backward pass replayed the segments: the forward's final state is no longer resident.
-    a.have_forward = false;
-    e.acc_ok = false;
+    e.acc_ok = false;  // (the replay's own force calls set them)
     e.tree_ok = false;
     return L;
 }

@@ -70,3 +70,18 @@ def test_a_pass_that_fails_leaves_the_arrays_alone(be, n):
         L.backend._check(be._lib.lg_adjoint_backward(be._h, *(d(t[k]) for k in range(3)), None,
                                                      *(d(seven[k]) for k in range(7))))
     assert (seven == 7.0).all()
+
+
+@pytest.mark.parametrize("seeded", [False, True])
+def test_a_pass_that_failed_needs_a_new_forward_pass(be, seeded):
+    b, p, target = problem(500, L.ForceMethod.direct)
+    backward = be.adjoint_backward_seeded if seeded else be.adjoint_backward
+    be.upload(b)
+    be.adjoint_forward(p, 1e-3, 3, 2)
+    be.probe_wait_pending(2048)
+    with pytest.raises(RuntimeError, match="device wait timed out"):
+        backward(target)
+    with pytest.raises(L.LogicError):
+        backward(target)
+    with pytest.raises(L.LogicError):
+        be.kick(1e-3)
